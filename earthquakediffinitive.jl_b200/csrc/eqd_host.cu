@@ -21,6 +21,7 @@
 #include "solver_kernels.cuh"
 #include "rhs_kernels.cuh"
 #include "ring_march.cuh"
+#include "resident_cg.cuh"
 
 using namespace eqd;
 
@@ -84,6 +85,7 @@ static constexpr int kMaxT64 = 384;
 static constexpr int kMaxT64b = 512;  // FP64 instances for wide x1 lines (n1 = 33 needs 7 x 66 threads)
 static constexpr int kNumVariants = 11;  // 9 plane-march variants, then 2 ring-march variants
 static constexpr int kFirstRingVariant = 9;
+static constexpr int kResidentVariant = kNumVariants;  // whole iterations resident on chip (resident_cg.cuh)
 
 // Ring-march instances per n1: (x2 tile capacity, register cap per thread)
 // of its two variants. A CTA's threads x registers must fit the SM's 65,536,
@@ -367,6 +369,16 @@ struct Workspace {
     }
 };
 
+// The resident CG of one precision: its plan, the device tables, and the
+// kernel instance that runs it.
+struct ResEngine {
+    bool tried = false, ok = false;
+    ResDims d{};
+    int t2 = 0, t3 = 0;  // tile capacity of the kernel instance
+    DevBuf ranks, chunks, lines, gofs, push, tab, off;
+    ResTables tb{};
+};
+
 struct eqd_grid {
     eqd_grid_desc desc;
     GridConst gc;
@@ -385,8 +397,11 @@ struct eqd_grid {
     int v32_lanes[kNumVariants] = {};
     int sel32 = 0;
     bool tuned = false;
+    int pin = -1;          // variant the caller (or eqd_autotune) chose, kResidentVariant included; -1: none,
+                           // and solves run resident where the grid has a plan
+    ResEngine res32, res64;
     int chunk_tuned = 0;   // eqd_tune_chunk's choice of columns per batch (0: as many as the budget allows)
-    double tune_ms[kNumVariants] = {};
+    double tune_ms[kNumVariants + 1] = {};
     int nchunks = 1;
     cudaStream_t stream = nullptr;
     cudaStream_t stream2 = nullptr;          // second half of a split batch (graph capture only)
@@ -557,6 +572,124 @@ static cudaError_t configure_kernels(int smem_max) {
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
+}
+
+// ---------------------------------------------------------------------------
+// Resident CG (resident_cg.cuh): plan, tables and launch
+// ---------------------------------------------------------------------------
+// Kernel instances: n1, and the largest tile of own lines. The x1 lines of the
+// BP8 grids at 100, 80, 50 and 40 m (9 to 21 points) and of the cubes up to
+// 25; FP64 planes of more than 13 points a line do not fit shared memory.
+#define EQD_RES_32(X) X(9, 8, 8) X(9, 8, 16) X(11, 8, 8) X(11, 8, 16) X(13, 8, 8) X(15, 8, 8) X(17, 8, 8) X(21, 8, 8) X(25, 8, 8)
+#define EQD_RES_64(X) X(9, 8, 8) X(11, 8, 8) X(13, 8, 8)
+
+// f.operator()<N1, T2, T3>() for the instances of precision T in turn, until
+// one returns true.
+template <typename T, typename F>
+static bool res_instances(F &&f) {
+#define EQD_CASE(N, A, B) f(std::integral_constant<int, N>(), std::integral_constant<int, A>(), std::integral_constant<int, B>()) ||
+    if constexpr (sizeof(T) == 4) return EQD_RES_32(EQD_CASE) false;
+    else return EQD_RES_64(EQD_CASE) false;
+#undef EQD_CASE
+}
+
+static void res_launch_config(const ResDims &d, int ncols, cudaStream_t s, cudaLaunchConfig_t &cfg,
+                              cudaLaunchAttribute &at) {
+    cfg = cudaLaunchConfig_t{};
+    at = cudaLaunchAttribute{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = (unsigned)d.M;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.gridDim = dim3((unsigned)ncols * (unsigned)d.M);
+    cfg.blockDim = dim3((unsigned)(64 * d.nch0max));
+    cfg.dynamicSmemBytes = (size_t)d.smem;
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+}
+
+// The team and the instance with the least work per column-iteration over the
+// team (whole K at h = 50 m: 8 CTAs of 8 x 16 lines 205 ms, 16 of 8 x 8 227 ms;
+// h = 100 m: 2 of 8 x 16 9.2 ms, 4 of 8 x 8 9.9 ms, 9 of them 15.1 ms).
+template <typename T>
+static int ensure_resident(eqd_grid *G, ResEngine &E) {
+    if (E.tried) return EQD_OK;
+    E.tried = true;
+    const GridConst &gc = G->gc;
+    ResPlan best;
+    double best_cost = 1e300;
+    res_instances<T>([&](auto n1, auto t2, auto t3) {
+        if (n1 != gc.n1) return false;
+        const void *k = (const void *)resident_cg_kernel<T, n1, t2, t3>;
+        cudaFuncAttributes fa{};
+        if (cudaFuncGetAttributes(&fa, k) != cudaSuccess ||
+            cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResSmemMax) != cudaSuccess ||
+            cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        for (int m2 = 1; m2 <= kResMaxTeam; ++m2)
+            for (int m3 = 1; m2 * m3 <= kResMaxTeam; ++m3) {
+                ResPlan P;
+                if (!make_res_plan(gc.n1, gc.n2, gc.n3, gc.PS, m2, m3, res_strides<sizeof(T), n1, t2, t3>(), P)) continue;
+                if (64 * P.d.nch0max > fa.maxThreadsPerBlock) continue;
+                cudaLaunchConfig_t cfg;
+                cudaLaunchAttribute at;
+                res_launch_config(P.d, 1, nullptr, cfg, at);
+                int fit = 0;
+                if (cudaOccupancyMaxActiveClusters(&fit, k, &cfg) != cudaSuccess) {
+                    cudaGetLastError();  // the device cannot place this cluster
+                    continue;
+                }
+                if (fit < 1 || P.cost >= best_cost) continue;
+                best_cost = P.cost;
+                best = P;
+                E.t2 = t2;
+                E.t3 = t3;
+            }
+        return false;
+    });
+    if (best_cost == 1e300) return EQD_OK;
+    E.d = best.d;
+    std::vector<T> tab;
+    std::vector<int> off;
+    if (!fill_res_tables<T>(gc.n2, gc.n3, G->h[1], G->h[2], gc.mu, tab, off)) return EQD_OK;
+    auto put = [&](DevBuf &b, const void *src, size_t bytes) -> cudaError_t {
+        cudaError_t e = b.ensure(std::max<size_t>(bytes, 16));
+        if (e == cudaSuccess && bytes) e = cudaMemcpyAsync(b.p, src, bytes, cudaMemcpyHostToDevice, G->stream);
+        return e;
+    };
+    CUDA_OR_RETURN(put(E.ranks, best.ranks.data(), best.ranks.size() * sizeof(ResRank)));
+    CUDA_OR_RETURN(put(E.chunks, best.chunks.data(), best.chunks.size() * sizeof(int)));
+    CUDA_OR_RETURN(put(E.lines, best.lines.data(), best.lines.size() * sizeof(ResLine)));
+    CUDA_OR_RETURN(put(E.gofs, best.gofs.data(), best.gofs.size() * sizeof(int)));
+    CUDA_OR_RETURN(put(E.push, best.push.data(), best.push.size() * sizeof(int)));
+    CUDA_OR_RETURN(put(E.tab, tab.data(), tab.size() * sizeof(T)));
+    CUDA_OR_RETURN(put(E.off, off.data(), off.size() * sizeof(int)));
+    CUDA_OR_RETURN(cudaStreamSynchronize(G->stream));
+    E.tb = ResTables{E.ranks.as<ResRank>(), E.chunks.as<int>(), E.lines.as<ResLine>(), E.gofs.as<int>(),
+                     E.push.as<int>(), E.tab.p, E.off.as<int>()};
+    E.ok = true;
+    return EQD_OK;
+}
+
+// Up to kmax iterations of every active column (x: the FP32 correction, or
+// the FP64 solution).
+template <typename T>
+static cudaError_t launch_resident(eqd_grid *G, const ResEngine &E, T *x, T *r, T *p, const ColState &st,
+                                   const SolveParams &sp, int mixed, int kmax, int ncols, cudaStream_t s) {
+    cudaError_t e = cudaErrorInvalidValue;
+    res_instances<T>([&](auto n1, auto t2, auto t3) {
+        if (n1 != G->gc.n1 || t2 != E.t2 || t3 != E.t3) return false;
+        cudaLaunchConfig_t cfg;
+        cudaLaunchAttribute at;
+        res_launch_config(E.d, ncols, s, cfg, at);
+        const ResCoef<T> C = res_coef<T>(G->h[0], G->gc.lam, G->gc.mu, G->gc.sat_c);
+        const ResX1<T, n1> X = res_x1<T, n1>(G->h[0], G->gc.mu, G->gc.hvol);
+        e = cudaLaunchKernelEx(&cfg, resident_cg_kernel<T, n1, t2, t3>, C, X, E.d, E.tb, x, r, p, st, sp, mixed, kmax);
+        return true;
+    });
+    return e;
 }
 
 static int check_device_error(eqd_grid *G) {
@@ -968,6 +1101,22 @@ static constexpr int kVecThreads = 128;
 // gave 6.0, 6.6, 6.5, 6.3 k columns/s; one chain with one CTA per item 6.2 k).
 static constexpr int kVecCtasPerSm = 4;
 
+// Mixed precision: the flagged columns' FP64 true residual.
+template <typename T>
+static void record_reliable(eqd_grid *G, const IterPtrs<T> &P, const SolveParams &sp, const Span &sn) {
+    // One CTA per item: in most iterations no column is flagged and every
+    // CTA returns at once.
+    const unsigned items = (unsigned)((long long)sn.n * G->nchunks);
+    fold_correction_kernel<<<items, kVecThreads, 0, sn.s>>>(P.x64, P.d, P.st, sp, sn.n);
+    ColumnSet cf = P.cs;
+    cf.flag = P.st.flag;
+    cf.dinv = sp.precond ? G->dinv64.as<double>() : nullptr;
+    launch_march<double, float, MODE_RHS>(G, P.x64, (float *)P.r, cf, P.res_part, sn.n, -1, sn.s);
+    SolveParams sp2 = sp;
+    sp2.ntiles = nparts(G->m64);
+    cg_true_residual_kernel<<<(unsigned)((sn.n + 127) / 128), 128, 0, sn.s>>>(P.st, sp2, P.res_part, sn.n, 1);
+}
+
 // The rest of iteration k: x, r updates; scalars; reliable update (mixed);
 // the next direction (unless the next apply forms it).
 template <typename T>
@@ -998,18 +1147,7 @@ static void record_rest(eqd_grid *G, Workspace &W, int mixed, int fused, int k, 
     }
     const unsigned sb = (unsigned)((sn.n + 127) / 128);
     cg_scalar_kernel<<<sb, 128, 0, sn.s>>>(P.st, sp, P.apply_part, P.rr_part, sn.n, mixed);
-    if (mixed) {
-        // One CTA per item: in most iterations no column is flagged and every
-        // CTA returns at once.
-        fold_correction_kernel<<<(unsigned)items, kVecThreads, 0, sn.s>>>(P.x64, P.d, P.st, sp, sn.n);
-        ColumnSet cf = P.cs;
-        cf.flag = P.st.flag;
-        cf.dinv = dinv64;
-        launch_march<double, float, MODE_RHS>(G, P.x64, (float *)P.r, cf, P.res_part, sn.n, -1, sn.s);
-        SolveParams sp2 = sp;
-        sp2.ntiles = nparts(G->m64);
-        cg_true_residual_kernel<<<sb, 128, 0, sn.s>>>(P.st, sp2, P.res_part, sn.n, 1);
-    }
+    if (mixed) record_reliable<T>(G, P, sp, sn);
     if (!fused) {
         const T *dinvT = (const T *)(sizeof(T) == 4 ? (const void *)dinv32 : (const void *)dinv64);
         if (mixed)
@@ -1066,6 +1204,21 @@ static void record_iterations(eqd_grid *G, Workspace &W, int cap, int mixed, int
     cudaStreamWaitEvent(A.s, G->evBrest, 0);
 }
 
+// Resident iterations of `cap` slots: every active column runs until it needs
+// its true residual (mixed) or is done, at most kmax iterations, `rounds`
+// times.
+template <typename T>
+static void record_resident(eqd_grid *G, Workspace &W, int cap, int mixed, const SolveParams &sp, const ColState &st,
+                            int kmax, int rounds) {
+    const Span all{0, cap, G->stream, false};
+    IterPtrs<T> P = span_ptrs<T>(G, W, sp, st, all);
+    T *x = sizeof(T) == 4 ? (T *)P.d : (T *)P.x64;
+    for (int k = 0; k < rounds; ++k) {
+        launch_resident<T>(G, sizeof(T) == 4 ? G->res32 : G->res64, x, P.r, P.p, P.st, sp, mixed, kmax, cap, G->stream);
+        if (mixed) record_reliable<T>(G, P, sp, all);
+    }
+}
+
 // Jacobi weights dinv = 1 / diag(A) (zeros floored to 1), computed once per
 // grid; a negative diagonal entry is an error, as in the reference.
 static int ensure_jacobi(eqd_grid *G) {
@@ -1115,7 +1268,7 @@ struct ColDone {
     int8_t status;
 };
 
-static int tune_by_iterations(eqd_grid *G, const eqd_solve_opts &o, int ncols);
+static int tune_by_iterations(eqd_grid *G, const eqd_solve_opts &o, int ncols, bool with_resident = false);
 
 template <typename T>
 struct SlotRun {
@@ -1123,6 +1276,8 @@ struct SlotRun {
     Workspace *W = nullptr;
     int cap = 0, mixed = 0, generic = 0, dense = 0;
     int fused = 0;  // the direction update runs inside the stencil apply (MODE_AF)
+    int resident = 0;            // iterations run in resident_cg_kernel
+    int kmax = 256, rounds = 1;  // resident: iterations a launch may run, launches per graph
     long long itmax = 0;
     SolveParams sp{};
     ColState st{};
@@ -1135,7 +1290,8 @@ struct SlotRun {
     int64_t launches = 0;
     static constexpr int kIter = 10;
 
-    int setup(eqd_grid *g, const eqd_solve_opts &o, int capacity, bool gen, bool dns) {
+    // `tuning`: the caller times kIter iterations a launch.
+    int setup(eqd_grid *g, const eqd_solve_opts &o, int capacity, bool gen, bool dns, bool tuning = false) {
         G = g;
         W = &G->ws;
         cap = capacity;
@@ -1145,7 +1301,16 @@ struct SlotRun {
         const GridConst &gc = G->gc;
         const long long ntot = 6LL * gc.n1 * gc.n2 * gc.n3;
         const size_t vec = (size_t)gc.colstride * cap;
-        if (mixed && !G->tuned) {
+        resident = 0;
+        if (!gen && o.precond != EQD_PRECOND_JACOBI && (G->pin < 0 || G->pin == kResidentVariant)) {
+            ResEngine &E = sizeof(T) == 4 ? G->res32 : G->res64;
+            int rc = ensure_resident<T>(G, E);
+            if (rc) return rc;
+            resident = E.ok;
+            kmax = tuning ? kIter : 256;
+            rounds = mixed && !tuning ? 2 : 1;
+        }
+        if (mixed && !G->tuned && !resident) {
             int rc = tune_by_iterations(G, o, std::min(cap, 1024));
             if (rc) return rc;
         }
@@ -1158,7 +1323,7 @@ struct SlotRun {
         if (mixed) CUDA_OR_RETURN(w.v3.ensure(sizeof(float) * vec));
         {
             const MarchCfg &mc = sizeof(T) == 4 ? G->v32[G->sel32] : G->m64;
-            fused = !generic && o.precond != EQD_PRECOND_JACOBI && (o.flags & EQD_FLAG_FUSE) && mc.smem_af > 0;
+            fused = !resident && !generic && o.precond != EQD_PRECOND_JACOBI && (o.flags & EQD_FLAG_FUSE) && mc.smem_af > 0;
         }
         if (fused) CUDA_OR_RETURN(w.v4.ensure(sizeof(T) * vec));
         else w.v4.release();
@@ -1220,7 +1385,8 @@ struct SlotRun {
         // workspace pointer (a buffer that grew or was released since the
         // capture must not be reached through the old graph).
         std::vector<uint64_t> kv = {(uint64_t)cap, (uint64_t)o.precision, (uint64_t)generic, (uint64_t)G->sel32,
-                                    (uint64_t)o.precond, (uint64_t)split, (uint64_t)sp.itmax, (uint64_t)fused};
+                                    (uint64_t)o.precond, (uint64_t)split, (uint64_t)sp.itmax, (uint64_t)fused, (uint64_t)resident,
+                                    (uint64_t)(kmax * 16 + rounds)};
         for (double d : {sp.rtol, sp.atol, sp.delta}) {
             uint64_t b;
             std::memcpy(&b, &d, sizeof(b));
@@ -1235,7 +1401,8 @@ struct SlotRun {
             w.graph = nullptr;
             cudaGraph_t g;
             CUDA_OR_RETURN(cudaStreamBeginCapture(G->stream, cudaStreamCaptureModeThreadLocal));
-            record_iterations<T>(G, w, cap, mixed, generic, fused, sp, st, kIter, split);
+            if (resident) record_resident<T>(G, w, cap, mixed, sp, st, kmax, rounds);
+            else record_iterations<T>(G, w, cap, mixed, generic, fused, sp, st, kIter, split);
             cudaError_t ce = cudaStreamEndCapture(G->stream, &g);
             if (ce != cudaSuccess) return fail(EQD_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(ce));
             ce = cudaGraphInstantiate(&w.graph, g, cudaGraphInstantiateFlagUseNodePriority);
@@ -1337,6 +1504,10 @@ struct SlotRun {
             cg_true_residual_kernel<<<sb, 128, 0, G->stream>>>(st, sp2, w.res_part.as<double>(), cap, 0, mask);
             launches += 2;
         }
+        if (resident) {  // the kernel forms the first direction, p = r + 0 p
+            CUDA_OR_RETURN(cudaGetLastError());
+            return EQD_OK;
+        }
         const T *dinvT = !sp.precond ? nullptr
                                      : (const T *)(sizeof(T) == 4 ? (const void *)G->dinv32.p : (const void *)G->dinv64.p);
         cg_pupdate_kernel<T><<<nb, 256, 0, G->stream>>>(w.v1.as<T>(), w.v0.as<T>(), st, sp, mask, dinvT, cap);
@@ -1354,7 +1525,8 @@ struct SlotRun {
         for (int s = 0; s < cap; ++s) running += tag[s] >= 0 && hst[s] == COL_ACTIVE;
         if (running > 0) {
             CUDA_OR_RETURN(cudaGraphLaunch(w.graph, G->stream));
-            launches += (int64_t)kIter * ((mixed ? 7 : 4) - (fused ? 1 : 0)) * (w.graph_split ? 2 : 1);
+            if (resident) launches += (int64_t)rounds * (mixed ? 4 : 1);
+            else launches += (int64_t)kIter * ((mixed ? 7 : 4) - (fused ? 1 : 0)) * (w.graph_split ? 2 : 1);
         }
         CUDA_OR_RETURN(cudaMemcpyAsync(hst.data(), w.status.p, cap, cudaMemcpyDeviceToHost, G->stream));
         CUDA_OR_RETURN(cudaMemcpyAsync(hit.data(), w.iters.p, sizeof(int) * cap, cudaMemcpyDeviceToHost, G->stream));
@@ -1377,7 +1549,7 @@ struct SlotRun {
         bool forced = false;
         for (int s = 0; s < cap; ++s) {
             if (tag[s] < 0) continue;
-            if (hst[s] == COL_ACTIVE && hit[s] > itmax + 2 * kIter) {  // defensive: the kernels stop at itmax
+            if (hst[s] == COL_ACTIVE && hit[s] > itmax + 2 * std::max(kIter, resident ? kmax * rounds : 0)) {  // defensive: the kernels stop at itmax
                 hst[s] = COL_MAXITER;
                 forced = true;
             }
@@ -1444,7 +1616,7 @@ struct SlotRun {
 // that packs more stencil CTAs per SM can leave less room for the other
 // half's vector kernels (measured at h = 50 m: the fastest stencil alone was
 // not the fastest iteration).
-static int tune_by_iterations(eqd_grid *G, const eqd_solve_opts &o, int ncols) {
+static int tune_by_iterations(eqd_grid *G, const eqd_solve_opts &o, int ncols, bool with_resident) {
     const GridConst &gc = G->gc;
     ncols = std::max(1, std::min(ncols, 2 * gc.nf));
     std::vector<ColWork> work(ncols);
@@ -1458,10 +1630,23 @@ static int tune_by_iterations(eqd_grid *G, const eqd_solve_opts &o, int ncols) {
     G->tuned = true;  // the slot engines below must not tune again
     double best = 1e30;
     int bestv = G->sel32;
-    for (int v = 0; v < kNumVariants; ++v) {
-        G->sel32 = v;
+    const int pin0 = G->pin;
+    struct PinGuard {
+        eqd_grid *G;
+        int v;
+        ~PinGuard() { G->pin = v; }
+    } guard{G, pin0};
+    if (with_resident && ot.precond != EQD_PRECOND_JACOBI) {
+        int rc = ensure_resident<float>(G, G->res32);
+        if (rc) return rc;
+    }
+    G->tune_ms[kResidentVariant] = 0.0;
+    const bool res = with_resident && ot.precond != EQD_PRECOND_JACOBI && G->res32.ok;
+    for (int v = 0; v < kNumVariants + (res ? 1 : 0); ++v) {
+        G->pin = v;
+        if (v < kNumVariants) G->sel32 = v;
         SlotRun<float> R;
-        int rc = R.setup(G, ot, ncols, false, false);
+        int rc = R.setup(G, ot, ncols, false, false, true);
         if (rc) return rc;
         int taken = 0;
         rc = R.admit(work.data(), ncols, taken);
@@ -1481,7 +1666,9 @@ static int tune_by_iterations(eqd_grid *G, const eqd_solve_opts &o, int ncols) {
             bestv = v;
         }
     }
-    G->sel32 = bestv;
+    // The streamed variant for what does not run resident, then the choice.
+    G->sel32 = (int)(std::min_element(G->tune_ms, G->tune_ms + kNumVariants) - G->tune_ms);
+    if (with_resident) guard.v = bestv;
     return check_device_error(G);
 }
 
@@ -1613,23 +1800,30 @@ static int run_batch_any(eqd_grid *G, const eqd_solve_opts *opts, const BatchSpe
         return fail(EQD_ERR_ARG, "precond must be :none or :jacobi");
     if (o.precision != EQD_PREC_FP64 && o.precision != EQD_PREC_MIXED) return fail(EQD_ERR_ARG, "unknown precision");
     if (B.rhs && o.precision != EQD_PREC_FP64) return fail(EQD_ERR_UNSUPPORTED, "explicit-RHS solves run in FP64");
-    if (o.variant < 0 || o.variant > kNumVariants)
-        return fail(EQD_ERR_ARG, "variant must be 0 (the grid's) or 1.." + std::to_string(kNumVariants));
+    if (o.variant < 0 || o.variant > kNumVariants + 1)
+        return fail(EQD_ERR_ARG, "variant must be 0 (the grid's) or 1.." + std::to_string(kNumVariants + 1));
     const auto t0 = std::chrono::steady_clock::now();
     std::lock_guard<std::mutex> lk(G->mtx);
     if (G->served) return fail(EQD_ERR_ARG, "the grid is attached to a server");
     CUDA_OR_RETURN(cudaSetDevice(G->desc.device));
     // A per-call variant replaces the grid's selection for this call only.
     const int sel_before = G->sel32;
+    const int pin_before = G->pin;
     const bool tuned_before = G->tuned;
     if (o.variant > 0) {
-        G->sel32 = o.variant - 1;
-        G->tuned = true;
+        G->pin = o.variant - 1;
+        if (G->pin != kResidentVariant) {
+            G->sel32 = G->pin;
+            G->tuned = true;
+        }
     }
     int rc = o.precision == EQD_PREC_MIXED ? run_batch<float>(G, o, B, stats) : run_batch<double>(G, o, B, stats);
     if (o.variant > 0) {
-        G->sel32 = sel_before;
-        G->tuned = tuned_before;
+        G->pin = pin_before;
+        if (o.variant - 1 != kResidentVariant) {
+            G->sel32 = sel_before;
+            G->tuned = tuned_before;
+        }
     }
     if (stats)
         stats->seconds += std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
@@ -1831,11 +2025,14 @@ extern "C" int eqd_autotune(eqd_grid *G, int32_t ncols, int32_t *selected, doubl
     if (ncols > 0) {
         eqd_solve_opts o;
         eqd_default_opts(&o);
-        int rc = tune_by_iterations(G, o, ncols);
+        int rc = tune_by_iterations(G, o, ncols, true);
         if (rc) return rc;
     }
-    if (selected) *selected = G->sel32;
-    if (nvariants) *nvariants = kNumVariants;
+    if (selected) *selected = G->pin >= 0 ? G->pin : G->sel32;
+    if (nvariants) *nvariants = kNumVariants + 1;
+    if (ms_per_variant) ms_per_variant[kResidentVariant] = G->tune_ms[kResidentVariant];
+    if (tile_rows) tile_rows[kResidentVariant] = 0;
+    if (threads) threads[kResidentVariant] = G->res32.ok ? 64 * G->res32.d.nch0max : 0;
     for (int v = 0; v < kNumVariants; ++v) {
         if (ms_per_variant) ms_per_variant[v] = G->tune_ms[v];
         if (tile_rows) tile_rows[v] = G->v32[v].g.t2max;
@@ -1875,7 +2072,7 @@ extern "C" int eqd_tune_chunk(eqd_grid *G, const int32_t *widths, int32_t nwidth
             work[i].tag = i;
         }
         SlotRun<float> R;
-        rc = R.setup(G, o, w, false, false);
+        rc = R.setup(G, o, w, false, false, true);
         if (rc) return rc;
         int taken = 0;
         rc = R.admit(work.data(), w, taken);
@@ -1903,11 +2100,14 @@ extern "C" int eqd_tune_chunk(eqd_grid *G, const int32_t *widths, int32_t nwidth
 }
 
 extern "C" int eqd_set_variant(eqd_grid *G, int32_t variant) {
-    if (!G || variant < 0 || variant >= kNumVariants) return fail(EQD_ERR_ARG, "invalid variant");
+    if (!G || variant < 0 || variant > kResidentVariant) return fail(EQD_ERR_ARG, "invalid variant");
     std::lock_guard<std::mutex> lk(G->mtx);
     if (G->served) return fail(EQD_ERR_ARG, "the grid is attached to a server");
-    G->sel32 = variant;
-    G->tuned = true;
+    G->pin = variant;
+    if (variant != kResidentVariant) {
+        G->sel32 = variant;
+        G->tuned = true;
+    }
     return EQD_OK;
 }
 

@@ -1,0 +1,566 @@
+// Resident CG: many iterations of one column's CG inside one launch, the
+// column's vectors held on chip by a cluster of CTAs.
+//
+// The streamed iteration moves a column's vectors eleven times through HBM
+// and pays four to seven launches; on a small grid neither the march's few
+// CTAs nor the launches fill the device (one column at h = 50 m: 98 us an
+// iteration, 60 us of it the three-CTA apply). Here a cluster of M CTAs owns
+// one column: p (with its halo) and two of the three stress sums F live in
+// shared memory, r, the solution and q in registers, so an iteration touches
+// no global memory; a line's new p is stored straight into the shared memory
+// of the CTAs that have it in their halo, dot products are exchanged the same
+// way, and two cluster barriers order an iteration. The kernel ends when the
+// column needs its FP64 true residual (mixed precision), is done (FP64), or
+// has run kmax iterations.
+//
+// Operator (plane_march.cuh has the reference citations), per side:
+//   G_k = D1_k v_k,  F_j = lam G_j + (lam + mu) sum_{k != j} G_k,
+//   w_j = mu (sum_a D2_a + D2_j) v_j + D1_j F_j,
+// which needs only five-point (closure: six-point) rows; w then gets the SAT
+// terms at x = 0, P and -H.
+//
+// A thread owns half a line (x1 points of one node and side): its x1
+// derivatives come from registers with coefficients from the kernel's
+// parameters (n1 is compiled in, so every closure row is straight code), and
+// the two sides of a line sit in adjacent lanes, so a fault node's sides
+// exchange by one shuffle. The x2 and x3 rows take their coefficients and the
+// places of their outer points from a table by the line's row class: interior
+// and closure rows run the same code, with the same number of loads. All that
+// reads p is done in one pass (F and the second derivatives share loads); the
+// F terms follow after a barrier.
+// Whole lines per thread left an SM four warps (19 k clocks an iteration at
+// 17 x 17 x 9 on four CTAs, against 11 k); one component of a line per thread
+// gave it 24 but 34 % more instructions.
+//
+// What bounds it: latency at 16 warps an SM (the two cluster barriers, the
+// stores to the neighbours, the FP64 reduction), then shared-memory wavefronts
+// (about 45 a point). Measured against the streamed iteration: one column at
+// h = 50 m 15 us an iteration (was 98), one slip's traction 2.3 ms (14.5), the
+// ten Toeplitz columns 3.5 ms (15.7), three columns at h = 100 m 1.7 ms (8.5),
+// all 578 there 12.6 ms (34), all 2,178 at h = 50 m 217 ms (300).
+//
+// The order of every sum is fixed by the plan, which depends on the grid and
+// the precision only: a column gives the same bits alone and in any batch.
+#pragma once
+#include "resident_plan.h"
+#include "solver_kernels.cuh"
+
+namespace eqd {
+
+template <typename T>
+struct ResCoef {
+    T lam, lpm, sat, mu, mu2;        // mu2 = 2 mu
+    T dlo[4];                        // boundary derivative
+};
+
+struct ResTables {
+    const ResRank *ranks;
+    const int *chunks;
+    const ResLine *lines;
+    const int *gofs;
+    const int *push;
+    const void *tab;  // fill_res_tables rows, T
+    const int *off;
+};
+
+template <typename T>
+__host__ __device__ __forceinline__ void res_load4(const T *t, T (&c)[4]) {
+#ifdef __CUDA_ARCH__
+    if constexpr (sizeof(T) == 4) {
+        const float4 v = *reinterpret_cast<const float4 *>(t);
+        c[0] = v.x, c[1] = v.y, c[2] = v.z, c[3] = v.w;
+    } else {
+        const double2 v = reinterpret_cast<const double2 *>(t)[0], w = reinterpret_cast<const double2 *>(t)[1];
+        c[0] = v.x, c[1] = v.y, c[2] = w.x, c[3] = w.y;
+    }
+#else
+    for (int k = 0; k < 4; ++k) c[k] = t[k];
+#endif
+}
+
+// The rows of one line on one axis: fill_res_tables' layout.
+template <typename T>
+struct ResLineRow {
+    const T *t;
+    const int *o;
+};
+
+// Row x of an x1 operator on a line held in registers (zero entries skipped).
+template <bool SECOND, int N1, typename T>
+__host__ __device__ __forceinline__ T res_x1_dot(const T (&c)[N1][6], const T (&l)[N1], int x) {
+    T s = T(0);
+    bool any = false;
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+        if (!res_nz(SECOND, x, N1, k)) continue;
+        const T t = l[res_start(x, N1) + k];
+        s = any ? s + c[x][k] * t : c[x][k] * t;
+        any = true;
+    }
+    return s;
+}
+
+// The first derivatives at the points [XA, XB) of a line whose p starts at v
+// (side included). put(x, G1, G2, G3).
+template <typename T, int N1, typename G, int XA, int XB, typename PUT>
+__host__ __device__ __forceinline__ void res_line_grad(const ResX1<T, N1> &X, const T *v, T sgn, ResLineRow<T> row2,
+                                                        ResLineRow<T> row3, PUT put) {
+    constexpr int LO = res_start(XA, N1), HI = res_start(XB - 1, N1) + 6;
+    T l[N1];
+#pragma unroll
+    for (int x = 0; x < N1; ++x) l[x] = x >= LO && x < HI && x < N1 - 1 ? v[x * G::PSZ] : T(0);  // p is 0 at N1 - 1
+    T c2[4], c3[4];
+    res_load4(row2.t, c2);
+    res_load4(row3.t, c3);
+    int o2[4], o3[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        o2[k] = row2.o[k] + G::CS;
+        o3[k] = row3.o[k] * G::R2 + 2 * G::CS;
+    }
+#pragma unroll
+    for (int x = XA; x < XB; ++x) {
+        const T G1 = sgn * res_x1_dot<false>(X.c1, l, x);
+        T G2 = T(0), G3 = T(0);
+        if (x < N1 - 1) {
+            const T *vx = v + x * G::PSZ;
+            G2 = c2[0] * vx[o2[0]];
+            G3 = c3[0] * vx[o3[0]];
+#pragma unroll
+            for (int k = 1; k < 4; ++k) {
+                G2 += c2[k] * vx[o2[k]];
+                G3 += c3[k] * vx[o3[k]];
+            }
+        }
+        put(x, G1, G2, G3);
+    }
+}
+
+// All that an own line's points [XA, XB) need of p: F there (putf(x, F1, F2,
+// F3); x = N1-1 has F1 only), the second derivatives w, the points' p itself,
+// and, where the points start at the fault, the traction on the fixed +x1 axis
+// there. v: the line's p, component 1.
+template <typename T, int N1, typename G, int XA, int XB, typename PUTF>
+__host__ __device__ __forceinline__ void res_own_p(const ResCoef<T> &C, const ResX1<T, N1> &X, const T *v, T sgn,
+                                                   ResLineRow<T> row2, ResLineRow<T> row3, T (&w)[XB - XA][3],
+                                                   T (&pv)[XB - XA][3], T (&tau)[3], PUTF putf) {
+    constexpr int XE = XB == N1 - 1 ? N1 : XB;  // the last half also has F1 at the far field
+    constexpr int LO = res_start(XA, N1), HI = res_start(XE - 1, N1) + 6;
+    const int oa2 = row2.o[0], ob2 = row2.o[3], oa3 = row3.o[0] * G::R2, ob3 = row3.o[3] * G::R2;
+    T c2[4], c3[4], s2[4], s3[4];  // D1; mu D2: outer, -1, own, +1, and the other outer
+    res_load4(row2.t, c2);
+    res_load4(row3.t, c3);
+    res_load4(row2.t + 4, s2);
+    res_load4(row3.t + 4, s3);
+    const T s24 = row2.t[8], s34 = row3.t[8];
+    T G1[XE - XA], G2[XB - XA], G3[XB - XA], dh[3], d2 = T(0), d3 = T(0);
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+        const T *u = v + j * G::CS;
+        T l[N1];
+#pragma unroll
+        for (int x = 0; x < N1; ++x) l[x] = x >= LO && x < HI && x < N1 - 1 ? u[x * G::PSZ] : T(0);  // p is 0 at N1 - 1
+#pragma unroll
+        for (int x = XA; x < XB; ++x) {
+            const T *ux = u + x * G::PSZ;
+            const T a2 = ux[oa2], m2 = ux[-1], p2 = ux[1], b2 = ux[ob2];
+            const T a3 = ux[oa3], m3 = ux[-G::R2], p3 = ux[G::R2], b3 = ux[ob3];
+            const T x1 = res_x1_dot<true>(X.c2, l, x);
+            const T x2 = s2[0] * a2 + s2[1] * m2 + s2[2] * l[x] + s2[3] * p2 + s24 * b2;
+            const T x3 = s3[0] * a3 + s3[1] * m3 + s3[2] * l[x] + s3[3] * p3 + s34 * b3;
+            w[x - XA][j] = (j == 0 ? x1 + x1 : x1) + (j == 1 ? x2 + x2 : x2) + (j == 2 ? x3 + x3 : x3);
+            pv[x - XA][j] = l[x];
+            if (j == 1) G2[x - XA] = c2[0] * a2 + c2[1] * m2 + c2[2] * p2 + c2[3] * b2;
+            if (j == 2) G3[x - XA] = c3[0] * a3 + c3[1] * m3 + c3[2] * p3 + c3[3] * b3;
+            if (j == 0 && x == 0) {
+                d2 = c2[0] * a2 + c2[1] * m2 + c2[2] * p2 + c2[3] * b2;
+                d3 = c3[0] * a3 + c3[1] * m3 + c3[2] * p3 + c3[3] * b3;
+            }
+        }
+        if (j == 0) {
+#pragma unroll
+            for (int x = XA; x < XE; ++x) G1[x - XA] = sgn * res_x1_dot<false>(X.c1, l, x);
+        }
+        if (XA == 0) {
+            T s = C.dlo[0] * l[0];
+#pragma unroll
+            for (int k = 1; k < 4; ++k) s += C.dlo[k] * l[k];
+            dh[j] = sgn * s;
+        }
+    }
+#pragma unroll
+    for (int x = XA; x < XE; ++x) {
+        const T g1 = G1[x - XA], g2 = x < XB ? G2[x < XB ? x - XA : 0] : T(0), g3 = x < XB ? G3[x < XB ? x - XA : 0] : T(0);
+        putf(x, C.lam * g1 + C.lpm * (g2 + g3), C.lam * g2 + C.lpm * (g1 + g3), C.lam * g3 + C.lpm * (g1 + g2));
+    }
+    if (XA == 0) {
+        tau[0] = C.lam * (G1[0] + G2[0] + G3[0]) + C.mu2 * dh[0];
+        tau[1] = C.mu * (d2 + dh[1]);
+        tau[2] = C.mu * (d3 + dh[2]);
+    }
+}
+
+// The F terms of w at the points [XA, XB) of an own line. f1: the line's F1
+// (stride f1s); f2, f3: its places in F2 and F3 (side included).
+template <typename T, int N1, typename G, int XA, int XB>
+__host__ __device__ __forceinline__ void res_own_f(const ResX1<T, N1> &X, const T *f1, int f1s, const T *f2,
+                                                   const T *f3, T sgn, ResLineRow<T> row2, ResLineRow<T> row3,
+                                                   T (&w)[XB - XA][3]) {
+    constexpr int LO = res_start(XA, N1), HI = res_start(XB - 1, N1) + 6;
+    const int oa2 = row2.o[0], ob2 = row2.o[3], oa3 = row3.o[0] * G::R2b, ob3 = row3.o[3] * G::R2b;
+    T c2[4], c3[4];
+    res_load4(row2.t, c2);
+    res_load4(row3.t, c3);
+    T l[N1];
+#pragma unroll
+    for (int x = 0; x < N1; ++x) l[x] = x >= LO && x < HI ? f1[x * f1s] : T(0);
+#pragma unroll
+    for (int x = XA; x < XB; ++x) {
+        const T *g2 = f2 + x * G::PSa, *g3 = f3 + x * G::PSb;
+        T(&o)[3] = w[x - XA];
+        o[0] += sgn * res_x1_dot<false>(X.c1, l, x);
+        o[1] += c2[0] * g2[oa2] + c2[1] * g2[-1] + c2[2] * g2[1] + c2[3] * g2[ob2];
+        o[2] += c3[0] * g3[oa3] + c3[1] * g3[-G::R2b] + c3[2] * g3[G::R2b] + c3[3] * g3[ob3];
+    }
+}
+
+template <typename T>
+inline ResCoef<T> res_coef(double h1, double lam, double mu, double sat) {
+    ResCoef<T> C{};
+    C.lam = (T)lam;
+    C.lpm = (T)(lam + mu);
+    C.sat = (T)sat;
+    C.mu = (T)mu;
+    C.mu2 = (T)(2 * mu);
+    for (int k = 0; k < 4; ++k) C.dlo[k] = (T)(kDb[k].v() / h1);
+    return C;
+}
+
+// ---------------------------------------------------------------------------
+// Cluster primitives
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ int cluster_rank() {
+    unsigned r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return (int)r;
+}
+
+// All threads of all CTAs of the cluster; orders their shared-memory writes
+// before what follows.
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// The same place in the shared memory of the cluster's CTA `rank`.
+template <typename T>
+__device__ __forceinline__ T *map_cluster(T *p, int rank) {
+    unsigned long long a;
+    asm("mapa.u64 %0, %1, %2;" : "=l"(a) : "l"(reinterpret_cast<unsigned long long>(p)), "r"(rank));
+    return reinterpret_cast<T *>(a);
+}
+
+// Threads of an instance at most: 512 x 128 registers, or 256 x 255 where half
+// a line's state needs them.
+template <typename T, int N1>
+constexpr int res_max_threads() {
+    return sizeof(T) == 4 && N1 <= 11 ? 32 * kResMaxWarps : 16 * kResMaxWarps;
+}
+
+// ---------------------------------------------------------------------------
+// One column per cluster of d.M CTAs (grid: ncols * d.M CTAs, 64 d.nch0max
+// threads each). x: the FP32 correction of mixed precision, or the FP64
+// solution. On entry the direction is p = r + beta p.
+// ---------------------------------------------------------------------------
+template <typename T, int N1, int T2, int T3>
+__global__ void __launch_bounds__(res_max_threads<T, N1>(), 1)
+resident_cg_kernel(const __grid_constant__ ResCoef<T> C, const __grid_constant__ ResX1<T, N1> X,
+                   const __grid_constant__ ResDims d, ResTables tb, T *__restrict__ x_, T *__restrict__ r_,
+                   T *__restrict__ p_, ColState st, SolveParams sp, int mixed, int kmax) {
+    using G = ResGeo<(int)sizeof(T), N1, T2, T3>;
+    static_assert(N1 % 2 == 1, "the two halves of a line have the same number of points");
+    constexpr int NX = N1 - 1, XH = NX / 2;  // p is zero at the far field x = N1 - 1
+    const int M = d.M;
+    const int slot = blockIdx.x / M;
+    if (st.status[slot] != COL_ACTIVE) return;  // the whole cluster: no barrier has been reached
+    const int rank = M > 1 ? cluster_rank() : 0;
+    const ResRank R = tb.ranks[rank];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nthr = blockDim.x, nwarp = nthr >> 5;
+
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    T *p = reinterpret_cast<T *>(smem_raw);
+    T *F1 = reinterpret_cast<T *>(smem_raw + G::oF1);
+    T *F2 = reinterpret_cast<T *>(smem_raw + G::oF2);
+    T *F3 = reinterpret_cast<T *>(smem_raw + G::oF3);
+    T *tab = reinterpret_cast<T *>(smem_raw + G::oTab);  // x2 row classes, then x3
+    int *off = reinterpret_cast<int *>(smem_raw + G::oOff);
+    double *red = reinterpret_cast<double *>(smem_raw + G::oRed);  // [rank][8], [warp][8], then alpha, beta, stop
+    double *wred = red + kResMaxTeam * 8;
+    volatile double *step = wred + kResMaxWarps * 8;
+    ResLine *lines = reinterpret_cast<ResLine *>(smem_raw + G::oLine);
+    int *chunks = reinterpret_cast<int *>(smem_raw + G::oChunk);
+    int *push = reinterpret_cast<int *>(smem_raw + G::oPush);
+
+    // Tables, and zeros everywhere else (the far-field entries of p stay zero).
+    for (int i = tid; i < G::oTab / (int)sizeof(T); i += nthr) p[i] = T(0);
+    for (int i = tid; i < 18 * kResRow; i += nthr) tab[i] = static_cast<const T *>(tb.tab)[i];
+    for (int i = tid; i < 18 * 4; i += nthr) off[i] = tb.off[i];
+    for (int i = tid; i < R.nch * kResLinesPerChunk; i += nthr)
+        lines[i] = tb.lines[R.chunk0 * kResLinesPerChunk + i];
+    for (int i = tid; i < R.nch; i += nthr) chunks[i] = tb.chunks[R.chunk0 + i];
+    for (int i = tid; i < R.nch0 * kResLinesPerChunk * d.npush; i += nthr) push[i] = tb.push[R.push0 * d.npush + i];
+    for (int i = tid; i < (kResMaxTeam + kResMaxWarps + 1) * 8; i += nthr) red[i] = 0.0;
+    __syncthreads();
+
+    // This thread's half line: warps 2c and 2c + 1 have the CTA's own chunk c.
+    const int side = lane & 1, sub = lane >> 1, chunk = warp >> 1, half = warp & 1;
+    const T sgn = side ? T(1) : T(-1);
+    const bool has = chunk < R.nch0;
+    ResLine L{};
+    if (has) L = lines[chunk * kResLinesPerChunk + sub];
+    const bool own = has && (L.info >> 8 & 1);
+    auto rows = [&](int cls) { return ResLineRow<T>{tab + cls * kResRow, off + cls * 4}; };
+    const ResLineRow<T> row2 = rows(L.info & 15), row3 = rows(9 + (L.info >> 4 & 15));
+    T *const line = p + side * G::SS + L.plo;
+    T *const mine = line + half * XH * G::PSZ;  // the own points of p
+    T *const f1 = F1 + chunk * 32 + lane, *const f2 = F2 + side * G::SSa + L.f2, *const f3 = F3 + side * G::SSb + L.f3;
+    const int f1s = R.nch0 * 32;
+    const T hw23 = own ? row2.t[9] * row3.t[9] : T(0);
+    const int cstr = d.n3 * d.PS, gstep = side ? 1 : -1;
+    const long long g0 = (long long)slot * d.colstride + 3LL * side * cstr +
+                         (own ? tb.gofs[(R.chunk0 + chunk) * kResLinesPerChunk + sub] : 0) +
+                         (side ? half * XH : NX - half * XH);
+
+    T r[XH][3], xs[XH][3];
+    double gamma = 0.0;
+    double beta = st.beta[slot];
+    const double tol = st.tol[slot], rr_ref = mixed ? st.rr_ref[slot] : 0.0;
+    const long long itmax = sp.itmax > 0 ? sp.itmax : 2 * sp.ntot;
+    int iters = st.iters[slot];
+
+    // The new p of the own points: into its own place and into the halo of
+    // every CTA that reads it. Those CTAs have left their last read of the
+    // old value (the exchange of the dot products, or the barrier below).
+    auto put_p = [&](const T (&v)[XH][3]) {
+        if (!own) return;
+#pragma unroll
+        for (int x = 0; x < XH; ++x)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) mine[x * G::PSZ + c * G::CS] = v[x][c];
+        const int *to = push + (chunk * kResLinesPerChunk + sub) * d.npush;
+        for (int k = 0; k < d.npush; ++k) {
+            const int w = to[k];
+            if (w == -1) continue;
+            T *q = map_cluster(p + side * G::SS + half * XH * G::PSZ, (int)((unsigned)w >> 28)) + (w & 0xffffff);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                if (!(w >> (24 + c) & 1)) continue;
+#pragma unroll
+                for (int x = 0; x < XH; ++x) q[x * G::PSZ + c * G::CS] = v[x][c];
+            }
+        }
+    };
+
+    if (M > 1) cluster_barrier();  // every CTA's p is zeroed before its neighbours store into it
+    {
+        const T b = (T)beta;
+        T v[XH][3];
+#pragma unroll
+        for (int x = 0; x < XH; ++x)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const long long g = g0 + c * (long long)cstr + x * gstep;
+                r[x][c] = own ? r_[g] : T(0);
+                xs[x][c] = own ? x_[g] : T(0);
+                v[x][c] = own ? r[x][c] + b * p_[g] : T(0);
+            }
+        put_p(v);
+    }
+
+    int status = COL_ACTIVE, flag = 0;
+    for (int k = 0;; ++k) {
+        if (M > 1) cluster_barrier();  // every CTA has its new p, halo included
+        else __syncthreads();
+
+        // ---- all that reads p: F = lam G_j + (lam + mu) sum_{k != j} G_k, and
+        // the second derivatives at the own points ---------------------------
+        T q[XH][3], pv[XH][3], tau[3];
+        if (has) {
+            auto putf = [&](int x, T a, T b, T c) {
+                f1[x * f1s] = a;
+                if (x < NX) {
+                    f2[x * G::PSa] = b;
+                    f3[x * G::PSb] = c;
+                }
+            };
+            if (half) res_own_p<T, N1, G, XH, NX>(C, X, line, sgn, row2, row3, q, pv, tau, putf);
+            else res_own_p<T, N1, G, 0, XH>(C, X, line, sgn, row2, row3, q, pv, tau, putf);
+        }
+        // Halo rows: F2 two rows beyond the tile along x2, F3 along x3.
+        for (int u = warp; u < 2 * (R.nch - R.nch0); u += nwarp) {
+            const int ch = R.nch0 + (u >> 1);
+            const bool two = chunks[ch] == 1;
+            const ResLine H = lines[ch * kResLinesPerChunk + sub];
+            const T *v = p + side * G::SS + H.plo;
+            T *f = two ? F2 + side * G::SSa + H.f2 : F3 + side * G::SSb + H.f3;
+            const int fs = two ? G::PSa : G::PSb;
+            auto put = [&](int x, T G1, T G2, T G3) {
+                f[x * fs] = two ? C.lam * G2 + C.lpm * (G1 + G3) : C.lam * G3 + C.lpm * (G1 + G2);
+            };
+            const ResLineRow<T> h2 = rows(H.info & 15), h3 = rows(9 + (H.info >> 4 & 15));
+            if (u & 1) res_line_grad<T, N1, G, XH, NX>(X, v, sgn, h2, h3, put);
+            else res_line_grad<T, N1, G, 0, XH>(X, v, sgn, h2, h3, put);
+        }
+        __syncthreads();
+
+        // ---- q = A p on the own points, and the dot products -----------------
+        double sums[5] = {0.0, 0.0, 0.0, 0.0, 0.0};  // p.q, p.p, r.q, q.q, r.r
+        if (has) {
+            if (half) {
+                res_own_f<T, N1, G, XH, NX>(X, f1, f1s, f2, f3, sgn, row2, row3, q);
+            } else {
+                res_own_f<T, N1, G, 0, XH>(X, f1, f1s, f2, f3, sgn, row2, row3, q);
+                // SAT c (tau+ - tau-) on both sides, then P averages the fault node.
+#pragma unroll
+                for (int j = 0; j < 3; ++j) {
+                    q[0][j] += C.sat * sgn * (tau[j] - __shfl_xor_sync(0xffffffffu, tau[j], 1));
+                    q[0][j] = T(0.5) * (q[0][j] + __shfl_xor_sync(0xffffffffu, q[0][j], 1));
+                }
+            }
+#pragma unroll
+            for (int x = 0; x < XH; ++x) {
+                const T hw = (half ? X.hx[XH + x] : X.hx[x]) * hw23;
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    q[x][c] *= hw;
+                    const double qd = (double)q[x][c], pd = own ? (double)pv[x][c] : 0.0;
+                    const double rd = (double)r[x][c];
+                    sums[0] += pd * qd;
+                    sums[1] += pd * pd;
+                    sums[2] += rd * qd;
+                    sums[3] += qd * qd;
+                    sums[4] += rd * rd;
+                }
+            }
+        }
+        // Sums of the warp: halving exchanges leave sum `lane >> 2` in each
+        // group of four lanes (5 to 7: none); then the CTA's, by warp 0, to
+        // every CTA.
+        const int sum = lane >> 2, part = lane & 3;
+        double h4[4], h2[2], c1;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const double lo = sums[j], hi = j == 0 ? sums[4] : 0.0;
+            h4[j] = ((lane & 16) ? hi : lo) + __shfl_xor_sync(0xffffffffu, (lane & 16) ? lo : hi, 16);
+        }
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+            h2[j] = ((lane & 8) ? h4[j + 2] : h4[j]) + __shfl_xor_sync(0xffffffffu, (lane & 8) ? h4[j] : h4[j + 2], 8);
+        c1 = ((lane & 4) ? h2[1] : h2[0]) + __shfl_xor_sync(0xffffffffu, (lane & 4) ? h2[0] : h2[1], 4);
+        c1 += __shfl_xor_sync(0xffffffffu, c1, 2);
+        c1 += __shfl_xor_sync(0xffffffffu, c1, 1);
+        if (part == 0) wred[warp * 8 + sum] = c1;
+        __syncthreads();
+        if (warp == 0) {
+            c1 = wred[part * 8 + sum];
+#pragma unroll
+            for (int w = 4; w < kResMaxWarps; w += 4) c1 += wred[(part + w) * 8 + sum];  // absent warps hold zero
+            c1 += __shfl_xor_sync(0xffffffffu, c1, 2);
+            c1 += __shfl_xor_sync(0xffffffffu, c1, 1);
+            if (M > 1) {
+                double *to = red + rank * 8 + sum;
+#pragma unroll
+                for (int w = 0; w < kResMaxTeam; w += 4)
+                    if (part + w < M) *map_cluster(to, part + w) = c1;
+            } else if (part == 0) {
+                red[sum] = c1;
+            }
+        }
+        if (M > 1) cluster_barrier();
+        else __syncthreads();
+
+        // ---- alpha, beta and the decision, by warp 0 of each CTA --------------
+        // The next residual's norm from the same sums, |r - a q|^2 =
+        // |r|^2 - 2 a r.q + a^2 q.q: no second exchange. |r|^2 is summed anew
+        // each time, so its rounding does not build up.
+        if (warp == 0) {
+            c1 = red[part * 8 + sum];
+#pragma unroll
+            for (int w = 4; w < kResMaxTeam; w += 4) c1 += red[(part + w) * 8 + sum];  // ranks beyond M hold zero
+            c1 += __shfl_xor_sync(0xffffffffu, c1, 2);
+            c1 += __shfl_xor_sync(0xffffffffu, c1, 1);
+            const double pq = __shfl_sync(0xffffffffu, c1, 0), pp = __shfl_sync(0xffffffffu, c1, 4),
+                         rq = __shfl_sync(0xffffffffu, c1, 8), qq = __shfl_sync(0xffffffffu, c1, 12);
+            gamma = __shfl_sync(0xffffffffu, c1, 16);
+            double alpha = gamma / pq;
+            const bool breakdown = !(pq > 2.220446049250313e-16 * pp);  // zero or negative curvature
+            if (breakdown || !isfinite(alpha)) alpha = 0.0;
+            const double ad = (double)(T)alpha;
+            const double rr = fmax(gamma - 2.0 * ad * rq + ad * ad * qq, 0.0);
+            ++iters;
+            if (breakdown) {
+                if (mixed) flag = 1;  // let the true residual decide
+                else status = COL_BREAKDOWN;
+            } else if (!isfinite(gamma) || !isfinite(rq) || !isfinite(qq)) {
+                status = COL_NONFINITE;
+            } else if (mixed) {
+                if (rr <= tol * tol || rr <= sp.delta * sp.delta * rr_ref || iters >= itmax) flag = 1;
+            } else if (sqrt(rr) <= tol) {
+                status = COL_CONVERGED;
+            } else if (iters >= itmax) {
+                status = COL_MAXITER;
+            }
+            const bool stop = flag || status != COL_ACTIVE;
+            if (!stop) {
+                beta = rr / gamma;
+            }
+            if (lane == 0) {
+                step[0] = alpha;
+                step[1] = beta;
+                step[2] = stop || k + 1 >= kmax ? 1.0 : 0.0;
+            }
+        }
+        __syncthreads();
+        const T at = (T)step[0], b = (T)step[1];
+        const bool last = step[2] != 0.0;
+        if (has) {
+#pragma unroll
+            for (int x = 0; x < XH; ++x)
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    xs[x][c] += at * pv[x][c];
+                    r[x][c] -= at * q[x][c];
+                }
+        }
+        if (last) break;
+        if (has) {
+#pragma unroll
+            for (int x = 0; x < XH; ++x)
+#pragma unroll
+                for (int c = 0; c < 3; ++c) pv[x][c] = r[x][c] + b * pv[x][c];
+            put_p(pv);
+        }
+    }
+    // Leave the state as the streamed iteration does: p is the last
+    // iteration's direction, beta the next one's factor.
+    if (own) {
+#pragma unroll
+        for (int x = 0; x < XH; ++x)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const long long g = g0 + c * (long long)cstr + x * gstep;
+                x_[g] = xs[x][c];
+                p_[g] = mine[x * G::PSZ + c * G::CS];
+                r_[g] = r[x][c];
+            }
+    }
+    if (rank == 0 && tid == 0) {
+        st.iters[slot] = iters;
+        st.beta[slot] = beta;
+        st.gamma[slot] = gamma;
+        if (mixed) st.flag[slot] = (int8_t)flag;
+        if (status != COL_ACTIVE) st.status[slot] = (int8_t)status;
+    }
+}
+
+}  // namespace eqd

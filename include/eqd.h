@@ -98,9 +98,10 @@ typedef struct {
                                  tuned, else as many as the HBM budget allows */
     double reliable_delta;    /* mixed: FP64 true-residual update when ||r|| drops by this factor (0 -> 0.01) */
     uint64_t hbm_budget_bytes;/* 0 -> free device memory minus 2 GiB */
-    int32_t variant;          /* FP32 stencil launch variant for this call: 0 -> the grid's (chosen by
-                                 eqd_autotune on first use, or pinned by eqd_set_variant); k > 0 ->
-                                 variant k - 1 of eqd_autotune's list, for this call only */
+    int32_t variant;          /* launch variant for this call: 0 -> the grid's (pinned by eqd_set_variant or
+                                 eqd_autotune; else the resident CG where the grid has a plan for it, else
+                                 the streamed variant that the tuner picks on first use); k > 0 -> variant
+                                 k - 1 of eqd_autotune's list, for this call only */
     uint32_t flags;
 } eqd_solve_opts;
 
@@ -185,11 +186,14 @@ int eqd_stiffness_toeplitz(eqd_grid *grid, const eqd_solve_opts *opts, double *K
 int eqd_profile_apply(eqd_grid *grid, int32_t ncols, int32_t precision, int32_t warmup, int32_t reps,
                       double *ms_per_launch, double *bytes_per_launch);
 
-/* Autotuner of the FP32 stencil launch configuration (x2 tile height, CTA
- * size, columns per thread, edge-partitioned tiles): times 20 mixed-precision
- * CG iterations of ncols unit-slip columns (<= 2nf) with every variant, keeps
- * the fastest for this grid (used by every later mixed-precision call) and
- * reports milliseconds per iteration. Arrays hold *nvariants (<= 16) entries.
+/* Autotuner of the CG's launch configuration: variants 0..10 stream the
+ * vectors and differ in the FP32 stencil (x2 tile height, CTA size, columns
+ * per thread, edge-partitioned tiles); variant 11 keeps each column's vectors
+ * on chip in a cluster of CTAs (small and middle grids; where the grid has no
+ * plan for it, it streams). Times 20 mixed-precision CG iterations of ncols
+ * unit-slip columns (<= 2nf) with every variant, keeps the fastest for this
+ * grid (used by every later call) and reports milliseconds per iteration
+ * (0 for variant 11 without a plan). Arrays hold *nvariants (<= 16) entries.
  * ncols = 0 re-tunes nothing: it reports the current selection and the times
  * of the last tuning (zeros if the grid was never tuned). */
 int eqd_autotune(eqd_grid *grid, int32_t ncols, int32_t *selected, double *ms_per_variant, int32_t *tile_rows,
@@ -202,8 +206,9 @@ int eqd_autotune(eqd_grid *grid, int32_t ncols, int32_t *selected, double *ms_pe
 int eqd_tune_chunk(eqd_grid *grid, const int32_t *widths, int32_t nwidths, double *ms_per_column_iteration,
                    int32_t *best);
 
-/* Pins the FP32 stencil launch variant (0 .. *nvariants-1 of eqd_autotune)
- * for this grid instead of autotuning (reproducibility across processes). */
+/* Pins the launch variant (0 .. *nvariants-1 of eqd_autotune) for this grid
+ * instead of choosing it (reproducibility across processes; a streamed variant
+ * also keeps FP64 solves streamed). */
 int eqd_set_variant(eqd_grid *grid, int32_t variant);
 
 /* Failure-path test hook (no counterpart in the reference): the next FP32
