@@ -22,6 +22,7 @@
 #include "rhs_kernels.cuh"
 #include "ring_march.cuh"
 #include "resident_cg.cuh"
+#include "xmarch.cuh"
 
 using namespace eqd;
 
@@ -86,6 +87,8 @@ static constexpr int kMaxT64b = 512;  // FP64 instances for wide x1 lines (n1 = 
 static constexpr int kNumVariants = 11;  // 9 plane-march variants, then 2 ring-march variants
 static constexpr int kFirstRingVariant = 9;
 static constexpr int kResidentVariant = kNumVariants;  // whole iterations resident on chip (resident_cg.cuh)
+static constexpr int kXMarchVariant = kNumVariants + 1;  // streamed, vectors x2-fastest (xmarch.cuh)
+static constexpr int kAllVariants = kNumVariants + 2;
 
 // Ring-march instances per n1: (x2 tile capacity, register cap per thread)
 // of its two variants. A CTA's threads x registers must fit the SM's 65,536,
@@ -363,6 +366,7 @@ struct Workspace {
     cudaGraphExec_t graph = nullptr;
     int graph_iters = 0;
     bool graph_split = false;  // the captured iterations run as two halves
+    CUtensorMap pmap;          // x1 march: the planes of p
     std::vector<uint64_t> graph_key;  // what the captured graph baked in (see SlotRun::setup)
     ~Workspace() {
         if (graph) cudaGraphExecDestroy(graph);
@@ -377,6 +381,16 @@ struct ResEngine {
     int t2 = 0, t3 = 0;  // tile capacity of the kernel instance
     DevBuf ranks, chunks, lines, gofs, push, tab, off;
     ResTables tb{};
+};
+
+// The streamed FP32 iteration on x2-fastest vectors: geometry and tables.
+struct XEngine {
+    bool tried = false, ok = false;
+    XGeom g{};
+    XCoef C{};
+    XLayout lay{};
+    int smem = 0;
+    DevBuf b2, b3, rows, tab, off;
 };
 
 struct eqd_grid {
@@ -400,8 +414,9 @@ struct eqd_grid {
     int pin = -1;          // variant the caller (or eqd_autotune) chose, kResidentVariant included; -1: none,
                            // and solves run resident where the grid has a plan
     ResEngine res32, res64;
+    XEngine xm;
     int chunk_tuned = 0;   // eqd_tune_chunk's choice of columns per batch (0: as many as the budget allows)
-    double tune_ms[kNumVariants + 1] = {};
+    double tune_ms[kAllVariants] = {};
     int nchunks = 1;
     cudaStream_t stream = nullptr;
     cudaStream_t stream2 = nullptr;          // second half of a split batch (graph capture only)
@@ -692,6 +707,114 @@ static cudaError_t launch_resident(eqd_grid *G, const ResEngine &E, T *x, T *r, 
     return e;
 }
 
+// ---------------------------------------------------------------------------
+// x1 march (xmarch.cuh): tiles, tables, tensor map and launch
+// ---------------------------------------------------------------------------
+static int ensure_xmarch(eqd_grid *G) {
+    XEngine &E = G->xm;
+    if (E.tried) return EQD_OK;
+    E.tried = true;
+    const GridConst &gc = G->gc;
+    std::vector<int> b2, b3, off;
+    std::vector<float> tab, rows((size_t)gc.n1 * 16, 0.f);
+    // Tiles start every fourth line along x2 (a tiled copy starts on 16 bytes).
+    if (!x_tiles(gc.n2, 1, kXT2, 4, b2) || !x_tiles(gc.n3, 1, kXT3, 1, b3) ||
+        !fill_res_tables<float>(gc.n2, gc.n3, G->h[1], G->h[2], gc.mu, tab, off))
+        return EQD_OK;
+    E.smem = xmarch_smem(gc.n1);
+    CUDA_OR_RETURN(cudaFuncSetAttribute((const void *)xmarch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        xmarch_smem(EQD_MAX_N1)));
+    const Dense1D M(gc.n1, G->h[0]);
+    for (int i = 0; i < gc.n1; ++i) {
+        float *r = &rows[(size_t)i * 16];
+        for (int o = -3; o <= 3; ++o) {
+            const int c = i + o;
+            if (c < 0 || c >= gc.n1) continue;
+            r[o + 3] = (float)M.d1(i, c);
+            r[7 + o + 3] = (float)(gc.mu * M.d2(i, c));
+        }
+        const int e = std::min(i, gc.n1 - 1 - i);
+        r[14] = (float)(-gc.hvol * (e < 4 ? kHw[e].v() : 1.0));
+    }
+    auto put = [&](DevBuf &b, const void *src, size_t bytes) -> cudaError_t {
+        cudaError_t e = b.ensure(bytes);
+        return e == cudaSuccess ? cudaMemcpyAsync(b.p, src, bytes, cudaMemcpyHostToDevice, G->stream) : e;
+    };
+    CUDA_OR_RETURN(put(E.b2, b2.data(), b2.size() * sizeof(int)));
+    CUDA_OR_RETURN(put(E.b3, b3.data(), b3.size() * sizeof(int)));
+    CUDA_OR_RETURN(put(E.rows, rows.data(), rows.size() * sizeof(float)));
+    CUDA_OR_RETURN(put(E.tab, tab.data(), tab.size() * sizeof(float)));
+    CUDA_OR_RETURN(put(E.off, off.data(), off.size() * sizeof(int)));
+    CUDA_OR_RETURN(cudaStreamSynchronize(G->stream));
+    XGeom &g = E.g;
+    g.n1 = gc.n1;
+    g.n2 = gc.n2;
+    g.n3 = gc.n3;
+    g.n2p = x_row_length(gc.n2);
+    g.colstride = 6LL * gc.n1 * gc.n3 * g.n2p;
+    g.nt2 = (int)b2.size() - 1;
+    g.nt3 = (int)b3.size() - 1;
+    g.b2 = E.b2.as<int>();
+    g.b3 = E.b3.as<int>();
+    g.rows = E.rows.as<float>();
+    g.tab = E.tab.as<float>();
+    g.off = E.off.as<int>();
+    XCoef &C = E.C;
+    C.lam = (float)gc.lam;
+    C.lpm = (float)(gc.lam + gc.mu);
+    C.mu = (float)gc.mu;
+    C.mu2 = (float)(2 * gc.mu);
+    C.sat = (float)gc.sat_c;
+    const double hi = 1.0 / G->h[0];
+    C.a = (float)(kD1Int[3].v() * hi);
+    C.b = (float)(kD1Int[4].v() * hi);
+    C.s0 = (float)(gc.mu * kD2Int[2].v() * hi * hi);
+    C.s1 = (float)(gc.mu * kD2Int[3].v() * hi * hi);
+    C.s2 = (float)(gc.mu * kD2Int[4].v() * hi * hi);
+    for (int k = 0; k < 4; ++k) C.dlo[k] = (float)(kDb[k].v() * hi);
+    E.lay = XLayout{gc.n1, gc.n2, gc.n3, g.n2p, gc.PS, gc.colstride, g.colstride};
+    E.ok = true;
+    return EQD_OK;
+}
+
+// The tensor map of `cap` columns of x2-fastest vectors: boxes of one x1 plane
+// of a tile and its halo, both sides and all components.
+static int make_plane_map(const XGeom &g, const float *p, int cap, CUtensorMap &map) {
+    using Encode = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
+                                const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
+                                CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+    void *fn = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    CUDA_OR_RETURN(cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &found));
+    if (!fn || found != cudaDriverEntryPointSuccess) return fail(EQD_ERR_CUDA, "cuTensorMapEncodeTiled not found");
+    const cuuint64_t row = (cuuint64_t)g.n2p * 4;
+    const cuuint64_t dims[5] = {(cuuint64_t)g.n2p, (cuuint64_t)g.n3, (cuuint64_t)g.n1, 6, (cuuint64_t)cap};
+    const cuuint64_t strides[4] = {row, row * g.n3, row * g.n3 * g.n1, row * g.n3 * g.n1 * 6};
+    const cuuint32_t box[5] = {kXR2, kXR3, 1, 6, 1}, one[5] = {1, 1, 1, 1, 1};
+    const CUresult r = reinterpret_cast<Encode>(fn)(
+        &map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 5, const_cast<float *>(p), dims, strides, box, one,
+        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? EQD_OK : fail(EQD_ERR_CUDA, "cuTensorMapEncodeTiled: " + std::to_string((int)r));
+}
+
+static cudaError_t launch_xmarch(eqd_grid *G, const CUtensorMap &map, float *q, const int8_t *status, double *partials,
+                                 int col0, int ncols, cudaStream_t s) {
+    const XEngine &E = G->xm;
+    const unsigned grid = (unsigned)((long long)ncols * E.g.nt2 * E.g.nt3);
+    xmarch_kernel<<<grid, kXThreads, E.smem, s>>>(map, E.g, E.C, q, status, partials, col0, G->err.as<unsigned>());
+    return cudaGetLastError();
+}
+
+// Layout changes of the flagged columns: x64 += d (fold), or r = src.
+static void launch_xlayout(eqd_grid *G, bool fold, double *x64, float *d, const float *src, const int8_t *status,
+                           const int8_t *flag, int ncols, cudaStream_t s) {
+    const XLayout &l = G->xm.lay;
+    const unsigned nb = (unsigned)ncols * 6 * kXLayoutSplit;
+    if (fold) xlayout_kernel<true><<<nb, 256, 0, s>>>(l, x64, d, nullptr, status, flag);
+    else xlayout_kernel<false><<<nb, 256, 0, s>>>(l, nullptr, d, src, status, flag);
+}
+
 static int check_device_error(eqd_grid *G) {
     unsigned h = 0;
     CUDA_OR_RETURN(cudaMemcpyAsync(&h, G->err.p, sizeof(unsigned), cudaMemcpyDeviceToHost, G->stream));
@@ -945,6 +1068,25 @@ static int apply_impl(eqd_grid *G, const double *x, double *y, int ncols, int mo
     cs.slip_comp = sc.as<int>();
     if (mode == 0) {
         CUDA_OR_RETURN((launch_march<T, T, MODE_AP>(G, dx.as<T>(), dy.as<T>(), cs, nullptr, ncols)));
+    } else if (mode == 2 && sizeof(T) == 4 && G->pin == kXMarchVariant && G->xm.ok) {
+        // The x1 march, on x2-fastest copies.
+        const XLayout &l = G->xm.lay;
+        DevBuf vx, vy;
+        CUDA_OR_RETURN(vx.ensure(sizeof(float) * l.cnew * ncols));
+        CUDA_OR_RETURN(vy.ensure(sizeof(float) * l.cnew * ncols));
+        CUDA_OR_RETURN(cudaMemsetAsync(vx.p, 0, vx.bytes, G->stream));
+        CUDA_OR_RETURN(cudaMemsetAsync(vy.p, 0, vy.bytes, G->stream));
+        CUtensorMap map;
+        int rc = make_plane_map(G->xm.g, vx.as<float>(), ncols, map);
+        if (rc) return rc;
+        const unsigned nb = (unsigned)((nel + tb - 1) / tb);
+        xref_kernel<true><<<nb, tb, 0, G->stream>>>(l, hx.as<double>(), vx.as<float>(), ncols);
+        CUDA_OR_RETURN(launch_xmarch(G, map, vy.as<float>(), nullptr, nullptr, 0, ncols, G->stream));
+        xref_kernel<false><<<nb, tb, 0, G->stream>>>(l, hx.as<double>(), vy.as<float>(), ncols);
+        CUDA_OR_RETURN(cudaGetLastError());
+        CUDA_OR_RETURN(cudaMemcpyAsync(y, hx.p, sizeof(double) * nel, cudaMemcpyDeviceToHost, G->stream));
+        CUDA_OR_RETURN(cudaStreamSynchronize(G->stream));
+        return check_device_error(G);
     } else if (mode == 2) {
         DevBuf part;
         int nt = nparts(G->m64);
@@ -970,7 +1112,13 @@ extern "C" int eqd_apply(eqd_grid *G, const double *x, double *y, int32_t ncols,
     if (G->served) return fail(EQD_ERR_ARG, "the grid is attached to a server");
     CUDA_OR_RETURN(cudaSetDevice(G->desc.device));
     if (precision == EQD_PREC_FP64) return apply_impl<double>(G, x, y, ncols, mode);
-    if (precision == EQD_PREC_MIXED) return apply_impl<float>(G, x, y, ncols, mode);
+    if (precision == EQD_PREC_MIXED) {
+        if (G->pin == kXMarchVariant) {
+            int rc = ensure_xmarch(G);
+            if (rc) return rc;
+        }
+        return apply_impl<float>(G, x, y, ncols, mode);
+    }
     return fail(EQD_ERR_ARG, "unknown precision");
 }
 
@@ -1000,8 +1148,9 @@ struct BatchSpec {
 static int resolve_chunk(eqd_grid *G, const eqd_solve_opts &o, int ncols, int prec, int &chunk) {
     const GridConst &gc = G->gc;
     // x64 + r, p, q (+ d) (+ the second direction buffer of the fused update).
-    const int nvec = 3 + (prec == EQD_PREC_MIXED ? 1 : 0) + ((o.flags & EQD_FLAG_FUSE) ? 1 : 0);
-    const size_t per_col = (size_t)gc.colstride * (8 + (size_t)nvec * (prec == EQD_PREC_MIXED ? 4 : 8)) +
+    // (The x1 march keeps its residuals in a second layout while they are formed, and pads x2 lines.)
+    const int nvec = 3 + (prec == EQD_PREC_MIXED ? 2 : 0) + ((o.flags & EQD_FLAG_FUSE) ? 1 : 0);
+    const size_t per_col = (size_t)std::max(gc.colstride, 6LL * gc.n1 * gc.n3 * x_row_length(gc.n2)) * (8 + (size_t)nvec * (prec == EQD_PREC_MIXED ? 4 : 8)) +
                            (size_t)16 * gc.nf + 1024;
     size_t budget = o.hbm_budget_bytes;
     if (budget == 0) {
@@ -1049,11 +1198,11 @@ static IterPtrs<T> span_ptrs(eqd_grid *G, Workspace &W, const SolveParams &sp, c
     P.cs.status = W.status.as<int8_t>() + c0;
     P.st = ColState{st0.gamma + c0, st0.beta + c0, st0.rr_ref + c0, st0.tol + c0, st0.bnorm + c0,
                     st0.iters + c0, st0.status + c0, st0.flag + c0};
-    P.r = W.v0.as<T>() + c0 * gc.colstride;
-    P.p = W.v1.as<T>() + c0 * gc.colstride;
-    P.q = W.v2.as<T>() + c0 * gc.colstride;
+    P.r = W.v0.as<T>() + c0 * sp.colstride;
+    P.p = W.v1.as<T>() + c0 * sp.colstride;
+    P.q = W.v2.as<T>() + c0 * sp.colstride;
     P.p2 = W.v4.p ? W.v4.as<T>() + c0 * gc.colstride : nullptr;
-    P.d = W.v3.p ? W.v3.as<float>() + c0 * gc.colstride : nullptr;
+    P.d = W.v3.p ? W.v3.as<float>() + c0 * sp.colstride : nullptr;
     P.x64 = W.x64.as<double>() + c0 * gc.colstride;
     P.apply_part = W.apply_part.as<double>() + c0 * sp.ntiles * 2;
     P.res_part = W.res_part.as<double>() + c0 * nparts(G->m64) * 2;
@@ -1076,7 +1225,9 @@ template <typename T>
 static void record_apply(eqd_grid *G, Workspace &W, int generic, int fused, int k, const SolveParams &sp,
                          const ColState &st0, const Span &sn) {
     IterPtrs<T> P = span_ptrs<T>(G, W, sp, st0, sn);
-    if (generic) {
+    if (sp.xlayout) {
+        launch_xmarch(G, W.pmap, (float *)P.q, P.cs.status, P.apply_part, sn.c0, sn.n, sn.s);
+    } else if (generic) {
         launch_march<T, T, MODE_AP>(G, P.p, P.q, P.cs, P.apply_part, sn.n, -1, sn.s);
     } else if (fused) {
         ColumnSet cs = P.cs;
@@ -1107,14 +1258,18 @@ static void record_reliable(eqd_grid *G, const IterPtrs<T> &P, const SolveParams
     // One CTA per item: in most iterations no column is flagged and every
     // CTA returns at once.
     const unsigned items = (unsigned)((long long)sn.n * G->nchunks);
-    fold_correction_kernel<<<items, kVecThreads, 0, sn.s>>>(P.x64, P.d, P.st, sp, sn.n);
+    if (sp.xlayout) launch_xlayout(G, true, P.x64, P.d, nullptr, P.st.status, P.st.flag, sn.n, sn.s);
+    else fold_correction_kernel<<<items, kVecThreads, 0, sn.s>>>(P.x64, P.d, P.st, sp, sn.n);
     ColumnSet cf = P.cs;
     cf.flag = P.st.flag;
     cf.dinv = sp.precond ? G->dinv64.as<double>() : nullptr;
-    launch_march<double, float, MODE_RHS>(G, P.x64, (float *)P.r, cf, P.res_part, sn.n, -1, sn.s);
+    launch_march<double, float, MODE_RHS>(G, P.x64, sp.xlayout ? (float *)P.p2 : (float *)P.r, cf, P.res_part, sn.n, -1,
+                                          sn.s);
+    if (sp.xlayout)
+        launch_xlayout(G, false, nullptr, (float *)P.r, (const float *)P.p2, P.st.status, P.st.flag, sn.n, sn.s);
     SolveParams sp2 = sp;
     sp2.ntiles = nparts(G->m64);
-    cg_true_residual_kernel<<<(unsigned)((sn.n + 127) / 128), 128, 0, sn.s>>>(P.st, sp2, P.res_part, sn.n, 1);
+    cg_true_residual_kernel<<<(unsigned)((sn.n + 3) / 4), 128, 0, sn.s>>>(P.st, sp2, P.res_part, sn.n, 1);
 }
 
 // The rest of iteration k: x, r updates; scalars; reliable update (mixed);
@@ -1145,7 +1300,7 @@ static void record_rest(eqd_grid *G, Workspace &W, int mixed, int fused, int k, 
                                                               (const double *)P.q, P.apply_part, P.st, sp,
                                                               P.rr_part, dinv64, sn.n);
     }
-    const unsigned sb = (unsigned)((sn.n + 127) / 128);
+    const unsigned sb = (unsigned)((sn.n + 3) / 4);
     cg_scalar_kernel<<<sb, 128, 0, sn.s>>>(P.st, sp, P.apply_part, P.rr_part, sn.n, mixed);
     if (mixed) record_reliable<T>(G, P, sp, sn);
     if (!fused) {
@@ -1277,6 +1432,7 @@ struct SlotRun {
     int cap = 0, mixed = 0, generic = 0, dense = 0;
     int fused = 0;  // the direction update runs inside the stencil apply (MODE_AF)
     int resident = 0;            // iterations run in resident_cg_kernel
+    int xm = 0;                  // the FP32 vectors are x2-fastest (xmarch_kernel)
     int kmax = 256, rounds = 1;  // resident: iterations a launch may run, launches per graph
     long long itmax = 0;
     SolveParams sp{};
@@ -1300,7 +1456,6 @@ struct SlotRun {
         dense = dns;
         const GridConst &gc = G->gc;
         const long long ntot = 6LL * gc.n1 * gc.n2 * gc.n3;
-        const size_t vec = (size_t)gc.colstride * cap;
         resident = 0;
         if (!gen && o.precond != EQD_PRECOND_JACOBI && (G->pin < 0 || G->pin == kResidentVariant)) {
             ResEngine &E = sizeof(T) == 4 ? G->res32 : G->res64;
@@ -1310,25 +1465,34 @@ struct SlotRun {
             kmax = tuning ? kIter : 256;
             rounds = mixed && !tuning ? 2 : 1;
         }
-        if (mixed && !G->tuned && !resident) {
+        xm = 0;
+        if (mixed && !gen && !resident && o.precond != EQD_PRECOND_JACOBI &&
+            (G->pin < 0 || G->pin == kResidentVariant || G->pin == kXMarchVariant)) {
+            int rc = ensure_xmarch(G);
+            if (rc) return rc;
+            xm = G->xm.ok;
+        }
+        if (mixed && !G->tuned && !resident && !xm) {
             int rc = tune_by_iterations(G, o, std::min(cap, 1024));
             if (rc) return rc;
         }
         const int nt32 = nparts(G->v32[G->sel32]), nt64 = nparts(G->m64);
         Workspace &w = *W;
-        CUDA_OR_RETURN(w.x64.ensure(sizeof(double) * vec));
+        const size_t vec64 = (size_t)gc.colstride * cap, vec = xm ? (size_t)G->xm.g.colstride * cap : vec64;
+        CUDA_OR_RETURN(w.x64.ensure(sizeof(double) * vec64));
         CUDA_OR_RETURN(w.v0.ensure(sizeof(T) * vec));
         CUDA_OR_RETURN(w.v1.ensure(sizeof(T) * vec));
         CUDA_OR_RETURN(w.v2.ensure(sizeof(T) * vec));
         if (mixed) CUDA_OR_RETURN(w.v3.ensure(sizeof(float) * vec));
         {
             const MarchCfg &mc = sizeof(T) == 4 ? G->v32[G->sel32] : G->m64;
-            fused = !resident && !generic && o.precond != EQD_PRECOND_JACOBI && (o.flags & EQD_FLAG_FUSE) && mc.smem_af > 0;
+            fused = !resident && !xm && !generic && o.precond != EQD_PRECOND_JACOBI && (o.flags & EQD_FLAG_FUSE) && mc.smem_af > 0;
         }
-        if (fused) CUDA_OR_RETURN(w.v4.ensure(sizeof(T) * vec));
+        if (fused || xm) CUDA_OR_RETURN(w.v4.ensure(sizeof(T) * vec64));
         else w.v4.release();
         int ntmax = std::max(nt64, nparts(G->m32));
         for (int v = 0; v < kNumVariants; ++v) ntmax = std::max(ntmax, nparts(G->v32[v]));
+        if (xm) ntmax = std::max(ntmax, G->xm.g.nt2 * G->xm.g.nt3);
         CUDA_OR_RETURN(w.apply_part.ensure(sizeof(double) * 2 * cap * ntmax));
         CUDA_OR_RETURN(w.res_part.ensure(sizeof(double) * 2 * cap * std::max(nt64, G->nchunks)));
         CUDA_OR_RETURN(w.rr_part.ensure(sizeof(double) * 2 * cap * G->nchunks));
@@ -1353,9 +1517,14 @@ struct SlotRun {
         sp.atol = o.atol;
         sp.itmax = o.itmax;
         sp.delta = o.reliable_delta > 0 ? o.reliable_delta : 0.01;
-        sp.ntiles = sizeof(T) == 4 ? nt32 : nt64;
+        sp.ntiles = xm ? G->xm.g.nt2 * G->xm.g.nt3 : sizeof(T) == 4 ? nt32 : nt64;
         sp.nchunks = G->nchunks;
-        sp.colstride = gc.colstride;
+        sp.colstride = xm ? G->xm.g.colstride : gc.colstride;
+        sp.xlayout = xm;
+        if (xm) {
+            int rc = make_plane_map(G->xm.g, w.v1.as<float>(), cap, w.pmap);
+            if (rc) return rc;
+        }
         sp.ntot = ntot;
         sp.precond = o.precond == EQD_PRECOND_JACOBI;
         if (sp.precond) {
@@ -1386,7 +1555,7 @@ struct SlotRun {
         // capture must not be reached through the old graph).
         std::vector<uint64_t> kv = {(uint64_t)cap, (uint64_t)o.precision, (uint64_t)generic, (uint64_t)G->sel32,
                                     (uint64_t)o.precond, (uint64_t)split, (uint64_t)sp.itmax, (uint64_t)fused, (uint64_t)resident,
-                                    (uint64_t)(kmax * 16 + rounds)};
+                                    (uint64_t)(kmax * 16 + rounds), (uint64_t)xm};
         for (double d : {sp.rtol, sp.atol, sp.delta}) {
             uint64_t b;
             std::memcpy(&b, &d, sizeof(b));
@@ -1462,8 +1631,8 @@ struct SlotRun {
         CUDA_OR_RETURN(cudaMemcpyAsync(w.newmask.p, hnew.data(), cap, cudaMemcpyHostToDevice, G->stream));
         const int8_t *mask = w.newmask.as<int8_t>();
         const unsigned nb = (unsigned)(cap * G->nchunks);
-        const long long cst = gc.colstride;
-        zero_columns_kernel<double><<<nb, 256, 0, G->stream>>>(w.x64.as<double>(), cst, G->nchunks, mask);
+        const long long cst = sp.colstride;
+        zero_columns_kernel<double><<<nb, 256, 0, G->stream>>>(w.x64.as<double>(), gc.colstride, G->nchunks, mask);
         zero_columns_kernel<T><<<nb, 256, 0, G->stream>>>(w.v0.as<T>(), cst, G->nchunks, mask);
         zero_columns_kernel<T><<<nb, 256, 0, G->stream>>>(w.v1.as<T>(), cst, G->nchunks, mask);
         zero_columns_kernel<T><<<nb, 256, 0, G->stream>>>(w.v2.as<T>(), cst, G->nchunks, mask);
@@ -1471,18 +1640,19 @@ struct SlotRun {
         // Fused: the second direction buffer's plane padding must read as zero.
         if (fused) zero_columns_kernel<T><<<nb, 256, 0, G->stream>>>(w.v4.as<T>(), cst, G->nchunks, mask);
         launches += (mixed ? 5 : 4) + (fused ? 1 : 0);
-        const unsigned sb = (unsigned)((cap + 127) / 128);
+        const unsigned sb = (unsigned)((cap + 3) / 4);
         if (!generic) {
             // r0 = b = H P (D+SAT) chi  (x = 0), in the working precision.
             ColumnSet cs = colset();
             cs.flag = mask;
             cs.dinv = sp.precond ? G->dinv64.as<double>() : nullptr;
-            CUDA_OR_RETURN((launch_march<double, T, MODE_RHS>(G, w.x64.as<double>(), w.v0.as<T>(), cs,
+            CUDA_OR_RETURN((launch_march<double, T, MODE_RHS>(G, w.x64.as<double>(), xm ? w.v4.as<T>() : w.v0.as<T>(), cs,
                                                                w.res_part.as<double>(), cap)));
             SolveParams sp2 = sp;
             sp2.ntiles = nparts(G->m64);
+            if (xm) launch_xlayout(G, false, nullptr, w.v0.as<float>(), w.v4.as<float>(), w.status.as<int8_t>(), mask, cap, G->stream);
             cg_true_residual_kernel<<<sb, 128, 0, G->stream>>>(st, sp2, w.res_part.as<double>(), cap, mixed, mask);
-            launches += 2;
+            launches += 2 + (xm ? 1 : 0);
         } else {
             // r0 = b given explicitly (reference layout, FP64).
             int j = 0;
@@ -1526,7 +1696,7 @@ struct SlotRun {
         if (running > 0) {
             CUDA_OR_RETURN(cudaGraphLaunch(w.graph, G->stream));
             if (resident) launches += (int64_t)rounds * (mixed ? 4 : 1);
-            else launches += (int64_t)kIter * ((mixed ? 7 : 4) - (fused ? 1 : 0)) * (w.graph_split ? 2 : 1);
+            else launches += (int64_t)kIter * ((mixed ? 7 : 4) - (fused ? 1 : 0) + (xm ? 1 : 0)) * (w.graph_split ? 2 : 1);
         }
         CUDA_OR_RETURN(cudaMemcpyAsync(hst.data(), w.status.p, cap, cudaMemcpyDeviceToHost, G->stream));
         CUDA_OR_RETURN(cudaMemcpyAsync(hit.data(), w.iters.p, sizeof(int) * cap, cudaMemcpyDeviceToHost, G->stream));
@@ -1636,13 +1806,16 @@ static int tune_by_iterations(eqd_grid *G, const eqd_solve_opts &o, int ncols, b
         int v;
         ~PinGuard() { G->pin = v; }
     } guard{G, pin0};
-    if (with_resident && ot.precond != EQD_PRECOND_JACOBI) {
+    if (with_resident) {
         int rc = ensure_resident<float>(G, G->res32);
         if (rc) return rc;
     }
     G->tune_ms[kResidentVariant] = 0.0;
-    const bool res = with_resident && ot.precond != EQD_PRECOND_JACOBI && G->res32.ok;
-    for (int v = 0; v < kNumVariants + (res ? 1 : 0); ++v) {
+    G->tune_ms[kXMarchVariant] = 0.0;
+    for (int v = 0; v < (with_resident ? kAllVariants : kNumVariants); ++v) {
+        // (A grid that a variant has no plan for streams; Jacobi streams x1-fastest.)
+        if (v >= kNumVariants && ot.precond == EQD_PRECOND_JACOBI) continue;
+        if (v == kResidentVariant && !G->res32.ok) continue;
         G->pin = v;
         if (v < kNumVariants) G->sel32 = v;
         SlotRun<float> R;
@@ -1800,8 +1973,8 @@ static int run_batch_any(eqd_grid *G, const eqd_solve_opts *opts, const BatchSpe
         return fail(EQD_ERR_ARG, "precond must be :none or :jacobi");
     if (o.precision != EQD_PREC_FP64 && o.precision != EQD_PREC_MIXED) return fail(EQD_ERR_ARG, "unknown precision");
     if (B.rhs && o.precision != EQD_PREC_FP64) return fail(EQD_ERR_UNSUPPORTED, "explicit-RHS solves run in FP64");
-    if (o.variant < 0 || o.variant > kNumVariants + 1)
-        return fail(EQD_ERR_ARG, "variant must be 0 (the grid's) or 1.." + std::to_string(kNumVariants + 1));
+    if (o.variant < 0 || o.variant > kAllVariants)
+        return fail(EQD_ERR_ARG, "variant must be 0 (the grid's) or 1.." + std::to_string(kAllVariants));
     const auto t0 = std::chrono::steady_clock::now();
     std::lock_guard<std::mutex> lk(G->mtx);
     if (G->served) return fail(EQD_ERR_ARG, "the grid is attached to a server");
@@ -1812,7 +1985,7 @@ static int run_batch_any(eqd_grid *G, const eqd_solve_opts *opts, const BatchSpe
     const bool tuned_before = G->tuned;
     if (o.variant > 0) {
         G->pin = o.variant - 1;
-        if (G->pin != kResidentVariant) {
+        if (G->pin < kNumVariants) {
             G->sel32 = G->pin;
             G->tuned = true;
         }
@@ -1820,7 +1993,7 @@ static int run_batch_any(eqd_grid *G, const eqd_solve_opts *opts, const BatchSpe
     int rc = o.precision == EQD_PREC_MIXED ? run_batch<float>(G, o, B, stats) : run_batch<double>(G, o, B, stats);
     if (o.variant > 0) {
         G->pin = pin_before;
-        if (o.variant - 1 != kResidentVariant) {
+        if (o.variant - 1 < kNumVariants) {
             G->sel32 = sel_before;
             G->tuned = tuned_before;
         }
@@ -2029,9 +2202,12 @@ extern "C" int eqd_autotune(eqd_grid *G, int32_t ncols, int32_t *selected, doubl
         if (rc) return rc;
     }
     if (selected) *selected = G->pin >= 0 ? G->pin : G->sel32;
-    if (nvariants) *nvariants = kNumVariants + 1;
-    if (ms_per_variant) ms_per_variant[kResidentVariant] = G->tune_ms[kResidentVariant];
-    if (tile_rows) tile_rows[kResidentVariant] = 0;
+    if (nvariants) *nvariants = kAllVariants;
+    for (int v = kNumVariants; v < kAllVariants; ++v) {
+        if (ms_per_variant) ms_per_variant[v] = G->tune_ms[v];
+        if (tile_rows) tile_rows[v] = v == kXMarchVariant ? kXT2 : 0;
+    }
+    if (threads) threads[kXMarchVariant] = kXThreads;
     if (threads) threads[kResidentVariant] = G->res32.ok ? 64 * G->res32.d.nch0max : 0;
     for (int v = 0; v < kNumVariants; ++v) {
         if (ms_per_variant) ms_per_variant[v] = G->tune_ms[v];
@@ -2100,11 +2276,11 @@ extern "C" int eqd_tune_chunk(eqd_grid *G, const int32_t *widths, int32_t nwidth
 }
 
 extern "C" int eqd_set_variant(eqd_grid *G, int32_t variant) {
-    if (!G || variant < 0 || variant > kResidentVariant) return fail(EQD_ERR_ARG, "invalid variant");
+    if (!G || variant < 0 || variant >= kAllVariants) return fail(EQD_ERR_ARG, "invalid variant");
     std::lock_guard<std::mutex> lk(G->mtx);
     if (G->served) return fail(EQD_ERR_ARG, "the grid is attached to a server");
     G->pin = variant;
-    if (variant != kResidentVariant) {
+    if (variant < kNumVariants) {
         G->sel32 = variant;
         G->tuned = true;
     }
@@ -2693,8 +2869,8 @@ extern "C" int eqd_server_add_grid(eqd_server *S, eqd_grid *G, int32_t slots) {
     CUDA_OR_RETURN(cudaSetDevice(G->desc.device));
     const GridConst &gc = G->gc;
     const int mixed = S->opts.precision == EQD_PREC_MIXED;
-    const int nvec = 3 + (mixed ? 1 : 0) + ((S->opts.flags & EQD_FLAG_FUSE) ? 1 : 0);
-    const size_t per_slot = (size_t)gc.colstride * (8 + (size_t)nvec * (mixed ? 4 : 8)) + (size_t)16 * gc.nf + 1024;
+    const int nvec = 3 + (mixed ? 2 : 0) + ((S->opts.flags & EQD_FLAG_FUSE) ? 1 : 0);  // as resolve_chunk
+    const size_t per_slot = (size_t)std::max(gc.colstride, 6LL * gc.n1 * gc.n3 * x_row_length(gc.n2)) * (8 + (size_t)nvec * (mixed ? 4 : 8)) + (size_t)16 * gc.nf + 1024;
     std::unique_ptr<SrvGrid> g(new SrvGrid());
     {
         std::lock_guard<std::mutex> lk(S->mu);

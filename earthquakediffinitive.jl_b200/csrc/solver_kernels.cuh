@@ -30,7 +30,20 @@ struct SolveParams {
     long long colstride;
     long long ntot;     // unpadded DOF count (for itmax default)
     int precond;        // 1: Jacobi (gamma = r.z, z = dinv r); 0: none (z = r)
+    int xlayout;        // the FP32 vectors are x2-fastest (xmarch.cuh)
 };
+
+// A column's n partial sums of quantity k, added up by one warp in a fixed
+// order (lane l takes every 32nd from l on, then a butterfly); the result in
+// every lane. One thread adding 100 to 200 of them held up every CTA of the
+// update and, at h = 50 m, 5.6 us an iteration in the scalar kernel.
+__device__ __forceinline__ double sum_parts(const double *part, int col, int n, int k) {
+    double s = 0.0;
+    for (int t = threadIdx.x & 31; t < n; t += 32) s += part[((long long)col * n + t) * 2 + k];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    return s;
+}
 
 // 16-byte group of vector elements: the CG vector kernels move whole groups
 // (a column's storage is a multiple of 4 elements, its start 16-byte
@@ -72,15 +85,11 @@ __global__ void __launch_bounds__(256) cg_update_kernel(TX *__restrict__ x, T *_
         const int col = item / sp.nchunks;
         const int chunk = item % sp.nchunks;
         if (st.status[col] != COL_ACTIVE) continue;
-        if (threadIdx.x == 0) {
-            double pq = 0.0, pp = 0.0;
-            for (int t = 0; t < sp.ntiles; ++t) {
-                pq += apply_part[((long long)col * sp.ntiles + t) * 2 + 0];
-                pp += apply_part[((long long)col * sp.ntiles + t) * 2 + 1];
-            }
+        if (threadIdx.x < 32) {
+            const double pq = sum_parts(apply_part, col, sp.ntiles, 0), pp = sum_parts(apply_part, col, sp.ntiles, 1);
             double a = st.gamma[col] / pq;
             if (!(pq > 2.220446049250313e-16 * pp) || !isfinite(a)) a = 0.0;  // breakdown: scalar kernel flags it
-            s_alpha = a;
+            if (threadIdx.x == 0) s_alpha = a;
         }
         __syncthreads();
         const double alpha = s_alpha;
@@ -249,15 +258,11 @@ __global__ void __launch_bounds__(128, 16) cg_update_bulk_kernel(
         const int col = item / sp.nchunks;
         const int chunk = item % sp.nchunks;
         if (st.status[col] != COL_ACTIVE) continue;
-        if (threadIdx.x == 0) {
-            double pq = 0.0, pp = 0.0;
-            for (int t = 0; t < sp.ntiles; ++t) {
-                pq += apply_part[((long long)col * sp.ntiles + t) * 2 + 0];
-                pp += apply_part[((long long)col * sp.ntiles + t) * 2 + 1];
-            }
+        if (threadIdx.x < 32) {
+            const double pq = sum_parts(apply_part, col, sp.ntiles, 0), pp = sum_parts(apply_part, col, sp.ntiles, 1);
             double a = st.gamma[col] / pq;
             if (!(pq > 2.220446049250313e-16 * pp) || !isfinite(a)) a = 0.0;  // breakdown: scalar kernel flags it
-            s_alpha = a;
+            if (threadIdx.x == 0) s_alpha = a;
         }
         __syncthreads();
         const double alpha = s_alpha;
@@ -422,22 +427,18 @@ __global__ void __launch_bounds__(256) fold_correction_kernel(double *__restrict
     }
 }
 
-__device__ __forceinline__ double sum_parts(const double *part, int col, int n, int stride, int k) {
-    double s = 0.0;
-    for (int t = 0; t < n; ++t) s += part[((long long)col * n + t) * stride + k];
-    return s;
-}
 
 // After the update: count the iteration, test convergence (plain: Krylov's
 // rule on the recursive residual), choose beta, or flag a reliable update.
 __global__ void cg_scalar_kernel(ColState st, SolveParams sp, const double *__restrict__ apply_part,
                                  const double *__restrict__ rr_part, int ncols, int mixed) {
-    const int col = blockIdx.x * blockDim.x + threadIdx.x;
+    const int col = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;  // one warp per column
     if (col >= ncols || st.status[col] != COL_ACTIVE) return;
-    const double pq = sum_parts(apply_part, col, sp.ntiles, 2, 0);
-    const double pp = sum_parts(apply_part, col, sp.ntiles, 2, 1);
-    const double rr = sum_parts(rr_part, col, sp.nchunks, 2, 0);
-    const double rz = sum_parts(rr_part, col, sp.nchunks, 2, 1);
+    const double pq = sum_parts(apply_part, col, sp.ntiles, 0);
+    const double pp = sum_parts(apply_part, col, sp.ntiles, 1);
+    const double rr = sum_parts(rr_part, col, sp.nchunks, 0);
+    const double rz = sum_parts(rr_part, col, sp.nchunks, 1);
+    if (threadIdx.x & 31) return;
     const long long itmax = sp.itmax > 0 ? sp.itmax : 2 * sp.ntot;
     const int it = st.iters[col] + 1;
     st.iters[col] = it;
@@ -480,11 +481,12 @@ __global__ void cg_scalar_kernel(ColState st, SolveParams sp, const double *__re
 // batch (their r0 = b evaluation).
 __global__ void cg_true_residual_kernel(ColState st, SolveParams sp, const double *__restrict__ res_part, int ncols,
                                         int mixed, const int8_t *__restrict__ mask = nullptr) {
-    const int col = blockIdx.x * blockDim.x + threadIdx.x;
+    const int col = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;  // one warp per column
     if (col >= ncols || st.status[col] != COL_ACTIVE) return;
     if (mask ? !mask[col] : (mixed && !st.flag[col])) return;
-    const double rr = sum_parts(res_part, col, sp.ntiles, 2, 0);
-    const double rz = sp.precond ? sum_parts(res_part, col, sp.ntiles, 2, 1) : rr;
+    const double rr = sum_parts(res_part, col, sp.ntiles, 0);
+    const double rz = sp.precond ? sum_parts(res_part, col, sp.ntiles, 1) : rr;
+    if (threadIdx.x & 31) return;
     const int it = st.iters[col];
     if (it == 0) {
         const double bn = sqrt(rr);

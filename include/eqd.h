@@ -100,7 +100,8 @@ typedef struct {
     uint64_t hbm_budget_bytes;/* 0 -> free device memory minus 2 GiB */
     int32_t variant;          /* launch variant for this call: 0 -> the grid's (pinned by eqd_set_variant or
                                  eqd_autotune; else the resident CG where the grid has a plan for it, else
-                                 the streamed variant that the tuner picks on first use); k > 0 -> variant
+                                 the x1 march; with Jacobi the streamed variant that the tuner picks on
+                                 first use); k > 0 -> variant
                                  k - 1 of eqd_autotune's list, for this call only */
     uint32_t flags;
 } eqd_solve_opts;
@@ -189,11 +190,12 @@ int eqd_profile_apply(eqd_grid *grid, int32_t ncols, int32_t precision, int32_t 
 /* Autotuner of the CG's launch configuration: variants 0..10 stream the
  * vectors and differ in the FP32 stencil (x2 tile height, CTA size, columns
  * per thread, edge-partitioned tiles); variant 11 keeps each column's vectors
- * on chip in a cluster of CTAs (small and middle grids; where the grid has no
- * plan for it, it streams). Times 20 mixed-precision CG iterations of ncols
+ * on chip in a cluster of CTAs (small and middle grids; elsewhere it runs as
+ * variant 12); variant 12 streams x2-fastest vectors with the x1-march
+ * stencil. Times 20 mixed-precision CG iterations of ncols
  * unit-slip columns (<= 2nf) with every variant, keeps the fastest for this
  * grid (used by every later call) and reports milliseconds per iteration
- * (0 for variant 11 without a plan). Arrays hold *nvariants (<= 16) entries.
+ * (0 for variants without a plan). Arrays hold *nvariants (<= 16) entries.
  * ncols = 0 re-tunes nothing: it reports the current selection and the times
  * of the last tuning (zeros if the grid was never tuned). */
 int eqd_autotune(eqd_grid *grid, int32_t ncols, int32_t *selected, double *ms_per_variant, int32_t *tile_rows,
