@@ -379,7 +379,9 @@ struct ResEngine {
     bool tried = false, ok = false;
     ResDims d{};
     int t2 = 0, t3 = 0;  // tile capacity of the kernel instance
-    DevBuf ranks, chunks, lines, gofs, push, tab, off;
+    int teams = 0;       // > 0: teams that meet through global memory (else one cluster a column)
+    bool few = false;    // for a few explicit right-hand sides only
+    DevBuf ranks, chunks, lines, gofs, push, pull, tab, off, team_p, team_red, team_count;
     ResTables tb{};
 };
 
@@ -592,31 +594,66 @@ static cudaError_t configure_kernels(int smem_max) {
 // ---------------------------------------------------------------------------
 // Resident CG (resident_cg.cuh): plan, tables and launch
 // ---------------------------------------------------------------------------
-// Kernel instances: n1, and the largest tile of own lines. The x1 lines of the
-// BP8 grids at 100, 80, 50 and 40 m (9 to 21 points) and of the cubes up to
-// 25; FP64 planes of more than 13 points a line do not fit shared memory.
-#define EQD_RES_32(X) X(9, 8, 8) X(9, 8, 16) X(11, 8, 8) X(11, 8, 16) X(13, 8, 8) X(15, 8, 8) X(17, 8, 8) X(21, 8, 8) X(25, 8, 8)
-#define EQD_RES_64(X) X(9, 8, 8) X(11, 8, 8) X(13, 8, 8)
+// Kernel instances: n1, the largest tile of own lines, and the parts that a
+// line is cut into. The x1 lines of the BP8 grids at 100, 80, 50 and 40 m (9 to
+// 21 points) and of the cubes up to 25. The last number: 0, one cluster to a
+// column; 2, a team that meets through global memory (17 points: 4 teams of 36
+// CTAs at 33 x 33, one column 3.1 ms against 19.6 streamed, 96 columns 67
+// against 89); 1, such a team for a few explicit right-hand sides only, up to
+// four a team (25^3: one 5.3 ms against 22, 12 32 against 45). Where a CTA has
+// fewer lines, the streamed iteration is the better one for many (25^3, 300
+// columns: 243 ms against 579), and the choice for columns does not depend on
+// their number, so that a column's bits do not either. FP32 teams, tried at
+// 17 and 21 points, halve a single column's time (h = 40 m 6.8 ms against
+// 15.3) but lose from 16 on (h = 20 m, 64 columns: 548 ms against 220).
+#define EQD_RES_32(X) \
+    X(9, 8, 8, 2, 0) X(9, 8, 16, 2, 0) X(11, 8, 8, 2, 0) X(11, 8, 16, 2, 0) X(13, 8, 8, 2, 0) X(15, 8, 8, 2, 0) \
+    X(17, 8, 8, 2, 0) X(21, 8, 8, 2, 0) X(25, 8, 8, 2, 0)
+#define EQD_RES_64(X) \
+    X(9, 8, 8, 2, 0) X(11, 8, 8, 2, 0) X(13, 8, 8, 2, 0) X(15, 8, 4, 3, 0) X(17, 8, 4, 4, 0) X(19, 8, 4, 4, 0) \
+    X(17, 8, 4, 4, 2) X(19, 8, 4, 4, 1) X(21, 7, 4, 4, 1) X(23, 4, 4, 4, 1) X(25, 4, 4, 4, 1) X(27, 4, 4, 5, 1) \
+    X(29, 4, 3, 5, 1)
 
-// f.operator()<N1, T2, T3>() for the instances of precision T in turn, until
-// one returns true.
+template <int N1, int T2, int T3, int NP, int GRID>
+struct ResInstance {
+    static constexpr int n1 = N1, t2 = T2, t3 = T3, np = NP;
+    static constexpr bool grid = GRID > 0, few = GRID == 1;
+    template <typename T>
+    static constexpr auto kernel() {
+        return resident_cg_kernel<T, N1, T2, T3, NP, grid>;
+    }
+};
+
+// f(ResInstance) for the instances of precision T in turn, until one returns true.
 template <typename T, typename F>
 static bool res_instances(F &&f) {
-#define EQD_CASE(N, A, B) f(std::integral_constant<int, N>(), std::integral_constant<int, A>(), std::integral_constant<int, B>()) ||
+#define EQD_CASE(N, A, B, P, R) f(ResInstance<N, A, B, P, R>()) ||
     if constexpr (sizeof(T) == 4) return EQD_RES_32(EQD_CASE) false;
     else return EQD_RES_64(EQD_CASE) false;
 #undef EQD_CASE
 }
 
-static void res_launch_config(const ResDims &d, int ncols, cudaStream_t s, cudaLaunchConfig_t &cfg,
-                              cudaLaunchAttribute &at) {
+// Warps of a CTA: one per part of a line and chunk of own lines; a team that
+// meets through global memory is small per CTA and has halo rows done by more.
+static int res_warps(const ResDims &d, int np, bool grid, int most) {
+    const int own = np * d.nch0max;
+    return grid ? std::max(own, std::min(most, np * d.nhalomax)) : own;
+}
+
+static void res_launch_config(const ResDims &d, int warps, int teams, bool grid, cudaStream_t s,
+                              cudaLaunchConfig_t &cfg, cudaLaunchAttribute &at) {
     cfg = cudaLaunchConfig_t{};
     at = cudaLaunchAttribute{};
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = (unsigned)d.M;
-    at.val.clusterDim.y = at.val.clusterDim.z = 1;
-    cfg.gridDim = dim3((unsigned)ncols * (unsigned)d.M);
-    cfg.blockDim = dim3((unsigned)(64 * d.nch0max));
+    if (grid) {
+        at.id = cudaLaunchAttributeCooperative;
+        at.val.cooperative = 1;
+    } else {
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = (unsigned)d.M;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    }
+    cfg.gridDim = dim3((unsigned)teams * (unsigned)d.M);
+    cfg.blockDim = dim3((unsigned)(32 * warps));
     cfg.dynamicSmemBytes = (size_t)d.smem;
     cfg.stream = s;
     cfg.attrs = &at;
@@ -633,35 +670,57 @@ static int ensure_resident(eqd_grid *G, ResEngine &E) {
     const GridConst &gc = G->gc;
     ResPlan best;
     double best_cost = 1e300;
-    res_instances<T>([&](auto n1, auto t2, auto t3) {
-        if (n1 != gc.n1) return false;
-        const void *k = (const void *)resident_cg_kernel<T, n1, t2, t3>;
+    res_instances<T>([&](auto I) {
+        if (I.n1 != gc.n1 || (I.grid && best_cost < 1e300)) return false;  // a cluster is listed, and taken, first
+        const void *k = (const void *)I.template kernel<T>();
         cudaFuncAttributes fa{};
         if (cudaFuncGetAttributes(&fa, k) != cudaSuccess ||
             cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResSmemMax) != cudaSuccess ||
-            cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+            (!I.grid && cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)) {
             cudaGetLastError();
             return false;
         }
-        for (int m2 = 1; m2 <= kResMaxTeam; ++m2)
-            for (int m3 = 1; m2 * m3 <= kResMaxTeam; ++m3) {
-                ResPlan P;
-                if (!make_res_plan(gc.n1, gc.n2, gc.n3, gc.PS, m2, m3, res_strides<sizeof(T), n1, t2, t3>(), P)) continue;
-                if (64 * P.d.nch0max > fa.maxThreadsPerBlock) continue;
-                cudaLaunchConfig_t cfg;
-                cudaLaunchAttribute at;
-                res_launch_config(P.d, 1, nullptr, cfg, at);
-                int fit = 0;
-                if (cudaOccupancyMaxActiveClusters(&fit, k, &cfg) != cudaSuccess) {
-                    cudaGetLastError();  // the device cannot place this cluster
-                    continue;
-                }
-                if (fit < 1 || P.cost >= best_cost) continue;
-                best_cost = P.cost;
-                best = P;
-                E.t2 = t2;
-                E.t3 = t3;
+        const auto strides = res_strides<sizeof(T), I.n1, I.t2, I.t3>();
+        auto consider = [&](int m2, int m3) {
+            ResPlan P;
+            if (!make_res_plan(gc.n1, gc.n2, gc.n3, gc.PS, m2, m3, strides, P, I.grid)) return;
+            const int warps = res_warps(P.d, I.np, I.grid, fa.maxThreadsPerBlock / 32);
+            if (32 * warps > fa.maxThreadsPerBlock || P.cost >= best_cost) return;
+            cudaLaunchConfig_t cfg;
+            cudaLaunchAttribute at;
+            res_launch_config(P.d, warps, 1, I.grid, nullptr, cfg, at);
+            int fit = 0;
+            if (I.grid) {
+                if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, k, 32 * warps, P.d.smem) != cudaSuccess) fit = 0;
+                fit = fit * G->num_sms / P.d.M;
+            } else if (cudaOccupancyMaxActiveClusters(&fit, k, &cfg) != cudaSuccess) {
+                fit = 0;
             }
+            cudaGetLastError();  // (the device cannot place this cluster)
+            if (fit < 1) return;
+            best_cost = P.cost;
+            best = P;
+            E.t2 = I.t2;
+            E.t3 = I.t3;
+            E.teams = I.grid ? fit : 0;
+            E.few = I.few;
+        };
+        if (I.grid) {  // the fewest tiles that fit
+            int m[2] = {1, 1};
+            const int n[2] = {gc.n2, gc.n3}, most[2] = {I.t2, I.t3};
+            for (int a = 0; a < 2; ++a)
+                for (; m[a] <= kResMaxGridTeam; ++m[a]) {
+                    std::vector<int> b;
+                    if (!res_split(n[a], m[a], b)) continue;
+                    int w = 0;
+                    for (int q = 0; q < m[a]; ++q) w = std::max(w, b[q + 1] - b[q]);
+                    if (w <= most[a]) break;
+                }
+            if (m[0] * m[1] <= kResMaxGridTeam) consider(m[0], m[1]);
+        } else {
+            for (int m2 = 1; m2 <= kResMaxTeam; ++m2)
+                for (int m3 = 1; m2 * m3 <= kResMaxTeam; ++m3) consider(m2, m3);
+        }
         return false;
     });
     if (best_cost == 1e300) return EQD_OK;
@@ -679,11 +738,27 @@ static int ensure_resident(eqd_grid *G, ResEngine &E) {
     CUDA_OR_RETURN(put(E.lines, best.lines.data(), best.lines.size() * sizeof(ResLine)));
     CUDA_OR_RETURN(put(E.gofs, best.gofs.data(), best.gofs.size() * sizeof(int)));
     CUDA_OR_RETURN(put(E.push, best.push.data(), best.push.size() * sizeof(int)));
+    CUDA_OR_RETURN(put(E.pull, best.pull.data(), best.pull.size() * sizeof(ResPull)));
     CUDA_OR_RETURN(put(E.tab, tab.data(), tab.size() * sizeof(T)));
     CUDA_OR_RETURN(put(E.off, off.data(), off.size() * sizeof(int)));
     CUDA_OR_RETURN(cudaStreamSynchronize(G->stream));
     E.tb = ResTables{E.ranks.as<ResRank>(), E.chunks.as<int>(), E.lines.as<ResLine>(), E.gofs.as<int>(),
-                     E.push.as<int>(), E.tab.p, E.off.as<int>()};
+                     E.push.as<int>(), E.pull.as<ResPull>(), E.tab.p, E.off.as<int>()};
+    if (E.teams) {
+        const size_t ctas = (size_t)E.teams * E.d.M;
+        size_t cs = 0;
+        res_instances<T>([&](auto I) {
+            if (I.grid && I.n1 == gc.n1 && I.t2 == E.t2 && I.t3 == E.t3)
+                cs = ResGeo<sizeof(T), I.n1, I.t2, I.t3>::CS;
+            return cs > 0;
+        });
+        CUDA_OR_RETURN(E.team_p.ensure(sizeof(T) * 3 * cs * ctas));
+        CUDA_OR_RETURN(E.team_red.ensure(sizeof(double) * 8 * ctas));
+        CUDA_OR_RETURN(E.team_count.ensure(sizeof(unsigned) * 32 * E.teams));
+        // (never written, or only read by a CTA that owns none: the far rows of a tile)
+        CUDA_OR_RETURN(cudaMemsetAsync(E.team_p.p, 0, sizeof(T) * 3 * cs * ctas, G->stream));
+        CUDA_OR_RETURN(cudaStreamSynchronize(G->stream));
+    }
     E.ok = true;
     return EQD_OK;
 }
@@ -694,14 +769,26 @@ template <typename T>
 static cudaError_t launch_resident(eqd_grid *G, const ResEngine &E, T *x, T *r, T *p, const ColState &st,
                                    const SolveParams &sp, int mixed, int kmax, int ncols, cudaStream_t s) {
     cudaError_t e = cudaErrorInvalidValue;
-    res_instances<T>([&](auto n1, auto t2, auto t3) {
-        if (n1 != G->gc.n1 || t2 != E.t2 || t3 != E.t3) return false;
+    res_instances<T>([&](auto I) {
+        if (I.n1 != G->gc.n1 || I.t2 != E.t2 || I.t3 != E.t3 || I.grid != (E.teams > 0)) return false;
+        const auto k = I.template kernel<T>();
+        cudaFuncAttributes fa{};
+        e = cudaFuncGetAttributes(&fa, (const void *)k);
+        if (e != cudaSuccess) return true;
+        const int teams = I.grid ? std::min(ncols, E.teams) : ncols;
         cudaLaunchConfig_t cfg;
         cudaLaunchAttribute at;
-        res_launch_config(E.d, ncols, s, cfg, at);
+        res_launch_config(E.d, res_warps(E.d, I.np, I.grid, fa.maxThreadsPerBlock / 32), teams, I.grid, s, cfg, at);
         const ResCoef<T> C = res_coef<T>(G->h[0], G->gc.lam, G->gc.mu, G->gc.sat_c);
-        const ResX1<T, n1> X = res_x1<T, n1>(G->h[0], G->gc.mu, G->gc.hvol);
-        e = cudaLaunchKernelEx(&cfg, resident_cg_kernel<T, n1, t2, t3>, C, X, E.d, E.tb, x, r, p, st, sp, mixed, kmax);
+        const ResX1<T, I.n1> X = res_x1<T, I.n1>(G->h[0], G->gc.mu, G->gc.hvol);
+        ResTeam<T> team{};
+        if constexpr (I.grid) {
+            team = ResTeam<T>{E.team_p.template as<T>(), E.team_red.template as<double>(),
+                              E.team_count.template as<unsigned>(), teams, G->err.as<unsigned>()};
+            e = cudaMemsetAsync(team.count, 0, sizeof(unsigned) * 32 * teams, s);
+            if (e != cudaSuccess) return true;
+        }
+        e = cudaLaunchKernelEx(&cfg, k, C, X, E.d, E.tb, x, r, p, st, sp, mixed, kmax, ncols, team);
         return true;
     });
     return e;
@@ -1446,8 +1533,10 @@ struct SlotRun {
     int64_t launches = 0;
     static constexpr int kIter = 10;
 
-    // `tuning`: the caller times kIter iterations a launch.
-    int setup(eqd_grid *g, const eqd_solve_opts &o, int capacity, bool gen, bool dns, bool tuning = false) {
+    // `tuning`: the caller times kIter iterations a launch. `projected`: every
+    // explicit right-hand side is in the range of P.
+    int setup(eqd_grid *g, const eqd_solve_opts &o, int capacity, bool gen, bool dns, bool tuning = false,
+              bool projected = false) {
         G = g;
         W = &G->ws;
         cap = capacity;
@@ -1457,11 +1546,11 @@ struct SlotRun {
         const GridConst &gc = G->gc;
         const long long ntot = 6LL * gc.n1 * gc.n2 * gc.n3;
         resident = 0;
-        if (!gen && o.precond != EQD_PRECOND_JACOBI && (G->pin < 0 || G->pin == kResidentVariant)) {
+        if ((!gen || projected) && o.precond != EQD_PRECOND_JACOBI && (G->pin < 0 || G->pin == kResidentVariant)) {
             ResEngine &E = sizeof(T) == 4 ? G->res32 : G->res64;
             int rc = ensure_resident<T>(G, E);
             if (rc) return rc;
-            resident = E.ok;
+            resident = E.ok && (!E.few || (gen && cap <= 4 * E.teams));
             kmax = tuning ? kIter : 256;
             rounds = mixed && !tuning ? 2 : 1;
         }
@@ -1845,6 +1934,25 @@ static int tune_by_iterations(eqd_grid *G, const eqd_solve_opts &o, int ncols, b
     return check_device_error(G);
 }
 
+// Whether P b = b exactly: zero at the outer boundary, the same on both sides
+// of every fault node. CG then stays in the range of P, which is all that the
+// resident kernel holds; b = H P (...) always is, and what is not takes the
+// streamed path, whose operator projects its input.
+static bool rhs_in_range(const GridConst &gc, const double *b) {
+    const int n1 = gc.n1, n2 = gc.n2, n3 = gc.n3;
+    const long long pl = (long long)n1 * n2, comp = pl * n3, side = 3 * comp;
+    for (int c = 0; c < 3; ++c)
+        for (int i3 = 0; i3 < n3; ++i3)
+            for (int i2 = 0; i2 < n2; ++i2) {
+                const double *m = b + c * comp + i3 * pl + (long long)i2 * n1, *p = m + side;
+                if (!(m[0] == 0.0 && p[n1 - 1] == 0.0 && m[n1 - 1] == p[0])) return false;
+                if (i3 > 0 && i3 < n3 - 1 && i2 > 0 && i2 < n2 - 1) continue;
+                for (int i = 0; i < n1; ++i)
+                    if (!(m[i] == 0.0 && p[i] == 0.0)) return false;
+            }
+    return true;
+}
+
 // Batched solve through the slot engine: columns enter as slots free up; K
 // columns go to the caller's device or host buffer as each column finishes.
 template <typename T>
@@ -1856,7 +1964,9 @@ static int run_batch(eqd_grid *G, const eqd_solve_opts &o, const BatchSpec &B, e
     int rc = resolve_chunk(G, o, B.ncols, o.precision, chunk);
     if (rc) return rc;
     SlotRun<T> R;
-    rc = R.setup(G, o, chunk, generic, B.slip_dense != nullptr);
+    bool projected = generic;
+    for (int i = 0; i < B.ncols && projected; ++i) projected = rhs_in_range(gc, B.rhs + (size_t)i * ntot);
+    rc = R.setup(G, o, chunk, generic, B.slip_dense != nullptr, false, projected);
     if (rc) return rc;
 
     std::vector<ColWork> work(B.ncols);

@@ -39,9 +39,19 @@
 // ten Toeplitz columns 3.5 ms (15.7), three columns at h = 100 m 1.7 ms (8.5),
 // all 578 there 12.6 ms (34), all 2,178 at h = 50 m 217 ms (300).
 //
+// FP64 lines of more than 13 points take smaller tiles and more parts a line:
+// one column at 17^3 1.8 ms (streamed 14), 96 at 19^3 33 ms (48), 200 at 15^3
+// 21 ms (42). A grid that no cluster holds (GRID) is shared by a team of CTAs
+// of one cooperative launch, which exchange p and the dot products through
+// global memory (L2) and meet at a counter there; each team takes columns in
+// turn. One right-hand side at 25^3 on 49 CTAs: 20 us an iteration, 5.3 ms
+// (streamed 22 to 27: four launches of 7 to 57 us an iteration on a few CTAs).
+//
 // The order of every sum is fixed by the plan, which depends on the grid and
 // the precision only: a column gives the same bits alone and in any batch.
 #pragma once
+#include <type_traits>
+
 #include "resident_plan.h"
 #include "solver_kernels.cuh"
 
@@ -59,6 +69,7 @@ struct ResTables {
     const ResLine *lines;
     const int *gofs;
     const int *push;
+    const ResPull *pull;
     const void *tab;  // fill_res_tables rows, T
     const int *off;
 };
@@ -140,10 +151,11 @@ __host__ __device__ __forceinline__ void res_line_grad(const ResX1<T, N1> &X, co
 // F3); x = N1-1 has F1 only), the second derivatives w, the points' p itself,
 // and, where the points start at the fault, the traction on the fixed +x1 axis
 // there. v: the line's p, component 1.
-template <typename T, int N1, typename G, int XA, int XB, typename PUTF>
+template <typename T, int N1, typename G, int XA, int XB, int W, typename PUTF>
 __host__ __device__ __forceinline__ void res_own_p(const ResCoef<T> &C, const ResX1<T, N1> &X, const T *v, T sgn,
-                                                   ResLineRow<T> row2, ResLineRow<T> row3, T (&w)[XB - XA][3],
-                                                   T (&pv)[XB - XA][3], T (&tau)[3], PUTF putf) {
+                                                   ResLineRow<T> row2, ResLineRow<T> row3, T (&w)[W][3],
+                                                   T (&pv)[W][3], T (&tau)[3], PUTF putf) {
+    static_assert(W >= XB - XA, "a place for every point");
     constexpr int XE = XB == N1 - 1 ? N1 : XB;  // the last half also has F1 at the far field
     constexpr int LO = res_start(XA, N1), HI = res_start(XE - 1, N1) + 6;
     const int oa2 = row2.o[0], ob2 = row2.o[3], oa3 = row3.o[0] * G::R2, ob3 = row3.o[3] * G::R2;
@@ -202,10 +214,10 @@ __host__ __device__ __forceinline__ void res_own_p(const ResCoef<T> &C, const Re
 
 // The F terms of w at the points [XA, XB) of an own line. f1: the line's F1
 // (stride f1s); f2, f3: its places in F2 and F3 (side included).
-template <typename T, int N1, typename G, int XA, int XB>
+template <typename T, int N1, typename G, int XA, int XB, int W>
 __host__ __device__ __forceinline__ void res_own_f(const ResX1<T, N1> &X, const T *f1, int f1s, const T *f2,
                                                    const T *f3, T sgn, ResLineRow<T> row2, ResLineRow<T> row3,
-                                                   T (&w)[XB - XA][3]) {
+                                                   T (&w)[W][3]) {
     constexpr int LO = res_start(XA, N1), HI = res_start(XB - 1, N1) + 6;
     const int oa2 = row2.o[0], ob2 = row2.o[3], oa3 = row3.o[0] * G::R2b, ob3 = row3.o[3] * G::R2b;
     T c2[4], c3[4];
@@ -260,30 +272,77 @@ __device__ __forceinline__ T *map_cluster(T *p, int rank) {
     return reinterpret_cast<T *>(a);
 }
 
-// Threads of an instance at most: 512 x 128 registers, or 256 x 255 where half
-// a line's state needs them.
-template <typename T, int N1>
+// Threads of an instance at most: 512 x 128 registers, or 256 x 255 where a
+// thread's part of a line needs them.
+template <typename T, int N1, int NP>
 constexpr int res_max_threads() {
-    return sizeof(T) == 4 && N1 <= 11 ? 32 * kResMaxWarps : 16 * kResMaxWarps;
+    return (int)sizeof(T) / 4 * (N1 - 1) / NP <= 5 ? 32 * kResMaxWarps : 16 * kResMaxWarps;
+}
+
+// A team of CTAs of a cooperative launch: its copy of p, its partial sums, and
+// the counter that it meets at.
+template <typename T>
+struct ResTeam {
+    T *p;             // [team][rank][3 CS]
+    double *red;      // [team][rank][8]
+    unsigned *count;  // [team][32], its first zero at launch
+    int teams;
+    unsigned *err;
+};
+
+// Every thread of every CTA of the team: what they wrote before is seen by all
+// after. False when the others have not come within about 2 s (recorded).
+__device__ __forceinline__ bool team_barrier(unsigned *count, unsigned target, unsigned *err) {
+    __syncthreads();
+    bool ok = true;
+    if (threadIdx.x == 0) {
+        __threadfence();
+        atomicAdd(count, 1u);
+        unsigned long long t0 = 0;
+        for (int i = 0;; ++i) {
+            unsigned v;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
+            if ((int)(v - target) >= 0) break;
+            if (i == 64) t0 = global_ns();
+            if (i > 64 && ((i & 63) == 0) && global_ns() - t0 > 2000000000ull) {
+                atomicOr(err, DERR_MBAR_TIMEOUT);
+                ok = false;
+                break;
+            }
+        }
+    }
+    return __syncthreads_and(ok);
+}
+
+// f(integral_constant<int, part>) for a run-time part of NP.
+template <int NP, int P = 0, typename F>
+__device__ __forceinline__ void res_with_part(int part, F &&f) {
+    if constexpr (P + 1 < NP) {
+        if (part != P) return res_with_part<NP, P + 1>(part, f);
+    }
+    f(std::integral_constant<int, P>());
 }
 
 // ---------------------------------------------------------------------------
-// One column per cluster of d.M CTAs (grid: ncols * d.M CTAs, 64 d.nch0max
-// threads each). x: the FP32 correction of mixed precision, or the FP64
-// solution. On entry the direction is p = r + beta p.
+// One column per cluster of d.M CTAs (grid: ncols * d.M CTAs, 32 NP d.nch0max
+// threads each), or, GRID, team.teams teams of d.M CTAs that share the ncols
+// columns (more warps there may take halo rows only). NP: parts of a line, one thread each. x: the FP32 correction of
+// mixed precision, or the FP64 solution. On entry the direction is
+// p = r + beta p.
 // ---------------------------------------------------------------------------
-template <typename T, int N1, int T2, int T3>
-__global__ void __launch_bounds__(res_max_threads<T, N1>(), 1)
+template <typename T, int N1, int T2, int T3, int NP, bool GRID>
+__global__ void __launch_bounds__((res_max_threads<T, N1, NP>()), 1)
 resident_cg_kernel(const __grid_constant__ ResCoef<T> C, const __grid_constant__ ResX1<T, N1> X,
                    const __grid_constant__ ResDims d, ResTables tb, T *__restrict__ x_, T *__restrict__ r_,
-                   T *__restrict__ p_, ColState st, SolveParams sp, int mixed, int kmax) {
+                   T *__restrict__ p_, ColState st, SolveParams sp, int mixed, int kmax, int ncols, ResTeam<T> team) {
     using G = ResGeo<(int)sizeof(T), N1, T2, T3>;
-    static_assert(N1 % 2 == 1, "the two halves of a line have the same number of points");
-    constexpr int NX = N1 - 1, XH = NX / 2;  // p is zero at the far field x = N1 - 1
+    constexpr int NX = N1 - 1, XH = (NX + NP - 1) / NP;  // p is zero at the far field x = N1 - 1
+    static_assert((NP - 1) * XH < NX, "every part of a line has points");
+    constexpr bool ragged = NX % NP != 0;  // the last part has fewer
     const int M = d.M;
-    const int slot = blockIdx.x / M;
-    if (st.status[slot] != COL_ACTIVE) return;  // the whole cluster: no barrier has been reached
-    const int rank = M > 1 ? cluster_rank() : 0;
+    const int tm = blockIdx.x / M;
+    if (!GRID && st.status[tm] != COL_ACTIVE) return;  // the whole cluster: no barrier has been reached
+    const int rank = GRID ? blockIdx.x % M : M > 1 ? cluster_rank() : 0;
     const ResRank R = tb.ranks[rank];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nthr = blockDim.x, nwarp = nthr >> 5;
 
@@ -312,13 +371,15 @@ resident_cg_kernel(const __grid_constant__ ResCoef<T> C, const __grid_constant__
     for (int i = tid; i < (kResMaxTeam + kResMaxWarps + 1) * 8; i += nthr) red[i] = 0.0;
     __syncthreads();
 
-    // This thread's half line: warps 2c and 2c + 1 have the CTA's own chunk c.
-    const int side = lane & 1, sub = lane >> 1, chunk = warp >> 1, half = warp & 1;
+    // This thread's part of a line: warps NP c .. NP c + NP - 1 have the CTA's own chunk c.
+    const int side = lane & 1, sub = lane >> 1, chunk = warp / NP, half = warp % NP;
     const T sgn = side ? T(1) : T(-1);
     const bool has = chunk < R.nch0;
     ResLine L{};
     if (has) L = lines[chunk * kResLinesPerChunk + sub];
     const bool own = has && (L.info >> 8 & 1);
+    const int npt = ragged && half == NP - 1 ? NX - (NP - 1) * XH : XH;  // this thread's points
+    auto live = [&](int x) { return !ragged || x < npt; };
     auto rows = [&](int cls) { return ResLineRow<T>{tab + cls * kResRow, off + cls * 4}; };
     const ResLineRow<T> row2 = rows(L.info & 15), row3 = rows(9 + (L.info >> 4 & 15));
     T *const line = p + side * G::SS + L.plo;
@@ -327,10 +388,28 @@ resident_cg_kernel(const __grid_constant__ ResCoef<T> C, const __grid_constant__
     const int f1s = R.nch0 * 32;
     const T hw23 = own ? row2.t[9] * row3.t[9] : T(0);
     const int cstr = d.n3 * d.PS, gstep = side ? 1 : -1;
-    const long long g0 = (long long)slot * d.colstride + 3LL * side * cstr +
-                         (own ? tb.gofs[(R.chunk0 + chunk) * kResLinesPerChunk + sub] : 0) +
-                         (side ? half * XH : NX - half * XH);
+    const int gline = 3 * side * cstr + (own ? tb.gofs[(R.chunk0 + chunk) * kResLinesPerChunk + sub] : 0) +
+                      (side ? half * XH : NX - half * XH);
+    T *const shared_p = GRID ? team.p + ((long long)tm * M + rank) * 3 * G::CS : nullptr;  // this CTA's part of the team's p
+    const T *const team_p = GRID ? team.p + (long long)tm * M * 3 * G::CS : nullptr;
+    double *const team_red = GRID ? team.red + (long long)tm * M * 8 : nullptr;
+    unsigned met = 0;  // GRID: barriers passed
 
+    // Everybody's p, or everybody's sums, are in place.
+    auto meet = [&]() -> bool {
+        if constexpr (GRID) {
+            met += (unsigned)M;
+            return team_barrier(team.count + 32 * tm, met, team.err);
+        } else {
+            if (M > 1) cluster_barrier();
+            else __syncthreads();
+            return true;
+        }
+    };
+
+    for (int slot = tm; slot < ncols; slot += GRID ? team.teams : ncols) {
+    if (GRID && st.status[slot] != COL_ACTIVE) continue;
+    const long long g0 = (long long)slot * d.colstride + gline;
     T r[XH][3], xs[XH][3];
     double gamma = 0.0;
     double beta = st.beta[slot];
@@ -346,7 +425,17 @@ resident_cg_kernel(const __grid_constant__ ResCoef<T> C, const __grid_constant__
 #pragma unroll
         for (int x = 0; x < XH; ++x)
 #pragma unroll
-            for (int c = 0; c < 3; ++c) mine[x * G::PSZ + c * G::CS] = v[x][c];
+            for (int c = 0; c < 3; ++c)
+                if (live(x)) mine[x * G::PSZ + c * G::CS] = v[x][c];
+        if constexpr (GRID) {
+            T *out = shared_p + (mine - p);
+#pragma unroll
+            for (int x = 0; x < XH; ++x)
+#pragma unroll
+                for (int c = 0; c < 3; ++c)
+                    if (live(x)) __stcg(out + x * G::PSZ + c * G::CS, v[x][c]);
+            return;
+        }
         const int *to = push + (chunk * kResLinesPerChunk + sub) * d.npush;
         for (int k = 0; k < d.npush; ++k) {
             const int w = to[k];
@@ -356,12 +445,13 @@ resident_cg_kernel(const __grid_constant__ ResCoef<T> C, const __grid_constant__
             for (int c = 0; c < 3; ++c) {
                 if (!(w >> (24 + c) & 1)) continue;
 #pragma unroll
-                for (int x = 0; x < XH; ++x) q[x * G::PSZ + c * G::CS] = v[x][c];
+                for (int x = 0; x < XH; ++x)
+                    if (live(x)) q[x * G::PSZ + c * G::CS] = v[x][c];
             }
         }
     };
 
-    if (M > 1) cluster_barrier();  // every CTA's p is zeroed before its neighbours store into it
+    if (!GRID && M > 1) cluster_barrier();  // every CTA's p is zeroed before its neighbours store into it
     {
         const T b = (T)beta;
         T v[XH][3];
@@ -370,21 +460,56 @@ resident_cg_kernel(const __grid_constant__ ResCoef<T> C, const __grid_constant__
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
                 const long long g = g0 + c * (long long)cstr + x * gstep;
-                r[x][c] = own ? r_[g] : T(0);
-                xs[x][c] = own ? x_[g] : T(0);
-                v[x][c] = own ? r[x][c] + b * p_[g] : T(0);
+                const bool at = own && live(x);
+                r[x][c] = at ? r_[g] : T(0);
+                xs[x][c] = at ? x_[g] : T(0);
+                v[x][c] = at ? r[x][c] + b * p_[g] : T(0);
             }
         put_p(v);
     }
 
     int status = COL_ACTIVE, flag = 0;
     for (int k = 0;; ++k) {
-        if (M > 1) cluster_barrier();  // every CTA has its new p, halo included
-        else __syncthreads();
+        if (!meet()) return;  // every CTA has its new p (clusters: halo included)
+        if constexpr (GRID) {
+            // The halo, from the team's copy: a lane per line and component, a
+            // warp per plane, up to 32 loads in flight a thread.
+            const ResPull *pl = tb.pull + R.pull0;
+            constexpr int UE = 4, UP = 32 / sizeof(T);
+            for (int e0 = lane; e0 < R.npull; e0 += 32 * UE) {
+                ResPull q[UE];
+#pragma unroll
+                for (int u = 0; u < UE; ++u) q[u] = pl[min(e0 + 32 * u, R.npull - 1)];
+                for (int s0 = warp; s0 < 2 * NX; s0 += UP * nwarp) {
+                    T v[UE][UP];
+#pragma unroll
+                    for (int w = 0; w < UP; ++w) {
+                        const int s = s0 + w * nwarp, o = s < NX ? s * G::PSZ : G::SS + (s - NX) * G::PSZ;
+#pragma unroll
+                        for (int u = 0; u < UE; ++u)
+                            if (s < 2 * NX && e0 + 32 * u < R.npull) v[u][w] = __ldcg(team_p + q[u].src + o);
+                    }
+#pragma unroll
+                    for (int w = 0; w < UP; ++w) {
+                        const int s = s0 + w * nwarp, o = s < NX ? s * G::PSZ : G::SS + (s - NX) * G::PSZ;
+#pragma unroll
+                        for (int u = 0; u < UE; ++u)
+                            if (s < 2 * NX && e0 + 32 * u < R.npull) p[q[u].dst + o] = v[u][w];
+                    }
+                }
+            }
+            __syncthreads();
+        }
 
         // ---- all that reads p: F = lam G_j + (lam + mu) sum_{k != j} G_k, and
         // the second derivatives at the own points ---------------------------
         T q[XH][3], pv[XH][3], tau[3];
+        if constexpr (ragged) {
+#pragma unroll
+            for (int x = 0; x < XH; ++x)
+#pragma unroll
+                for (int c = 0; c < 3; ++c) q[x][c] = pv[x][c] = T(0);
+        }
         if (has) {
             auto putf = [&](int x, T a, T b, T c) {
                 f1[x * f1s] = a;
@@ -393,12 +518,14 @@ resident_cg_kernel(const __grid_constant__ ResCoef<T> C, const __grid_constant__
                     f3[x * G::PSb] = c;
                 }
             };
-            if (half) res_own_p<T, N1, G, XH, NX>(C, X, line, sgn, row2, row3, q, pv, tau, putf);
-            else res_own_p<T, N1, G, 0, XH>(C, X, line, sgn, row2, row3, q, pv, tau, putf);
+            res_with_part<NP>(half, [&](auto P) {
+                constexpr int A = decltype(P)::value * XH, B = A + XH < NX ? A + XH : NX;
+                res_own_p<T, N1, G, A, B>(C, X, line, sgn, row2, row3, q, pv, tau, putf);
+            });
         }
         // Halo rows: F2 two rows beyond the tile along x2, F3 along x3.
-        for (int u = warp; u < 2 * (R.nch - R.nch0); u += nwarp) {
-            const int ch = R.nch0 + (u >> 1);
+        for (int u = GRID ? nwarp - 1 - warp : warp; u < NP * (R.nch - R.nch0); u += nwarp) {
+            const int ch = R.nch0 + u / NP;
             const bool two = chunks[ch] == 1;
             const ResLine H = lines[ch * kResLinesPerChunk + sub];
             const T *v = p + side * G::SS + H.plo;
@@ -408,18 +535,21 @@ resident_cg_kernel(const __grid_constant__ ResCoef<T> C, const __grid_constant__
                 f[x * fs] = two ? C.lam * G2 + C.lpm * (G1 + G3) : C.lam * G3 + C.lpm * (G1 + G2);
             };
             const ResLineRow<T> h2 = rows(H.info & 15), h3 = rows(9 + (H.info >> 4 & 15));
-            if (u & 1) res_line_grad<T, N1, G, XH, NX>(X, v, sgn, h2, h3, put);
-            else res_line_grad<T, N1, G, 0, XH>(X, v, sgn, h2, h3, put);
+            res_with_part<NP>(u % NP, [&](auto P) {
+                constexpr int A = decltype(P)::value * XH, B = A + XH < NX ? A + XH : NX;
+                res_line_grad<T, N1, G, A, B>(X, v, sgn, h2, h3, put);
+            });
         }
         __syncthreads();
 
         // ---- q = A p on the own points, and the dot products -----------------
         double sums[5] = {0.0, 0.0, 0.0, 0.0, 0.0};  // p.q, p.p, r.q, q.q, r.r
         if (has) {
-            if (half) {
-                res_own_f<T, N1, G, XH, NX>(X, f1, f1s, f2, f3, sgn, row2, row3, q);
-            } else {
-                res_own_f<T, N1, G, 0, XH>(X, f1, f1s, f2, f3, sgn, row2, row3, q);
+            res_with_part<NP>(half, [&](auto P) {
+                constexpr int A = decltype(P)::value * XH, B = A + XH < NX ? A + XH : NX;
+                res_own_f<T, N1, G, A, B>(X, f1, f1s, f2, f3, sgn, row2, row3, q);
+            });
+            if (half == 0) {
                 // SAT c (tau+ - tau-) on both sides, then P averages the fault node.
 #pragma unroll
                 for (int j = 0; j < 3; ++j) {
@@ -429,7 +559,11 @@ resident_cg_kernel(const __grid_constant__ ResCoef<T> C, const __grid_constant__
             }
 #pragma unroll
             for (int x = 0; x < XH; ++x) {
-                const T hw = (half ? X.hx[XH + x] : X.hx[x]) * hw23;
+                T hw = X.hx[x];
+#pragma unroll
+                for (int P = 1; P < NP; ++P)
+                    if (half == P) hw = X.hx[P * XH + x < N1 ? P * XH + x : NX];
+                hw *= hw23;
 #pragma unroll
                 for (int c = 0; c < 3; ++c) {
                     q[x][c] *= hw;
@@ -467,7 +601,9 @@ resident_cg_kernel(const __grid_constant__ ResCoef<T> C, const __grid_constant__
             for (int w = 4; w < kResMaxWarps; w += 4) c1 += wred[(part + w) * 8 + sum];  // absent warps hold zero
             c1 += __shfl_xor_sync(0xffffffffu, c1, 2);
             c1 += __shfl_xor_sync(0xffffffffu, c1, 1);
-            if (M > 1) {
+            if constexpr (GRID) {
+                if (part == 0) __stcg(team_red + rank * 8 + sum, c1);
+            } else if (M > 1) {
                 double *to = red + rank * 8 + sum;
 #pragma unroll
                 for (int w = 0; w < kResMaxTeam; w += 4)
@@ -476,17 +612,21 @@ resident_cg_kernel(const __grid_constant__ ResCoef<T> C, const __grid_constant__
                 red[sum] = c1;
             }
         }
-        if (M > 1) cluster_barrier();
-        else __syncthreads();
+        if (!meet()) return;
 
         // ---- alpha, beta and the decision, by warp 0 of each CTA --------------
         // The next residual's norm from the same sums, |r - a q|^2 =
         // |r|^2 - 2 a r.q + a^2 q.q: no second exchange. |r|^2 is summed anew
         // each time, so its rounding does not build up.
         if (warp == 0) {
-            c1 = red[part * 8 + sum];
+            if constexpr (GRID) {
+                c1 = 0.0;
+                for (int w = part; w < M; w += 4) c1 += __ldcg(team_red + w * 8 + sum);
+            } else {
+                c1 = red[part * 8 + sum];
 #pragma unroll
-            for (int w = 4; w < kResMaxTeam; w += 4) c1 += red[(part + w) * 8 + sum];  // ranks beyond M hold zero
+                for (int w = 4; w < kResMaxTeam; w += 4) c1 += red[(part + w) * 8 + sum];  // ranks beyond M hold zero
+            }
             c1 += __shfl_xor_sync(0xffffffffu, c1, 2);
             c1 += __shfl_xor_sync(0xffffffffu, c1, 1);
             const double pq = __shfl_sync(0xffffffffu, c1, 0), pp = __shfl_sync(0xffffffffu, c1, 4),
@@ -548,6 +688,7 @@ resident_cg_kernel(const __grid_constant__ ResCoef<T> C, const __grid_constant__
         for (int x = 0; x < XH; ++x)
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
+                if (!live(x)) continue;
                 const long long g = g0 + c * (long long)cstr + x * gstep;
                 x_[g] = xs[x][c];
                 p_[g] = mine[x * G::PSZ + c * G::CS];
@@ -560,6 +701,7 @@ resident_cg_kernel(const __grid_constant__ ResCoef<T> C, const __grid_constant__
         st.gamma[slot] = gamma;
         if (mixed) st.flag[slot] = (int8_t)flag;
         if (status != COL_ACTIVE) st.status[slot] = (int8_t)status;
+    }
     }
 }
 

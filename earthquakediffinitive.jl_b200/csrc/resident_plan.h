@@ -23,9 +23,9 @@
 
 namespace eqd {
 
-constexpr int kResMaxTeam = 16;
-constexpr int kResMaxChunks = 8;       // chunks of own lines of a CTA: two warps each, one per half of the lines
-constexpr int kResMaxWarps = 2 * kResMaxChunks;
+constexpr int kResMaxTeam = 16;        // CTAs of a cluster
+constexpr int kResMaxGridTeam = 100;   // CTAs of a team that meets through global memory
+constexpr int kResMaxWarps = 16;       // of a CTA: one per chunk of own lines and part of the lines
 constexpr int kResLinesPerChunk = 16;  // a warp holds 16 lines x 2 sides, the sides of a line in adjacent lanes
 constexpr int kResRow = 12;            // elements of a table row (ResAxisRow)
 constexpr size_t kResSmemMax = 232448; // 227 KB, the most a CTA of sm_100 may use
@@ -39,6 +39,7 @@ constexpr size_t kResSmemTwo = 115712; // and two of them on an SM: (228 - 2) / 
 // on distinct banks.
 template <int EB, int N1, int T2, int T3>
 struct ResGeo {
+    static constexpr int n1 = N1;
     static constexpr int NX = N1 - 1;                       // p and F2, F3 need no far-field plane
     static constexpr int R2 = T2 + 8, R3 = T3 + 8;
     static constexpr int lanes = EB == 8 ? 16 : 32;         // elements per bank row
@@ -85,6 +86,13 @@ struct ResRank {
     int nch, nch0;        // chunks; the first nch0 hold this CTA's own lines
     int chunk0;
     int push0;            // first row of its own lines in the push table
+    int pull0, npull;     // its halo in the pull table
+};
+
+// One halo line of one component: where it is in the team's copy of p (a rank's
+// part is 3 CS long), and in this CTA's p.
+struct alignas(8) ResPull {
+    int src, dst;
 };
 
 // Chunk types: 0 own lines, 1 F2 halo rows, 2 F3 halo rows.
@@ -92,7 +100,7 @@ struct ResDims {
     int n3, PS;
     long long colstride;
     int M, Mt2, Mt3;
-    int nch0max;              // a CTA has two warps per chunk of own lines
+    int nch0max, nhalomax;    // a CTA has a warp per chunk of own lines and part of the lines
     int npush;                // places a line's p may have to be pushed to
     int smem;                 // bytes
 };
@@ -106,6 +114,7 @@ struct ResPlan {
     // npush words per own line (16 per chunk): rank << 28 | components << 24 | offset of the line in that rank's
     // p; -1: none. A line's new p goes to every CTA that has it in its halo.
     std::vector<int> push;
+    std::vector<ResPull> pull;    // the same, as the reader sees it
     double cost = 0;              // warps' work of one iteration over the team
 };
 
@@ -145,8 +154,10 @@ inline bool res_split(int n, int parts, std::vector<int> &b) {
 }
 
 // The plan of n1 x n2 x n3 nodes on a team of M = Mt2 x Mt3 CTAs; false if a
-// tile does not fit the planes of `s`.
-inline bool make_res_plan(int n1, int n2, int n3, int PS, int Mt2, int Mt3, const ResStrides &s, ResPlan &out) {
+// tile does not fit the planes of `s`. `pull`: the halo is read by its owner
+// (a rank beyond 15 does not fit a push word).
+inline bool make_res_plan(int n1, int n2, int n3, int PS, int Mt2, int Mt3, const ResStrides &s, ResPlan &out,
+                          bool pull = false) {
     std::vector<int> b2, b3;
     if (!res_split(n2, Mt2, b2) || !res_split(n3, Mt3, b3)) return false;
     for (int k = 0; k < Mt2; ++k)
@@ -189,6 +200,7 @@ inline bool make_res_plan(int n1, int n2, int n3, int PS, int Mt2, int Mt3, cons
         }
         r.nch = (int)out.chunks.size() - r.chunk0;
         d.nch0max = std::max(d.nch0max, r.nch0);
+        d.nhalomax = std::max(d.nhalomax, r.nch - r.nch0);
         for (const L &l : all[q]) {
             ResLine w;
             w.plo = (l.i3 - lo(a3, 4)) * s.R2 + l.i2 - lo(a2, 4);
@@ -217,6 +229,8 @@ inline bool make_res_plan(int n1, int n2, int n3, int PS, int Mt2, int Mt3, cons
         const int a2 = b2[q % Mt2], e2 = b2[q % Mt2 + 1], a3 = b3[q / Mt2], e3 = b3[q / Mt2 + 1];
         for (int o = 0; o < d.M; ++o) {
             if (o == q) continue;
+            const int o2 = o % Mt2, o3 = o / Mt2;
+            if (b2[o2] >= e2 + 4 || b2[o2 + 1] + 4 <= a2 || b3[o3] >= e3 + 4 || b3[o3 + 1] + 4 <= a3) continue;
             for (int l = 0; l < out.ranks[o].nch0 * kResLinesPerChunk; ++l) {
                 const L &w = all[o][l];
                 if (!w.valid) continue;
@@ -228,9 +242,15 @@ inline bool make_res_plan(int n1, int n2, int n3, int PS, int Mt2, int Mt3, cons
                 if (d3 == 0 || (d2 <= 2 && d3 <= 2)) mask |= 2;
                 if (d2 == 0 || (d2 <= 2 && d3 <= 2)) mask |= 4;
                 const int off = (w.i3 - lo(a3, 4)) * s.R2 + w.i2 - lo(a2, 4);
-                if (mask) dest[d3 == 0 ? 0 : d2 == 0 ? 1 : 2][o][l].push_back(q << 28 | mask << 24 | off);
+                if (!mask) continue;
+                dest[d3 == 0 ? 0 : d2 == 0 ? 1 : 2][o][l].push_back(q << 28 | mask << 24 | off);
+                const int from = o * 3 * s.CS + out.lines[(size_t)out.ranks[o].chunk0 * kResLinesPerChunk + l].plo;
+                for (int c = 0; c < 3; ++c)
+                    if (mask >> c & 1) out.pull.push_back(ResPull{from + c * s.CS, off + c * s.CS});
             }
         }
+        out.ranks[q].npull = (int)out.pull.size() - out.ranks[q].pull0;
+        if (q + 1 < d.M) out.ranks[q + 1].pull0 = (int)out.pull.size();
     }
     for (int q = 1; q < d.M; ++q)
         out.ranks[q].push0 = out.ranks[q - 1].push0 + out.ranks[q - 1].nch0 * kResLinesPerChunk;
@@ -244,6 +264,10 @@ inline bool make_res_plan(int n1, int n2, int n3, int PS, int Mt2, int Mt3, cons
             for (int k = 0; k < 3; ++k)
                 for (int u = 0; u < most[k]; ++u)
                     out.push.push_back(u < (int)dest[k][q][l].size() ? dest[k][q][l][u] : -1);
+    if (pull) {
+        out.push.clear();
+        d.npush = 0;
+    }
     d.smem = s.oPush + d.nch0max * kResLinesPerChunk * d.npush * (int)sizeof(int);
     return (size_t)d.smem <= kResSmemMax;
 }
