@@ -2561,28 +2561,63 @@ extern "C" int eqd_kmat_create(int32_t device, int32_t n, const double *K, eqd_k
     return EQD_OK;
 }
 
-// The GEMV's first pass: 16-byte loads of K where K and n allow them
-// (gemv_vec2_ok), 8-byte loads otherwise.
-static void launch_gemv_partial(dim3 grid, cudaStream_t st, const double *K, const double *s, long long n, int nslice,
-                                int nvec, double *part) {
-    if (gemv_vec2_ok(K, n))
-        gemv_partial_kernel<true><<<grid, 256, 0, st>>>(K, s, n, nslice, nvec, part);
-    else
-        gemv_partial_kernel<false><<<grid, 256, 0, st>>>(K, s, n, nslice, nvec, part);
+// Row pairs of a cluster (gemv_kernel): the least of 32, 64 and 128 whose
+// clusters run in one wave, 111 of them on 148 SMs (n = 7,104, 14,208).
+static int gemv_lx(long long n) { return n <= 7104 ? 32 : n <= 14208 ? 64 : 128; }
+
+// y = K s, nothing of y in s.
+static cudaError_t launch_gemv(cudaStream_t st, const double *K, const double *s, int n, int nvec, double *y) {
+    const int nv = nvec >= 3 ? 4 : nvec, lx = gemv_lx(n);
+    const long long tiles = (n + 2 * lx - 1) / (2 * lx), groups = ((long long)nvec + nv - 1) / nv;
+    const unsigned gy = (unsigned)std::min<long long>(groups, 65535);
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = kGemvCluster;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.gridDim = dim3((unsigned)(tiles * kGemvCluster), gy, (unsigned)((groups + gy - 1) / gy));
+    cfg.blockDim = dim3(256);
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    const bool v2 = gemv_vec2_ok(K, n);
+#define EQD_GEMV(NV)                                                                                            \
+    if (nv == NV)                                                                                               \
+        return cudaLaunchKernelEx(&cfg,                                                                         \
+                                  lx == 32   ? (v2 ? gemv_kernel<true, NV, 32> : gemv_kernel<false, NV, 32>)    \
+                                  : lx == 64 ? (v2 ? gemv_kernel<true, NV, 64> : gemv_kernel<false, NV, 64>)    \
+                                             : (v2 ? gemv_kernel<true, NV, 128> : gemv_kernel<false, NV, 128>), \
+                                  K, s, n, nvec, y)
+    EQD_GEMV(1);
+    EQD_GEMV(2);
+    EQD_GEMV(4);
+#undef EQD_GEMV
+    return cudaErrorInvalidValue;
 }
 
-static int gemv_slices(int n) {
-    // Enough CTAs to cover every SM several times over.
-    const int rows_blocks = (n / 2 + 255) / 256;
-    int s = std::max(1, (148 * 8) / std::max(1, rows_blocks));
-    return std::min(s, std::max(1, n / 64));
+// The same for any s and y of `ne` values: a y that overlaps s is finished in `scratch` first.
+static bool gemv_overlap(const double *s, const double *y, long long ne) { return s < y + ne && y < s + ne; }
+
+static cudaError_t launch_gemv_any(cudaStream_t st, const double *K, const double *s, int n, int nvec, double *y,
+                                   double *scratch) {
+    const long long ne = (long long)n * nvec;
+    if (!gemv_overlap(s, y, ne)) return launch_gemv(st, K, s, n, nvec, y);
+    cudaError_t e = launch_gemv(st, K, s, n, nvec, scratch);
+    return e != cudaSuccess ? e : cudaMemcpyAsync(y, scratch, sizeof(double) * ne, cudaMemcpyDeviceToDevice, st);
 }
 
-// Vectors from which y = K s runs as the blocked K S on the FP64 tensor
-// cores (K read once per 16-64 vectors) instead of the GEMV (K read once per
-// 4). Measured at n = 13,122: GEMV 0.25 / 0.25 / 0.32 / 0.44 ms for 1-4
-// vectors (1.1-1.8 ms for 5-8), the tensor-core path 0.27-0.32 ms for 2-8.
-static constexpr int kGemmMinVectors = 3;
+// Whether y = K s for nvec vectors runs as the GEMV (K read once per 4) or as
+// the blocked K S on the FP64 tensor cores (once per 16 to 64). Measured, GEMV
+// against blocked: 1 and 2 vectors always (n = 4,356: 27 us, and 40 from 3 on
+// blocked); 3 and 4 while one group of them is one wave (n = 4,356 31 us
+// against 40, n = 6,000 69 against 64); more while K is read a few times from
+// L2, groups x n^2 up to 1e7: n = 578 64 vectors 14.5 us against 22.8, n =
+// 1,156 16 12.5 against 12.6 and 32 18.7 against 15.7, n = 2,178 8 14.5 against
+// 16.7 and 12 20.7 against 17.6, n = 3,000 8 27 against 23.5.
+static bool gemv_better(long long n, int nvec) {
+    const long long groups = (nvec + 3) / 4;
+    return nvec <= 2 || (groups == 1 && n <= 4736) || groups * n * n <= 10000000;
+}
 
 // Column slices of the blocked K S: the count (1..16, slices of at least 128
 // columns) with the least time in whole waves of resident CTAs,
@@ -2608,7 +2643,7 @@ static int kmat_apply(eqd_kmat *M, const double *s, double *y, int nvec, cudaStr
     const int n = M->n;
     const long long ne = (long long)n * nvec;
     const double *K = M->K.as<double>();
-    if (nvec >= kGemmMinVectors) {
+    if (!gemv_better(n, nvec)) {
         // Vector tile: 16, 32 or 64 vectors per CTA, the narrowest that holds nvec.
         const int tk = nvec <= 16 ? 0 : nvec <= 32 ? 1 : 2, bn = 16 << tk;
         // The slice count depends only on n, nvec and the tile (the
@@ -2626,11 +2661,8 @@ static int kmat_apply(eqd_kmat *M, const double *s, double *y, int nvec, cudaStr
 #undef EQD_KS
         gemv_reduce_kernel<<<(unsigned)((ne + 255) / 256), 256, 0, st>>>(M->part.as<double>(), n, ns, nvec, y);
     } else {
-        const int nslice = gemv_slices(n);
-        CUDA_OR_RETURN(M->part.ensure(sizeof(double) * (size_t)ne * nslice));
-        dim3 grid((unsigned)(((n + 1) / 2 + 255) / 256), (unsigned)nslice);
-        launch_gemv_partial(grid, st, K, s, n, nslice, nvec, M->part.as<double>());
-        gemv_reduce_kernel<<<(unsigned)((ne + 255) / 256), 256, 0, st>>>(M->part.as<double>(), n, nslice, nvec, y);
+        if (gemv_overlap(s, y, ne)) CUDA_OR_RETURN(M->part.ensure(sizeof(double) * (size_t)ne));
+        CUDA_OR_RETURN(launch_gemv_any(st, K, s, n, nvec, y, M->part.as<double>()));
     }
     CUDA_OR_RETURN(cudaGetLastError());
     return EQD_OK;
@@ -2678,15 +2710,13 @@ extern "C" int eqd_kmat_destroy(eqd_kmat *M) {
 // Julia CuArray pool, a PyTorch caching allocator), where a hidden cudaMalloc
 // would break capture or fragment the caller's pool, and latency-critical
 // loops that may not block on the allocator. The caller passes K, s and y as
-// device pointers it already owns; the only scratch (the per-slice partial
-// row sums of the two-pass GEMV) lives in this file-scope array, 4 MiB per
-// device, held by every GPU that loads the library until exit. The first call
-// on a device looks the array's device address up (with that device current);
-// make that first call before any stream capture. All calls on a device share
-// the array: calls that overlap on the GPU race, so serialise them (one
-// stream, or events). The array keeps the last call's contents; nothing in it
-// needs to start at zero, because every partial sum read in a call was written
-// in the same call.
+// device pointers it already owns; the only scratch (the result, where y
+// overlaps s) lives in this file-scope array, 4 MiB per device, held by every
+// GPU that loads the library until exit. The first call on a device looks the
+// array's device address up (with that device current); make that first call
+// before any stream capture. Calls on a device with overlapping s and y share
+// the array: where they overlap on the GPU they race, so serialise them (one
+// stream, or events).
 // ---------------------------------------------------------------------------
 #define EQD_GEMV_STATIC_SCRATCH_DOUBLES (1 << 19)
 
@@ -2722,14 +2752,8 @@ extern "C" int eqd_kmat_gemv_static(int32_t device, int32_t n, const double *K_d
         }
         scratch = g_gemv_static_ptr[device];
     }
-    int nslice = gemv_slices(n);
-    nslice = std::max(1, std::min<int>(nslice, (int)(EQD_GEMV_STATIC_SCRATCH_DOUBLES / ((long long)n * nvec))));
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-    dim3 grid((unsigned)(((n + 1) / 2 + 255) / 256), (unsigned)nslice);
-    launch_gemv_partial(grid, st, K_device, s_device, n, nslice, nvec, scratch);
-    const long long ne = (long long)n * nvec;
-    gemv_reduce_kernel<<<(unsigned)((ne + 255) / 256), 256, 0, st>>>(scratch, n, nslice, nvec, y_device);
-    cudaError_t e = cudaGetLastError();
+    const cudaError_t e =
+        launch_gemv_any(static_cast<cudaStream_t>(stream), K_device, s_device, n, nvec, y_device, scratch);
     if (prev != device) cudaSetDevice(prev);
     if (e != cudaSuccess) return fail(EQD_ERR_CUDA, std::string("eqd_kmat_gemv_static launch: ") + cudaGetErrorString(e));
     return EQD_OK;
@@ -3146,10 +3170,9 @@ extern "C" int eqd_server_destroy(eqd_server *S) {
 struct eqd_rhs {
     int device = 0;
     int nf = 0;
-    int nslice = 1;
     eqd_rhs_params p{};
-    DevBuf K, part, u, du, ap_ptr, ap_idx, ap_val, source, active, vprev, tau, sigma_low, floor_nodes, floor_hits,
-        status;
+    DevBuf K, dtau, io, ap_ptr, ap_idx, ap_val, source, active, vprev, tau, sigma_low, floor_nodes, floor_hits;
+    PinnedArr<double> host;  // io's image: u, the status word, du
     cudaStream_t stream = nullptr;
 };
 
@@ -3184,12 +3207,11 @@ extern "C" int eqd_rhs_create(int32_t device, int32_t nf, const double *K, const
     R->nf = nf;
     R->p = *params;
     const long long n = 2LL * nf;
-    R->nslice = gemv_slices((int)n);
     CUDA_OR_RETURN(cudaStreamCreateWithFlags(&R->stream, cudaStreamNonBlocking));
     CUDA_OR_RETURN(R->K.ensure(sizeof(double) * n * n));
-    CUDA_OR_RETURN(R->part.ensure(sizeof(double) * n * R->nslice));
-    CUDA_OR_RETURN(R->u.ensure(sizeof(double) * (4LL * nf + 1)));
-    CUDA_OR_RETURN(R->du.ensure(sizeof(double) * (4LL * nf + 1)));
+    CUDA_OR_RETURN(R->dtau.ensure(sizeof(double) * n));
+    CUDA_OR_RETURN(R->io.ensure(sizeof(double) * (8LL * nf + 3)));
+    CUDA_OR_RETURN(R->host.assign(8 * nf + 3, 0.0));
     CUDA_OR_RETURN(R->ap_ptr.ensure(sizeof(int) * (nf + 1)));
     CUDA_OR_RETURN(R->ap_idx.ensure(sizeof(int) * std::max(nnz, 1)));
     CUDA_OR_RETURN(R->ap_val.ensure(sizeof(double) * std::max(nnz, 1)));
@@ -3200,7 +3222,6 @@ extern "C" int eqd_rhs_create(int32_t device, int32_t nf, const double *K, const
     CUDA_OR_RETURN(R->sigma_low.ensure(sizeof(double) * nf));
     CUDA_OR_RETURN(R->floor_nodes.ensure(nf));
     CUDA_OR_RETURN(R->floor_hits.ensure(sizeof(unsigned long long)));
-    CUDA_OR_RETURN(R->status.ensure(sizeof(unsigned)));
     cudaStream_t st = R->stream;
     CUDA_OR_RETURN(cudaMemcpyAsync(R->K.p, K, sizeof(double) * n * n, cudaMemcpyHostToDevice, st));
     CUDA_OR_RETURN(cudaMemcpyAsync(R->ap_ptr.p, ap_ptr, sizeof(int) * (nf + 1), cudaMemcpyHostToDevice, st));
@@ -3230,10 +3251,13 @@ extern "C" int eqd_rhs_eval(eqd_rhs *R, double t, const double *u, double *du) {
     const long long nu = 4LL * nf + (R->p.injection == 1 ? 1 : 0);
     const long long n = 2LL * nf;
     cudaStream_t st = R->stream;
-    CUDA_OR_RETURN(cudaMemcpyAsync(R->u.p, u, sizeof(double) * nu, cudaMemcpyHostToDevice, st));
-    CUDA_OR_RETURN(cudaMemsetAsync(R->status.p, 0, sizeof(unsigned), st));
-    dim3 g1((unsigned)(((n + 1) / 2 + 255) / 256), (unsigned)R->nslice);
-    launch_gemv_partial(g1, st, R->K.as<double>(), R->u.as<double>(), n, R->nslice, 1, R->part.as<double>());
+    // One copy each way, through page-locked memory: u and a zero status word
+    // in, the status and du out.
+    double *hu = R->host.data(), *du_dev = R->io.as<double>() + nu + 1;
+    std::memcpy(hu, u, sizeof(double) * nu);
+    hu[nu] = 0.0;
+    CUDA_OR_RETURN(cudaMemcpyAsync(R->io.p, hu, sizeof(double) * (nu + 1), cudaMemcpyHostToDevice, st));
+    CUDA_OR_RETURN(launch_gemv(st, R->K.as<double>(), R->io.as<double>(), (int)n, 1, R->dtau.as<double>()));
     RhsParams P{};
     P.fr = friction_const(R->p);
     P.sigma0 = R->p.sigma0;
@@ -3246,7 +3270,6 @@ extern "C" int eqd_rhs_eval(eqd_rhs *R, double t, const double *u, double *du) {
     P.maxstep = R->p.newton_maxstep;
     P.maxiter = R->p.newton_maxiter;
     P.nf = nf;
-    P.nslice = R->nslice;
     P.peaceman = R->p.injection == 1;
     P.well_cell = R->p.well_cell;
     P.WI = R->p.WI;
@@ -3254,15 +3277,16 @@ extern "C" int eqd_rhs_eval(eqd_rhs *R, double t, const double *u, double *du) {
     P.S_well = R->p.S_well;
     P.Qinj = t < R->p.t_off ? R->p.Q0 : 0.0;
     rhs_node_kernel<<<(unsigned)((nf + 127) / 128), 128, 0, st>>>(
-        P, R->part.as<double>(), R->u.as<double>(), R->du.as<double>(), R->ap_ptr.as<int>(), R->ap_idx.as<int>(),
+        P, R->dtau.as<double>(), R->io.as<double>(), du_dev, R->ap_ptr.as<int>(), R->ap_idx.as<int>(),
         R->ap_val.as<double>(), R->source.as<double>(), R->active.as<unsigned char>(), R->vprev.as<double>(),
         R->tau.as<double>(), R->sigma_low.as<double>(), R->floor_nodes.as<unsigned char>(),
-        R->floor_hits.as<unsigned long long>(), R->status.as<unsigned>());
+        R->floor_hits.as<unsigned long long>(), reinterpret_cast<unsigned *>(du_dev - 1));
     CUDA_OR_RETURN(cudaGetLastError());
-    unsigned h = 0;
-    CUDA_OR_RETURN(cudaMemcpyAsync(du, R->du.p, sizeof(double) * nu, cudaMemcpyDeviceToHost, st));
-    CUDA_OR_RETURN(cudaMemcpyAsync(&h, R->status.p, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
+    CUDA_OR_RETURN(cudaMemcpyAsync(hu + nu, du_dev - 1, sizeof(double) * (nu + 1), cudaMemcpyDeviceToHost, st));
     CUDA_OR_RETURN(cudaStreamSynchronize(st));
+    unsigned h = 0;
+    std::memcpy(&h, hu + nu, sizeof(h));
+    std::memcpy(du, hu + nu + 1, sizeof(double) * nu);
     if (h & RHS_NEWTON_FAILED)
         return fail(EQD_ERR_NOT_CONVERGED, "solve_slip_rate did not converge at some fault node");
     return EQD_OK;

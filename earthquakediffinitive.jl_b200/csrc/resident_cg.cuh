@@ -248,30 +248,6 @@ inline ResCoef<T> res_coef(double h1, double lam, double mu, double sat) {
     return C;
 }
 
-// ---------------------------------------------------------------------------
-// Cluster primitives
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ int cluster_rank() {
-    unsigned r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return (int)r;
-}
-
-// All threads of all CTAs of the cluster; orders their shared-memory writes
-// before what follows.
-__device__ __forceinline__ void cluster_barrier() {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
-// The same place in the shared memory of the cluster's CTA `rank`.
-template <typename T>
-__device__ __forceinline__ T *map_cluster(T *p, int rank) {
-    unsigned long long a;
-    asm("mapa.u64 %0, %1, %2;" : "=l"(a) : "l"(reinterpret_cast<unsigned long long>(p)), "r"(rank));
-    return reinterpret_cast<T *>(a);
-}
-
 // Threads of an instance at most: 512 x 128 registers, or 256 x 255 where a
 // thread's part of a line needs them.
 template <typename T, int N1, int NP>

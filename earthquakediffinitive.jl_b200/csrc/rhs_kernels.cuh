@@ -61,16 +61,15 @@ struct RhsParams {
     double src_scale;   // q0 / (beta phi) while t < t_off, else 0 (Gaussian source)
     double tol, maxstep;
     int maxiter;
-    int nf, nslice;
+    int nf;
     int peaceman;       // 1: Peaceman well at well_cell; 0: Gaussian source
     int well_cell;
     double WI, S_e, S_well, Qinj;
 };
 
-// One thread per fault node: finish the GEMV (fixed-order sum over column
-// slices, as gemv_reduce_kernel), solve the force balance, aging law, and
-// the node's row of the pore-pressure equation (CSR SpMV).
-__global__ void rhs_node_kernel(RhsParams P, const double *__restrict__ part, const double *__restrict__ u,
+// One thread per fault node: solve the force balance (dtau = K s), the aging
+// law, and the node's row of the pore-pressure equation (CSR SpMV).
+__global__ void rhs_node_kernel(RhsParams P, const double *__restrict__ dtau, const double *__restrict__ u,
                                 double *__restrict__ du, const int *__restrict__ ap_ptr,
                                 const int *__restrict__ ap_idx, const double *__restrict__ ap_val,
                                 const double *__restrict__ source, const unsigned char *__restrict__ active,
@@ -80,12 +79,7 @@ __global__ void rhs_node_kernel(RhsParams P, const double *__restrict__ part, co
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int nf = P.nf;
     if (i >= nf) return;
-    const long long n = 2LL * nf;
-    double d2 = 0.0, d3 = 0.0;
-    for (int t = 0; t < P.nslice; ++t) {
-        d2 += part[(long long)t * n + i];
-        d3 += part[(long long)t * n + nf + i];
-    }
+    const double d2 = dtau[i], d3 = dtau[nf + i];
     const double *phi = u + 2LL * nf;
     const double *pres = u + 3LL * nf;
     double V2 = 0.0, V3 = 0.0, Vm = 0.0;

@@ -763,11 +763,22 @@ __global__ void toeplitz_expand_kernel(const double *__restrict__ src_cols, cons
 }
 
 // ---------------------------------------------------------------------------
-// Dense FP64 GEMV y = K s (K column-major n x n), two passes: column slices
-// write partial row sums, then a fixed-order reduction over slices. Vectors
-// go four at a time, so one pass over K serves four right-hand sides (the
-// time loop's Runge-Kutta stages or an ensemble): K is read ceil(nvec / 4)
-// times instead of nvec times.
+// Dense FP64 GEMV y = K s (K column-major n x n), one pass. A cluster of eight
+// CTAs has 2 LX rows: each CTA takes an eighth of the columns, each of its
+// 256 / LX groups of LX threads every (256 / LX)-th of those, two rows a
+// thread, eight columns in flight. The groups' and the CTAs' sums meet in
+// shared memory (of the CTA that owns the row), in a fixed order. Vectors go
+// NV at a time, so one pass over K serves NV right-hand sides; the sums of a
+// vector do not depend on NV.
+//
+// What bounds it: HBM where K is larger than L2 (n = 13,122, 1.38 GB: 197 us =
+// 7.0 TB/s; one pass of column slices by long rows and a second launch that
+// added them took 232), latency where it is not: n = 578 4.3 us (14.5: nine
+// slices on 18 CTAs, 16 loads deep), n = 2,178 8.4 (17.3), n = 4,356 27 (57).
+// LX is 32, or the least that runs in one wave of 6 CTAs an SM (so the launch
+// bounds: 48 registers, 5 an SM, take 231 us at n = 13,122): n = 4,356 27 us
+// with LX = 32 and 37 with 64, n = 8,192 94 and 82. Clusters of 4: 37 us at
+// 4,356; of 16: no faster at 578 to 2,178 and 230 us at 13,122.
 // VEC2: each thread reads its two rows of a column as one 16-byte load, which
 // needs K 16-byte aligned and n even (then every column starts on a 16-byte
 // boundary); gemv_vec2_ok() decides. Otherwise the two rows are read as two
@@ -783,68 +794,88 @@ __device__ __forceinline__ double2 gemv_load2(const double *__restrict__ K, long
     else return make_double2(K[off], K[off + 1]);
 }
 
-template <bool VEC2>
-__global__ void __launch_bounds__(256) gemv_partial_kernel(const double *__restrict__ K, const double *__restrict__ s,
-                                                           long long n, int nslice, int nvec,
-                                                           double *__restrict__ part) {
-    constexpr int VB = 4;
-    const long long row2 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 2;
-    const int slice = blockIdx.y;
-    const long long c0 = n * slice / nslice, c1 = n * (slice + 1) / nslice;
-    for (int v0 = 0; v0 < nvec; v0 += VB) {
-        const int nv = min(VB, nvec - v0);
-        const double *sv[VB];
+constexpr int kGemvCluster = 8;
+
+template <bool VEC2, int NV, int LX>
+__global__ void __launch_bounds__(256, NV <= 2 ? 6 : 4) gemv_kernel(const double *__restrict__ K, const double *__restrict__ s, int n,
+                                                   int nvec, double *__restrict__ y) {
+    constexpr int GP = 256 / LX, R = 2 * LX, U = 8, RC = R / kGemvCluster;
+    const long long v0 = ((long long)blockIdx.z * gridDim.y + blockIdx.y) * NV;
+    if (v0 >= nvec) return;  // the whole cluster
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");  // this CTA runs: its memory may be written
+    __shared__ double red[GP][NV][R];
+    __shared__ double fin[kGemvCluster][NV][RC];
+    const int rank = cluster_rank(), lx = threadIdx.x % LX, g = threadIdx.x / LX;
+    const int row0 = (int)(blockIdx.x / kGemvCluster) * R, row = row0 + 2 * lx;
+    const int c0 = (int)((long long)n * rank / kGemvCluster), c1 = (int)((long long)n * (rank + 1) / kGemvCluster);
+    const int nv = (int)(nvec - v0 < NV ? nvec - v0 : NV);
+    const double *sv[NV];
 #pragma unroll
-        for (int u = 0; u < VB; ++u) sv[u] = s + (long long)(v0 + (u < nv ? u : 0)) * n;
-        double a0[VB], a1[VB];
+    for (int v = 0; v < NV; ++v) sv[v] = s + (v0 + (v < nv ? v : 0)) * n;
+    double a[NV][2];
 #pragma unroll
-        for (int u = 0; u < VB; ++u) a0[u] = a1[u] = 0.0;
-        if (row2 + 1 < n) {
-            long long c = c0;
-            for (; c + 4 <= c1; c += 4) {  // four columns in flight per thread
-                double2 kk[4];
+    for (int v = 0; v < NV; ++v) a[v][0] = a[v][1] = 0.0;
+    if (row + 1 < n) {
+        const double *k = K + row;
+        int c = c0 + g;
+        for (; c + (U - 1) * GP < c1; c += U * GP) {
+            double2 kk[U];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) kk[j] = gemv_load2<VEC2>(K, (c + j) * n + row2);
+            for (int j = 0; j < U; ++j) kk[j] = gemv_load2<VEC2>(k, (long long)(c + j * GP) * n);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
+            for (int j = 0; j < U; ++j)
 #pragma unroll
-                    for (int u = 0; u < VB; ++u) {
-                        if (u < nv) {
-                            const double sc = sv[u][c + j];
-                            a0[u] += kk[j].x * sc;
-                            a1[u] += kk[j].y * sc;
-                        }
-                    }
+                for (int v = 0; v < NV; ++v) {
+                    const double sc = sv[v][c + j * GP];
+                    a[v][0] += kk[j].x * sc;
+                    a[v][1] += kk[j].y * sc;
                 }
-            }
-            for (; c < c1; ++c) {
-                const double2 kk = gemv_load2<VEC2>(K, c * n + row2);
-#pragma unroll
-                for (int u = 0; u < VB; ++u) {
-                    if (u < nv) {
-                        const double sc = sv[u][c];
-                        a0[u] += kk.x * sc;
-                        a1[u] += kk.y * sc;
-                    }
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < VB; ++u) {
-                if (u < nv) {
-                    part[((long long)(v0 + u) * nslice + slice) * n + row2] = a0[u];
-                    part[((long long)(v0 + u) * nslice + slice) * n + row2 + 1] = a1[u];
-                }
-            }
-        } else if (row2 < n) {
-            for (long long c = c0; c < c1; ++c) {
-                const double kk = K[c * n + row2];
-#pragma unroll
-                for (int u = 0; u < VB; ++u) a0[u] += kk * sv[u][c];
-            }
-#pragma unroll
-            for (int u = 0; u < VB; ++u)
-                if (u < nv) part[((long long)(v0 + u) * nslice + slice) * n + row2] = a0[u];
         }
+        if (c < c1) {  // the last few columns, as one batch of loads too
+            double2 kk[U];
+#pragma unroll
+            for (int j = 0; j < U; ++j) {
+                kk[j] = make_double2(0.0, 0.0);
+                if (c + j * GP < c1) kk[j] = gemv_load2<VEC2>(k, (long long)(c + j * GP) * n);
+            }
+#pragma unroll
+            for (int j = 0; j < U; ++j)
+#pragma unroll
+                for (int v = 0; v < NV; ++v)
+                    if (c + j * GP < c1) {
+                        const double sc = sv[v][c + j * GP];
+                        a[v][0] += kk[j].x * sc;
+                        a[v][1] += kk[j].y * sc;
+                    }
+        }
+    } else if (row < n) {
+        for (int c = c0 + g; c < c1; c += GP) {
+            const double kk = K[(long long)c * n + row];
+#pragma unroll
+            for (int v = 0; v < NV; ++v) a[v][0] += kk * sv[v][c];
+        }
+    }
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+        red[g][v][2 * lx] = a[v][0];
+        red[g][v][2 * lx + 1] = a[v][1];
+    }
+    __syncthreads();
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    for (int i = threadIdx.x; i < NV * R; i += 256) {
+        const int v = i / R, r = i % R;
+        double t = red[0][v][r];
+#pragma unroll
+        for (int q = 1; q < GP; ++q) t += red[q][v][r];
+        *map_cluster(&fin[rank][v][r % RC], r / RC) = t;
+    }
+    cluster_barrier();
+    for (int i = threadIdx.x; i < NV * RC; i += 256) {
+        const int v = i / RC, r = i % RC, yr = row0 + rank * RC + r;
+        double t = fin[0][v][r];
+#pragma unroll
+        for (int q = 1; q < kGemvCluster; ++q) t += fin[q][v][r];
+        if (yr < n && v < nv) y[(v0 + v) * n + yr] = t;
     }
 }
 
@@ -870,9 +901,8 @@ __global__ void __launch_bounds__(256) gemv_partial_kernel(const double *__restr
 // slice, vectors past nvec) are zero-filled in registers, so every tile the
 // tensor cores see is finite; that includes the columns of a step that lie
 // past the slice's end. Slice bounds are multiples of 16 columns (the last
-// ends at n). Partial sums go to part[(v * nslice + slice) * n + row], the
-// GEMV's layout, and the same fixed-order reduction over slices finishes
-// them; the tensor cores' own summation order is fixed, so results are the
+// ends at n). Partial sums go to part[(v * nslice + slice) * n + row], and a
+// fixed-order reduction over slices finishes them; the tensor cores' own summation order is fixed, so results are the
 // same bits on every run.
 // VEC2: 16-byte loads (n even, K and S 16-byte aligned).
 // ---------------------------------------------------------------------------

@@ -260,14 +260,15 @@ int eqd_kmat_destroy(eqd_kmat *kmat);
  * graph capture or under a framework's own allocator). K (n x n, column-major),
  * s and y (n x nvec) are DEVICE pointers owned by the caller, on `device`;
  * any n >= 1 and any 8-byte-aligned K (16-byte loads are used only when K is
- * 16-byte aligned and n is even). Scratch is a static 4 MiB array per device:
- * n * nvec must not exceed 524,288 (EQD_ERR_ARG otherwise). The first call on
- * a device looks the array's address up and caches it for the life of the
- * process (make that call before any stream capture; the cached address does
- * not survive a reset of the device's primary context, e.g. cudaDeviceReset).
- * Launches on `stream` (a cudaStream_t, NULL = default stream) and returns
- * without synchronizing. All calls on a device share the scratch array:
- * serialise them (one stream, or events); calls that overlap on the GPU race. */
+ * 16-byte aligned and n is even). Scratch, used where
+ * y overlaps s, is a static 4 MiB array per device: n * nvec must not exceed
+ * 524,288 (EQD_ERR_ARG otherwise). The first call on a device looks the array's
+ * address up and caches it for the life of the process (make that call before
+ * any stream capture; the cached address does not survive a reset of the
+ * device's primary context, e.g. cudaDeviceReset). Launches on `stream` (a
+ * cudaStream_t, NULL = default stream) and returns without synchronizing. Calls
+ * whose y overlaps s share the scratch array of a device: serialise those (one
+ * stream, or events); where they overlap on the GPU they race. */
 int eqd_kmat_gemv_static(int32_t device, int32_t n, const double *K_device, const double *s_device,
                          double *y_device, int32_t nvec, void *stream);
 
