@@ -357,7 +357,7 @@ struct Workspace {
     DevBuf x64, v0, v1, v2, v3;  // x64 + (r, p, q, d) in the working precision
     DevBuf v4;                   // fused direction update: the other p buffer (p alternates v1, v4)
     DevBuf apply_part, res_part, rr_part;
-    DevBuf gamma, beta, rr_ref, tol, bnorm, iters, status, flag;
+    DevBuf gamma, beta, rr_ref, tol, bnorm, pp, iters, status, flag;
     DevBuf slip_node, slip_comp, slip_dense;
     DevBuf kout;
     DevBuf newmask, slot_list, dst_list;  // slot engine: entering columns, extraction lists
@@ -894,12 +894,14 @@ static cudaError_t launch_xmarch(eqd_grid *G, const CUtensorMap &map, float *q, 
 }
 
 // Layout changes of the flagged columns: x64 += d (fold), or r = src.
-static void launch_xlayout(eqd_grid *G, bool fold, double *x64, float *d, const float *src, const int8_t *status,
-                           const int8_t *flag, int ncols, cudaStream_t s) {
-    const XLayout &l = G->xm.lay;
-    const unsigned nb = (unsigned)ncols * 6 * kXLayoutSplit;
-    if (fold) xlayout_kernel<true><<<nb, 256, 0, s>>>(l, x64, d, nullptr, status, flag);
-    else xlayout_kernel<false><<<nb, 256, 0, s>>>(l, nullptr, d, src, status, flag);
+static void launch_xfold(eqd_grid *G, double *x64, float *d, const int8_t *status, const int8_t *flag, int ncols,
+                         cudaStream_t s) {
+    xlayout_kernel<true><<<(unsigned)ncols * 6 * kXLayoutSplit, 256, 0, s>>>(G->xm.lay, x64, d, nullptr, nullptr, status, flag);
+}
+
+static void launch_xresidual(eqd_grid *G, float *r, float *p, const float *src, const int8_t *status,
+                             const int8_t *flag, int ncols, cudaStream_t s) {
+    xlayout_kernel<false><<<(unsigned)ncols * 6 * kXLayoutSplit, 256, 0, s>>>(G->xm.lay, nullptr, r, src, p, status, flag);
 }
 
 static int check_device_error(eqd_grid *G) {
@@ -1284,7 +1286,7 @@ static IterPtrs<T> span_ptrs(eqd_grid *G, Workspace &W, const SolveParams &sp, c
     P.cs.slip_dense = W.slip_dense.p ? W.slip_dense.as<double>() + c0 * 2 * gc.nf : nullptr;
     P.cs.status = W.status.as<int8_t>() + c0;
     P.st = ColState{st0.gamma + c0, st0.beta + c0, st0.rr_ref + c0, st0.tol + c0, st0.bnorm + c0,
-                    st0.iters + c0, st0.status + c0, st0.flag + c0};
+                    st0.iters + c0, st0.status + c0, st0.flag + c0, st0.pp + c0};
     P.r = W.v0.as<T>() + c0 * sp.colstride;
     P.p = W.v1.as<T>() + c0 * sp.colstride;
     P.q = W.v2.as<T>() + c0 * sp.colstride;
@@ -1345,7 +1347,7 @@ static void record_reliable(eqd_grid *G, const IterPtrs<T> &P, const SolveParams
     // One CTA per item: in most iterations no column is flagged and every
     // CTA returns at once.
     const unsigned items = (unsigned)((long long)sn.n * G->nchunks);
-    if (sp.xlayout) launch_xlayout(G, true, P.x64, P.d, nullptr, P.st.status, P.st.flag, sn.n, sn.s);
+    if (sp.xlayout) launch_xfold(G, P.x64, P.d, P.st.status, P.st.flag, sn.n, sn.s);
     else fold_correction_kernel<<<items, kVecThreads, 0, sn.s>>>(P.x64, P.d, P.st, sp, sn.n);
     ColumnSet cf = P.cs;
     cf.flag = P.st.flag;
@@ -1353,7 +1355,7 @@ static void record_reliable(eqd_grid *G, const IterPtrs<T> &P, const SolveParams
     launch_march<double, float, MODE_RHS>(G, P.x64, sp.xlayout ? (float *)P.p2 : (float *)P.r, cf, P.res_part, sn.n, -1,
                                           sn.s);
     if (sp.xlayout)
-        launch_xlayout(G, false, nullptr, (float *)P.r, (const float *)P.p2, P.st.status, P.st.flag, sn.n, sn.s);
+        launch_xresidual(G, (float *)P.r, (float *)P.p, (const float *)P.p2, P.st.status, P.st.flag, sn.n, sn.s);
     SolveParams sp2 = sp;
     sp2.ntiles = nparts(G->m64);
     cg_true_residual_kernel<<<(unsigned)((sn.n + 3) / 4), 128, 0, sn.s>>>(P.st, sp2, P.res_part, sn.n, 1);
@@ -1378,6 +1380,14 @@ static void record_rest(eqd_grid *G, Workspace &W, int mixed, int fused, int k, 
     // FP64: the register versions (the bulk-staged ones measured 17 % slower
     // beside the FP64 stencil).
     unsigned *err = G->err.as<unsigned>();
+    const unsigned sb = (unsigned)((sn.n + 3) / 4);
+    if (sp.xlayout) {
+        cg_step_bulk_kernel<<<nb, kVecThreads, kStepBulkSmem, sn.s>>>(P.d, (float *)P.r, (float *)P.p, (const float *)P.q,
+                                                                      P.apply_part, P.st, sp, P.rr_part, sn.n, err);
+        cg_check_kernel<<<sb, 128, 0, sn.s>>>(P.st, sp, P.apply_part, P.rr_part, sn.n);
+        record_reliable<T>(G, P, sp, sn);
+        return;
+    }
     if (mixed) {
         cg_update_bulk_kernel<float, float><<<nb, kVecThreads, kUpdateBulkSmem, sn.s>>>(
             P.d, (float *)P.r, (const float *)pk, (const float *)P.q, P.apply_part, P.st, sp, P.rr_part, dinv32, sn.n,
@@ -1387,7 +1397,6 @@ static void record_rest(eqd_grid *G, Workspace &W, int mixed, int fused, int k, 
                                                               (const double *)P.q, P.apply_part, P.st, sp,
                                                               P.rr_part, dinv64, sn.n);
     }
-    const unsigned sb = (unsigned)((sn.n + 3) / 4);
     cg_scalar_kernel<<<sb, 128, 0, sn.s>>>(P.st, sp, P.apply_part, P.rr_part, sn.n, mixed);
     if (mixed) record_reliable<T>(G, P, sp, sn);
     if (!fused) {
@@ -1585,7 +1594,7 @@ struct SlotRun {
         CUDA_OR_RETURN(w.apply_part.ensure(sizeof(double) * 2 * cap * ntmax));
         CUDA_OR_RETURN(w.res_part.ensure(sizeof(double) * 2 * cap * std::max(nt64, G->nchunks)));
         CUDA_OR_RETURN(w.rr_part.ensure(sizeof(double) * 2 * cap * G->nchunks));
-        for (DevBuf *b : {&w.gamma, &w.beta, &w.rr_ref, &w.tol, &w.bnorm}) CUDA_OR_RETURN(b->ensure(sizeof(double) * cap));
+        for (DevBuf *b : {&w.gamma, &w.beta, &w.rr_ref, &w.tol, &w.bnorm, &w.pp}) CUDA_OR_RETURN(b->ensure(sizeof(double) * cap));
         CUDA_OR_RETURN(w.iters.ensure(sizeof(int) * cap));
         CUDA_OR_RETURN(w.status.ensure(cap));
         CUDA_OR_RETURN(w.flag.ensure(cap));
@@ -1600,7 +1609,7 @@ struct SlotRun {
         if (generic) CUDA_OR_RETURN(w.hbuf.ensure(sizeof(double) * ntot * cap));
 
         st = ColState{w.gamma.as<double>(), w.beta.as<double>(), w.rr_ref.as<double>(), w.tol.as<double>(),
-                      w.bnorm.as<double>(), w.iters.as<int>(), w.status.as<int8_t>(), w.flag.as<int8_t>()};
+                      w.bnorm.as<double>(), w.iters.as<int>(), w.status.as<int8_t>(), w.flag.as<int8_t>(), w.pp.as<double>()};
         sp = SolveParams{};
         sp.rtol = o.rtol;
         sp.atol = o.atol;
@@ -1651,7 +1660,7 @@ struct SlotRun {
             kv.push_back(b);
         }
         for (const void *q : {w.x64.p, w.v0.p, w.v1.p, w.v2.p, w.v3.p, w.v4.p, w.apply_part.p, w.res_part.p, w.rr_part.p,
-                              w.gamma.p, w.beta.p, w.rr_ref.p, w.tol.p, w.bnorm.p, w.iters.p, w.status.p, w.flag.p,
+                              w.gamma.p, w.beta.p, w.rr_ref.p, w.tol.p, w.bnorm.p, w.pp.p, w.iters.p, w.status.p, w.flag.p,
                               w.slip_node.p, w.slip_comp.p, w.slip_dense.p, G->dinv64.p, G->dinv32.p})
             kv.push_back((uint64_t)(uintptr_t)q);
         if (!w.graph || w.graph_key != kv) {
@@ -1739,7 +1748,7 @@ struct SlotRun {
                                                                w.res_part.as<double>(), cap)));
             SolveParams sp2 = sp;
             sp2.ntiles = nparts(G->m64);
-            if (xm) launch_xlayout(G, false, nullptr, w.v0.as<float>(), w.v4.as<float>(), w.status.as<int8_t>(), mask, cap, G->stream);
+            if (xm) launch_xresidual(G, w.v0.as<float>(), w.v1.as<float>(), w.v4.as<float>(), w.status.as<int8_t>(), mask, cap, G->stream);
             cg_true_residual_kernel<<<sb, 128, 0, G->stream>>>(st, sp2, w.res_part.as<double>(), cap, mixed, mask);
             launches += 2 + (xm ? 1 : 0);
         } else {
@@ -1763,7 +1772,7 @@ struct SlotRun {
             cg_true_residual_kernel<<<sb, 128, 0, G->stream>>>(st, sp2, w.res_part.as<double>(), cap, 0, mask);
             launches += 2;
         }
-        if (resident) {  // the kernel forms the first direction, p = r + 0 p
+        if (resident || xm) {  // the kernel forms the first direction, p = r + 0 p, or it is formed with r
             CUDA_OR_RETURN(cudaGetLastError());
             return EQD_OK;
         }
@@ -1785,7 +1794,7 @@ struct SlotRun {
         if (running > 0) {
             CUDA_OR_RETURN(cudaGraphLaunch(w.graph, G->stream));
             if (resident) launches += (int64_t)rounds * (mixed ? 4 : 1);
-            else launches += (int64_t)kIter * ((mixed ? 7 : 4) - (fused ? 1 : 0) + (xm ? 1 : 0)) * (w.graph_split ? 2 : 1);
+            else launches += (int64_t)kIter * ((mixed ? 7 : 4) - (fused ? 1 : 0)) * (w.graph_split ? 2 : 1);
         }
         CUDA_OR_RETURN(cudaMemcpyAsync(hst.data(), w.status.p, cap, cudaMemcpyDeviceToHost, G->stream));
         CUDA_OR_RETURN(cudaMemcpyAsync(hit.data(), w.iters.p, sizeof(int) * cap, cudaMemcpyDeviceToHost, G->stream));

@@ -19,6 +19,7 @@ struct ColState {
     int *iters;
     int8_t *status;
     int8_t *flag;       // mixed: reliable update pending this iteration
+    double *pp;         // p.p of the current search direction (x2-fastest vectors)
 };
 
 struct SolveParams {
@@ -208,6 +209,7 @@ __global__ void __launch_bounds__(256) cg_pupdate_kernel(T *__restrict__ p, cons
 constexpr int kVecStages = 2;
 constexpr int kVecTileBytes = 4096;
 constexpr size_t kUpdateBulkSmem = 64 + (size_t)kVecStages * 5 * kVecTileBytes;
+constexpr size_t kStepBulkSmem = 64 + (size_t)kVecStages * 4 * kVecTileBytes;
 constexpr size_t kDirBulkSmem = 64 + (size_t)kVecStages * 3 * kVecTileBytes;
 // Launched without a shared-memory opt-in: dynamic plus the update kernel's
 // static 264 bytes must stay within the default 48 KB.
@@ -409,6 +411,122 @@ __global__ void __launch_bounds__(128, 16) cg_pupdate_bulk_kernel(T *__restrict_
     }
 }
 
+// alpha and the next beta of a column whose apply summed p.q and q.q (the
+// x2-fastest FP32 vectors), from |r|^2 of its current residual: r.q = p.q for
+// conjugate directions, so the next |r|^2 is |r|^2 - 2 a p.q + a^2 q.q before
+// the residual is formed (G. Meurant, "Multitasking the conjugate gradient
+// method on the CRAY X-MP/48", Parallel Computing 5, 1987). It serves beta
+// alone: |r|^2 itself is summed anew each iteration, for the next alpha and for
+// every decision. False: zero or negative curvature (then alpha = 0).
+__device__ __forceinline__ bool cg_step(const ColState &st, int col, double pq, double qq, double &alpha, double &beta) {
+    const double rr = st.gamma[col];
+    alpha = rr / pq;
+    const bool curved = pq > 2.220446049250313e-16 * st.pp[col];
+    if (!curved || !isfinite(alpha)) alpha = 0.0;
+    const double a = (double)(float)alpha;
+    beta = fmax(rr - 2.0 * a * pq + a * a * qq, 0.0) / rr;
+    return curved;
+}
+
+// The whole update of an iteration on the x2-fastest vectors in one pass:
+// d += alpha p, r -= alpha q, p = r + beta p, partial r.r and p.p. HBM bound:
+// seven vector passes an iteration beside the apply's two (the two kernels
+// above make nine of it, the last p and r read twice).
+__global__ void __launch_bounds__(128, 16) cg_step_bulk_kernel(float *__restrict__ d, float *__restrict__ r,
+                                                               float *__restrict__ p, const float *__restrict__ q,
+                                                               const double *__restrict__ apply_part, ColState st,
+                                                               SolveParams sp, double *__restrict__ rr_part, int ncols,
+                                                               unsigned *__restrict__ err) {
+    using G = Group<float>;
+    constexpr int V = G::N;
+    constexpr int TE = kVecTileBytes / (int)sizeof(float), TG = TE / V;
+    extern __shared__ __align__(128) unsigned char vsm[];
+    uint64_t *bar = reinterpret_cast<uint64_t *>(vsm);
+    float *buf = reinterpret_cast<float *>(vsm + 64);  // [stage][p, q, r, d][TE]
+    __shared__ double red[32];
+    __shared__ double s_ab[2];
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < kVecStages; ++s) mbar_init(&bar[s], 1);
+        fence_mbar_init();
+    }
+    __syncthreads();
+    unsigned g0 = 0;  // tiles this CTA started before the current item
+    const int nitems = ncols * sp.nchunks;
+    for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
+        const int col = item / sp.nchunks;
+        const int chunk = item % sp.nchunks;
+        if (st.status[col] != COL_ACTIVE) continue;
+        const long long ng = sp.colstride / V;
+        const long long e0 = ng * chunk / sp.nchunks * V, e1 = ng * (chunk + 1) / sp.nchunks * V;
+        const long long off = (long long)col * sp.colstride;
+        const int ntile = (int)((e1 - e0 + TE - 1) / TE);
+        auto issue = [&](int t) {
+            const int s = vec_stage(g0 + t);
+            const long long b0 = e0 + (long long)t * TE;
+            const unsigned bytes = (unsigned)(min((long long)TE, e1 - b0) * (long long)sizeof(float));
+            float *dst = buf + (size_t)s * 4 * TE;
+            mbar_arrive_expect_tx(&bar[s], 4u * bytes);
+            bulk_g2s(dst + 0 * TE, p + off + b0, bytes, &bar[s]);
+            bulk_g2s(dst + 1 * TE, q + off + b0, bytes, &bar[s]);
+            bulk_g2s(dst + 2 * TE, r + off + b0, bytes, &bar[s]);
+            bulk_g2s(dst + 3 * TE, d + off + b0, bytes, &bar[s]);
+        };
+        if (threadIdx.x == 0)
+            for (int t = 0; t < min(kVecStages, ntile); ++t) issue(t);
+        if (threadIdx.x < 32) {  // (beside the first copies)
+            const double pq = sum_parts(apply_part, col, sp.ntiles, 0), qq = sum_parts(apply_part, col, sp.ntiles, 1);
+            double alpha, beta;
+            cg_step(st, col, pq, qq, alpha, beta);
+            if (threadIdx.x == 0) {
+                s_ab[0] = alpha;
+                s_ab[1] = beta;
+            }
+        }
+        __syncthreads();
+        const float a = (float)s_ab[0], b = (float)s_ab[1];
+        double acc = 0.0, accp = 0.0;
+        for (int t = 0; t < ntile; ++t) {
+            const int s = vec_stage(g0 + t);
+            const bool landed = mbar_wait_bounded(&bar[s], vec_parity(g0 + t), err);
+            if (!__syncthreads_and(landed)) {
+                vec_bulk_drain(bar, g0 + t, t + 1 < ntile, err);
+                return;
+            }
+            const long long b0 = e0 + (long long)t * TE;
+            const int ngrp = (int)(min((long long)TE, e1 - b0) / V);
+            const G *tile = reinterpret_cast<const G *>(buf + (size_t)s * 4 * TE);
+            G *dg = reinterpret_cast<G *>(d + off + b0), *rg = reinterpret_cast<G *>(r + off + b0),
+              *pg = reinterpret_cast<G *>(p + off + b0);
+            for (int gi = threadIdx.x; gi < ngrp; gi += blockDim.x) {
+                const G pi = tile[gi], qi = tile[TG + gi], ri = tile[2 * TG + gi], di = tile[3 * TG + gi];
+                G dn, rn, pn;
+#pragma unroll
+                for (int k = 0; k < V; ++k) {
+                    dn.v[k] = di.v[k] + a * pi.v[k];
+                    rn.v[k] = ri.v[k] - a * qi.v[k];
+                    pn.v[k] = rn.v[k] + b * pi.v[k];
+                    acc += (double)rn.v[k] * (double)rn.v[k];
+                    accp += (double)pn.v[k] * (double)pn.v[k];
+                }
+                dg[gi] = dn;
+                rg[gi] = rn;
+                pg[gi] = pn;
+            }
+            __syncthreads();  // stage s is read: refill it
+            if (threadIdx.x == 0 && t + kVecStages < ntile) issue(t + kVecStages);
+        }
+        g0 += (unsigned)ntile;
+        const double rr = block_sum(acc, red);
+        __syncthreads();
+        const double pp = block_sum(accp, red);
+        if (threadIdx.x == 0) {
+            rr_part[((long long)col * sp.nchunks + chunk) * 2 + 0] = rr;
+            rr_part[((long long)col * sp.nchunks + chunk) * 2 + 1] = pp;
+        }
+        __syncthreads();
+    }
+}
+
 // Mixed precision: fold the FP32 correction into the FP64 solution.
 __global__ void __launch_bounds__(256) fold_correction_kernel(double *__restrict__ x, float *__restrict__ d, ColState st,
                                                               SolveParams sp, int ncols) {
@@ -475,6 +593,31 @@ __global__ void cg_scalar_kernel(ColState st, SolveParams sp, const double *__re
     }
 }
 
+// After cg_step_bulk_kernel: count the iteration, and flag a reliable update.
+__global__ void cg_check_kernel(ColState st, SolveParams sp, const double *__restrict__ apply_part,
+                                const double *__restrict__ rr_part, int ncols) {
+    const int col = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;  // one warp per column
+    if (col >= ncols || st.status[col] != COL_ACTIVE) return;
+    const double pq = sum_parts(apply_part, col, sp.ntiles, 0), qq = sum_parts(apply_part, col, sp.ntiles, 1);
+    const double rr = sum_parts(rr_part, col, sp.nchunks, 0), pp = sum_parts(rr_part, col, sp.nchunks, 1);
+    if (threadIdx.x & 31) return;
+    double alpha, beta;
+    const bool curved = cg_step(st, col, pq, qq, alpha, beta);
+    const long long itmax = sp.itmax > 0 ? sp.itmax : 2 * sp.ntot;
+    const int it = st.iters[col] + 1;
+    st.iters[col] = it;
+    const double tol = st.tol[col];
+    if (!curved) {
+        st.flag[col] = 1;  // let the true residual decide
+    } else if (!isfinite(rr)) {
+        st.status[col] = COL_NONFINITE;
+    } else {
+        st.flag[col] = rr <= tol * tol || rr <= sp.delta * sp.delta * st.rr_ref[col] || it >= itmax;
+    }
+    st.gamma[col] = rr;
+    st.pp[col] = pp;
+}
+
 // After a true-residual evaluation (start of a solve, or a reliable update).
 // `first`: this is r0 = b (sets ||b|| and the tolerance).
 // `mask` (optional) restricts the kernel to the columns that just entered the
@@ -494,6 +637,7 @@ __global__ void cg_true_residual_kernel(ColState st, SolveParams sp, const doubl
         st.tol[col] = sp.atol + sp.rtol * bn;
         st.beta[col] = 0.0;
         st.gamma[col] = rz;
+        st.pp[col] = rr;  // (p = r)
         st.rr_ref[col] = rr;
         st.flag[col] = 0;
         if (rr == 0.0) st.status[col] = COL_CONVERGED;  // x = 0 solves it exactly

@@ -278,9 +278,9 @@ __device__ __forceinline__ bool x_step(const XGeom &g, const XCoef &C, const XTh
         }
         const double p2 = t.own ? (double)S.v2[PC] : 0.0, p3 = t.own ? (double)S.v3[PC] : 0.0;
         S.acc0 = fma(p2, (double)q2, S.acc0);
-        S.acc1 = fma(p2, p2, S.acc1);
+        S.acc1 = fma((double)q2, (double)q2, S.acc1);
         S.acc0 = fma(p3, (double)q3, S.acc0);
-        S.acc1 = fma(p3, p3, S.acc1);
+        S.acc1 = fma((double)q3, (double)q3, S.acc1);
     }
     if (e >= 0 && e < n1 - 1) {
         float E;
@@ -297,7 +297,7 @@ __device__ __forceinline__ bool x_step(const XGeom &g, const XCoef &C, const XTh
         if (t.own) *reinterpret_cast<float *>(qcol + (t.q + (unsigned)e * qx)) = q1;
         const double p1 = t.own ? (double)S.v1[PE] : 0.0;
         S.acc0 = fma(p1, (double)q1, S.acc0);
-        S.acc1 = fma(p1, p1, S.acc1);
+        S.acc1 = fma((double)q1, (double)q1, S.acc1);
     }
     return true;
 }
@@ -451,12 +451,14 @@ struct XLayout {
 };
 
 // FOLD: x += d, d = 0 (x FP64, x1-fastest; d x2-fastest). Else: r = src (src
-// x1-fastest, r x2-fastest). kXLayoutSplit blocks per column, side and
+// x1-fastest, r in d, x2-fastest) and p += the change of r, so that p = r +
+// beta p holds for the new r (a column that enters has r = p = 0: p = r). kXLayoutSplit blocks per column, side and
 // component: in most iterations no column is flagged and every block returns.
 constexpr int kXLayoutSplit = 8;
 template <bool FOLD>
 __global__ void __launch_bounds__(256) xlayout_kernel(XLayout g, double *__restrict__ x, float *__restrict__ d,
-                                                      const float *__restrict__ src, const int8_t *__restrict__ status,
+                                                      const float *__restrict__ src, float *__restrict__ p,
+                                                      const int8_t *__restrict__ status,
                                                       const int8_t *__restrict__ flag) {
     __shared__ float t[32][EQD_MAX_N1 + 1];
     const int part = blockIdx.x % kXLayoutSplit, sc = blockIdx.x / kXLayoutSplit % 6, col = blockIdx.x / kXLayoutSplit / 6;
@@ -465,7 +467,8 @@ __global__ void __launch_bounds__(256) xlayout_kernel(XLayout g, double *__restr
     const long long xs = (long long)g.n3 * g.n2p;
     for (int b = part; b < nb * g.n3; b += kXLayoutSplit) {
         const int i3 = b / nb, i2b = (b % nb) * 32, m = min(32, g.n2 - i2b);
-        float *dn = d + col * g.cnew + ((long long)sc * g.n1 * g.n3 + i3) * g.n2p + i2b + kXLead;
+        const long long at = col * g.cnew + ((long long)sc * g.n1 * g.n3 + i3) * g.n2p + i2b + kXLead;
+        float *dn = d + at;
         const long long po = col * g.cold + ((long long)sc * g.n3 + i3) * g.PS + (long long)i2b * g.n1;
         if (FOLD) {
             for (int xx = warp; xx < g.n1; xx += 8)
@@ -479,7 +482,11 @@ __global__ void __launch_bounds__(256) xlayout_kernel(XLayout g, double *__restr
             for (int i = threadIdx.x; i < m * g.n1; i += 256) t[i / g.n1][i % g.n1] = src[po + i];
             __syncthreads();
             for (int xx = warp; xx < g.n1; xx += 8)
-                if (lane < m) dn[xx * xs + lane] = t[lane][side ? xx : g.n1 - 1 - xx];
+                if (lane < m) {
+                    const float v = t[lane][side ? xx : g.n1 - 1 - xx];
+                    p[at + xx * xs + lane] += v - dn[xx * xs + lane];
+                    dn[xx * xs + lane] = v;
+                }
         }
         __syncthreads();
     }
