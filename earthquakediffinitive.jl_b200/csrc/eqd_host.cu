@@ -204,6 +204,7 @@ static bool make_ring_cfg(const GridConst &gc, const double h[3], int which, Mar
     out.g.nblk = 1;
     out.g.nseg = 1;
     out.g.segblk = 1;
+    out.g.target = 0;
     out.g.edge = kRingEdge;
     out.threads = ring_threads(gc.n1, t2);
     out.smem = ring_smem(gc.n1, t2);
@@ -279,6 +280,7 @@ static bool make_march_cfg(int n1, int n2, int n3, int PS, long long colstride, 
     out.g.nblk = sizeof(T) == 8 ? (n3 + EQD_PBLK - 1) / EQD_PBLK : 1;
     out.g.nseg = 1;
     out.g.segblk = out.g.nblk;
+    out.g.target = 0;
     int threads = per_row * t2max;
     threads = (threads + 31) / 32 * 32;
     out.threads = threads;
@@ -311,6 +313,11 @@ static MarchCfg segmented(const MarchCfg &m, long long groups, int num_sms) {
     r.g.nseg = (m.g.nblk + r.g.segblk - 1) / r.g.segblk;
     return r;
 }
+
+// Columns that a launch is split for: with flags (reliable updates, columns
+// that enter) four of them at most; where more are flagged the kernel joins
+// segments again, and where none is, more CTAs would only have to leave.
+static int flagged_cols(const ColumnSet &cs, int ncols) { return cs.flag ? std::min(ncols, 4) : ncols; }
 
 template <typename T>
 static void fill_op(OpConst<T> &C, const GridConst &gc, const double h[3]) {
@@ -533,7 +540,8 @@ static cudaError_t launch_march(eqd_grid *G, const T *in, TO *out, ColumnSet cs,
         return cudaGetLastError();
     }
     constexpr int MAXT = sizeof(T) == 4 ? kMaxT32 : kMaxT64;
-    MarchCfg m = segmented(sizeof(T) == 4 ? G->m32 : G->m64, ncols, G->num_sms);
+    MarchCfg m = segmented(sizeof(T) == 4 ? G->m32 : G->m64, flagged_cols(cs, ncols), G->num_sms);
+    if (sizeof(T) == 8 && cs.flag) m.g.target = 2 * G->num_sms;
     if (MODE == MODE_AF) m.smem = m.smem_af;
     const OpConst<T> &C = *reinterpret_cast<const OpConst<T> *>(sizeof(T) == 4 ? (const void *)&G->c32
                                                                                : (const void *)&G->c64);
@@ -894,14 +902,20 @@ static cudaError_t launch_xmarch(eqd_grid *G, const CUtensorMap &map, float *q, 
 }
 
 // Layout changes of the flagged columns: x64 += d (fold), or r = src.
+static unsigned xlayout_blocks(const XLayout &l, int ncols) {
+    return (unsigned)std::min<long long>(kXLayoutBlocks, 6LL * l.n3 * ((l.n2 + 31) / 32) * ncols);
+}
+
 static void launch_xfold(eqd_grid *G, double *x64, float *d, const int8_t *status, const int8_t *flag, int ncols,
                          cudaStream_t s) {
-    xlayout_kernel<true><<<(unsigned)ncols * 6 * kXLayoutSplit, 256, 0, s>>>(G->xm.lay, x64, d, nullptr, nullptr, status, flag);
+    const XLayout &l = G->xm.lay;
+    xlayout_kernel<true><<<xlayout_blocks(l, ncols), 256, 0, s>>>(l, x64, d, nullptr, nullptr, status, flag, ncols);
 }
 
 static void launch_xresidual(eqd_grid *G, float *r, float *p, const float *src, const int8_t *status,
                              const int8_t *flag, int ncols, cudaStream_t s) {
-    xlayout_kernel<false><<<(unsigned)ncols * 6 * kXLayoutSplit, 256, 0, s>>>(G->xm.lay, nullptr, r, src, p, status, flag);
+    const XLayout &l = G->xm.lay;
+    xlayout_kernel<false><<<xlayout_blocks(l, ncols), 256, 0, s>>>(l, nullptr, r, src, p, status, flag, ncols);
 }
 
 static int check_device_error(eqd_grid *G) {

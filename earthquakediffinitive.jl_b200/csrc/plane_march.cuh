@@ -97,6 +97,9 @@ struct MarchGeom {
                            // (column, tile, block), so any x3 segmentation gives the same bits
     int nseg;              // x3 segments per (column, tile) in this launch
     int segblk;            // blocks per segment
+    int target;            // > 0: CTAs wanted over the flagged columns; segments are joined where more are flagged
+                           // than the launch was split for (a column alone marched all of x3 in one CTA a tile:
+                           // 330 us of a 400 us iteration of 48 columns at h = 20 m, whenever one was flagged)
     int edge;              // > 0: the first and last tiles have `edge` rows and the
                            // tiles between split the rest evenly; 0: all balanced
     int CH;                // ring chunk capacity (elements) per (side, comp)
@@ -295,6 +298,17 @@ plane_march_kernel(const __grid_constant__ OpConst<T> C, const __grid_constant__
 
     const int n1 = N1 > 0 ? N1 : g.n1;
     const int n2 = g.n2, n3 = g.n3;
+    int segblk = g.segblk;
+    if (SEG && g.target > 0) {
+        int busy = 0;  // columns with work
+        for (int c0 = 0; c0 < cs.ncols; c0 += blockDim.x) {
+            const int c = c0 + threadIdx.x;
+            busy += __syncthreads_count(c < cs.ncols && (!cs.status || cs.status[c] == COL_ACTIVE) && cs.flag[c]);
+        }
+        const int ctas = busy * g.ntiles, want = ctas >= g.target ? 1 : min((g.target + ctas - 1) / ctas, g.nblk);
+        segblk = max(segblk, (g.nblk + want - 1) / want);
+        if (seg * segblk >= g.nblk) return;
+    }
     // x3 segment (FP64-input instances). March step s ingests plane s, does
     // the in-plane work and finishes components 1, 2 of plane p = s - 3, and
     // finishes component 3 of plane z = s - 6. Steps are grouped in blocks of
@@ -308,8 +322,8 @@ plane_march_kernel(const __grid_constant__ OpConst<T> C, const __grid_constant__
     // p - 3 .. p + 3); the start is a multiple of the ring depth, so plane q
     // always uses ring slot q % EQD_NSLOT. FP32 instances march the whole
     // column: steps [0, n3 + 6).
-    const int q0 = SEG ? seg * g.segblk * EQD_PBLK : 0;
-    const int q1 = SEG ? min(q0 + g.segblk * EQD_PBLK, n3) : n3;
+    const int q0 = SEG ? seg * segblk * EQD_PBLK : 0;
+    const int q1 = SEG ? min(q0 + segblk * EQD_PBLK, n3) : n3;
     const int blk0 = q0 / EQD_PBLK;
     const int nbs = (q1 - q0 + EQD_PBLK - 1) / EQD_PBLK;   // blocks of this segment
     const int o_beg = q0 + 3;                               // owned steps: [o_beg, s_end)
@@ -431,7 +445,7 @@ plane_march_kernel(const __grid_constant__ OpConst<T> C, const __grid_constant__
         if constexpr (MODE == MODE_AF)
             for (int i = tid; i < nring; i += blockDim.x) rring[i] = T(0);
         if constexpr (SEG) {
-            const int nrb = L * g.segblk * nwarps * 2;
+            const int nrb = L * segblk * nwarps * 2;
             for (int i = tid; i < nrb; i += blockDim.x) rblk[i] = 0.0;
         }
         fence_proxy_async_smem();
@@ -585,7 +599,7 @@ plane_march_kernel(const __grid_constant__ OpConst<T> C, const __grid_constant__
                 y += __shfl_down_sync(0xffffffffu, y, o);
             }
             if (lane == 0) {
-                double *slot = rblk + (((size_t)l * g.segblk + b) * nwarps + warp) * 2;
+                double *slot = rblk + (((size_t)l * segblk + b) * nwarps + warp) * 2;
                 slot[0] += x;
                 slot[1] += y;
             }
@@ -913,7 +927,7 @@ plane_march_kernel(const __grid_constant__ OpConst<T> C, const __grid_constant__
                 if (!act[l]) continue;
                 for (int i = tid; i < nbs * 2; i += blockDim.x) {
                     const int k = i & 1, b = i >> 1;
-                    const double *src = rblk + ((size_t)l * g.segblk + b) * nwarps * 2 + k;
+                    const double *src = rblk + ((size_t)l * segblk + b) * nwarps * 2 + k;
                     double sum = 0.0;
                     for (int w = 0; w < nwarps; ++w) sum += src[(size_t)w * 2];
                     partials[(((long long)colv[l] * g.ntiles + tile) * g.nblk + blk0 + b) * 2 + k] = sum;

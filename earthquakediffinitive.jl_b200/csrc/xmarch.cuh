@@ -442,8 +442,8 @@ xmarch_kernel(const __grid_constant__ CUtensorMap map, const __grid_constant__ X
     }
 }
 
-// Between the two layouts, for the flagged (or masked) columns: one block per
-// (column, side and component, x3 plane, 32 lines along x2), transposed
+// Between the two layouts, for the flagged (or masked) columns: an item is one
+// column's side and component, x3 plane and 32 lines along x2, transposed
 // through shared memory so that both sides move whole sectors.
 struct XLayout {
     int n1, n2, n3, n2p, PS;
@@ -452,43 +452,54 @@ struct XLayout {
 
 // FOLD: x += d, d = 0 (x FP64, x1-fastest; d x2-fastest). Else: r = src (src
 // x1-fastest, r in d, x2-fastest) and p += the change of r, so that p = r +
-// beta p holds for the new r (a column that enters has r = p = 0: p = r). kXLayoutSplit blocks per column, side and
-// component: in most iterations no column is flagged and every block returns.
-constexpr int kXLayoutSplit = 8;
+// beta p holds for the new r (a column that enters has r = p = 0: p = r).
+// The blocks share out the items of the flagged columns, of which there are
+// usually none or a few: one column then has the whole chip (a few blocks to
+// each column took 100 to 170 us whenever one was flagged, of 400 an iteration
+// of 48 columns at h = 20 m).
+constexpr int kXLayoutBlocks = 592;  // four an SM
 template <bool FOLD>
 __global__ void __launch_bounds__(256) xlayout_kernel(XLayout g, double *__restrict__ x, float *__restrict__ d,
                                                       const float *__restrict__ src, float *__restrict__ p,
                                                       const int8_t *__restrict__ status,
-                                                      const int8_t *__restrict__ flag) {
+                                                      const int8_t *__restrict__ flag, int ncols) {
     __shared__ float t[32][EQD_MAX_N1 + 1];
-    const int part = blockIdx.x % kXLayoutSplit, sc = blockIdx.x / kXLayoutSplit % 6, col = blockIdx.x / kXLayoutSplit / 6;
-    if (status[col] != COL_ACTIVE || !flag[col]) return;
-    const int nb = (g.n2 + 31) / 32, side = sc / 3, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int nb = (g.n2 + 31) / 32, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int per = 6 * g.n3 * nb;  // items of a column: side and component, x3 plane, 32 lines along x2
     const long long xs = (long long)g.n3 * g.n2p;
-    for (int b = part; b < nb * g.n3; b += kXLayoutSplit) {
-        const int i3 = b / nb, i2b = (b % nb) * 32, m = min(32, g.n2 - i2b);
-        const long long at = col * g.cnew + ((long long)sc * g.n1 * g.n3 + i3) * g.n2p + i2b + kXLead;
-        float *dn = d + at;
-        const long long po = col * g.cold + ((long long)sc * g.n3 + i3) * g.PS + (long long)i2b * g.n1;
-        if (FOLD) {
-            for (int xx = warp; xx < g.n1; xx += 8)
-                if (lane < m) {
-                    t[lane][side ? xx : g.n1 - 1 - xx] = dn[xx * xs + lane];
-                    dn[xx * xs + lane] = 0.f;
+    int k0 = blockIdx.x;  // this block's next item, counted from the current flagged column's first
+    for (int cb = 0; cb < ncols; cb += 32) {
+        const bool f = cb + lane < ncols && status[cb + lane] == COL_ACTIVE && flag[cb + lane];
+        for (unsigned m32 = __ballot_sync(0xffffffffu, f); m32; m32 &= m32 - 1) {
+            const int col = cb + __ffs(m32) - 1;
+            for (; k0 < per; k0 += gridDim.x) {
+                const int b = k0 % nb, i3 = k0 / nb % g.n3, sc = k0 / nb / g.n3, side = sc / 3;
+                const int i2b = b * 32, m = min(32, g.n2 - i2b);
+                const long long at = col * g.cnew + ((long long)sc * g.n1 * g.n3 + i3) * g.n2p + i2b + kXLead;
+                const long long po = col * g.cold + ((long long)sc * g.n3 + i3) * g.PS + (long long)i2b * g.n1;
+                float *dn = d + at;
+                if (FOLD) {
+                    for (int xx = warp; xx < g.n1; xx += 8)
+                        if (lane < m) {
+                            t[lane][side ? xx : g.n1 - 1 - xx] = dn[xx * xs + lane];
+                            dn[xx * xs + lane] = 0.f;
+                        }
+                    __syncthreads();
+                    for (int i = threadIdx.x; i < m * g.n1; i += 256) x[po + i] += (double)t[i / g.n1][i % g.n1];
+                } else {
+                    for (int i = threadIdx.x; i < m * g.n1; i += 256) t[i / g.n1][i % g.n1] = src[po + i];
+                    __syncthreads();
+                    for (int xx = warp; xx < g.n1; xx += 8)
+                        if (lane < m) {
+                            const float v = t[lane][side ? xx : g.n1 - 1 - xx];
+                            p[at + xx * xs + lane] += v - dn[xx * xs + lane];
+                            dn[xx * xs + lane] = v;
+                        }
                 }
-            __syncthreads();
-            for (int i = threadIdx.x; i < m * g.n1; i += 256) x[po + i] += (double)t[i / g.n1][i % g.n1];
-        } else {
-            for (int i = threadIdx.x; i < m * g.n1; i += 256) t[i / g.n1][i % g.n1] = src[po + i];
-            __syncthreads();
-            for (int xx = warp; xx < g.n1; xx += 8)
-                if (lane < m) {
-                    const float v = t[lane][side ? xx : g.n1 - 1 - xx];
-                    p[at + xx * xs + lane] += v - dn[xx * xs + lane];
-                    dn[xx * xs + lane] = v;
-                }
+                __syncthreads();
+            }
+            k0 -= per;
         }
-        __syncthreads();
     }
 }
 
