@@ -399,6 +399,7 @@ struct XEngine {
     XCoef C{};
     XLayout lay{};
     int smem = 0;
+    int nchunks = 1;  // of a column in cg_step_bulk_kernel
     DevBuf b2, b3, rows, tab, off;
 };
 
@@ -868,6 +869,9 @@ static int ensure_xmarch(eqd_grid *G) {
     C.s2 = (float)(gc.mu * kD2Int[4].v() * hi * hi);
     for (int k = 0; k < 4; ++k) C.dlo[k] = (float)(kDb[k].v() * hi);
     E.lay = XLayout{gc.n1, gc.n2, gc.n3, g.n2p, gc.PS, gc.colstride, g.colstride};
+    // Chunks of 8,192 elements: a column alone at h = 20 m 15.7 ms (17.4 with
+    // 16,384, 15.0 with 4,096), 64 columns at h = 25 m 94 ms (93, 98).
+    E.nchunks = (int)std::max<long long>(1, (g.colstride + 8191) / 8192);
     E.ok = true;
     return EQD_OK;
 }
@@ -1068,7 +1072,9 @@ extern "C" int eqd_grid_create(const eqd_grid_desc *d, eqd_grid **out) {
         }
         G->sel32 = 1;
     }
-    G->nchunks = (int)std::max<long long>(1, (gc.colstride + 16383) / 16384);
+    // Chunks of 8,192 elements in the vector kernels: one FP64 column at 25^3 20.0
+    // ms (22.5 with 16,384; 17.5 with 4,096), 64 at h = 40 m 132 (130; 135).
+    G->nchunks = (int)std::max<long long>(1, (gc.colstride + 8191) / 8192);
 
     CUDA_OR_RETURN(cudaSetDevice(d->device));
     {
@@ -1309,7 +1315,7 @@ static IterPtrs<T> span_ptrs(eqd_grid *G, Workspace &W, const SolveParams &sp, c
     P.x64 = W.x64.as<double>() + c0 * gc.colstride;
     P.apply_part = W.apply_part.as<double>() + c0 * sp.ntiles * 2;
     P.res_part = W.res_part.as<double>() + c0 * nparts(G->m64) * 2;
-    P.rr_part = W.rr_part.as<double>() + c0 * G->nchunks * 2;
+    P.rr_part = W.rr_part.as<double>() + c0 * sp.nchunks * 2;
     return P;
 }
 
@@ -1382,7 +1388,7 @@ static void record_rest(eqd_grid *G, Workspace &W, int mixed, int fused, int k, 
                         const ColState &st0, const Span &sn) {
     IterPtrs<T> P = span_ptrs<T>(G, W, sp, st0, sn);
     const T *pk = fused ? dir_out(P, k) : P.p;  // this iteration's direction
-    const int nch = G->nchunks;
+    const int nch = sp.nchunks;
     const double *dinv64 = sp.precond ? G->dinv64.as<double>() : nullptr;
     const float *dinv32 = sp.precond ? G->dinv32.as<float>() : nullptr;
     // Split: a few CTAs per SM (grid-stride over the items) so they fit
@@ -1607,7 +1613,8 @@ struct SlotRun {
         if (xm) ntmax = std::max(ntmax, G->xm.g.nt2 * G->xm.g.nt3);
         CUDA_OR_RETURN(w.apply_part.ensure(sizeof(double) * 2 * cap * ntmax));
         CUDA_OR_RETURN(w.res_part.ensure(sizeof(double) * 2 * cap * std::max(nt64, G->nchunks)));
-        CUDA_OR_RETURN(w.rr_part.ensure(sizeof(double) * 2 * cap * G->nchunks));
+        const int nch = xm ? G->xm.nchunks : G->nchunks;
+        CUDA_OR_RETURN(w.rr_part.ensure(sizeof(double) * 2 * cap * nch));
         for (DevBuf *b : {&w.gamma, &w.beta, &w.rr_ref, &w.tol, &w.bnorm, &w.pp}) CUDA_OR_RETURN(b->ensure(sizeof(double) * cap));
         CUDA_OR_RETURN(w.iters.ensure(sizeof(int) * cap));
         CUDA_OR_RETURN(w.status.ensure(cap));
@@ -1630,7 +1637,7 @@ struct SlotRun {
         sp.itmax = o.itmax;
         sp.delta = o.reliable_delta > 0 ? o.reliable_delta : 0.01;
         sp.ntiles = xm ? G->xm.g.nt2 * G->xm.g.nt3 : sizeof(T) == 4 ? nt32 : nt64;
-        sp.nchunks = G->nchunks;
+        sp.nchunks = nch;
         sp.colstride = xm ? G->xm.g.colstride : gc.colstride;
         sp.xlayout = xm;
         if (xm) {

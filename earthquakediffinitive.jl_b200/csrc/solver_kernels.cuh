@@ -516,14 +516,20 @@ __global__ void __launch_bounds__(128, 16) cg_step_bulk_kernel(float *__restrict
             if (threadIdx.x == 0 && t + kVecStages < ntile) issue(t + kVecStages);
         }
         g0 += (unsigned)ntile;
-        const double rr = block_sum(acc, red);
-        __syncthreads();
-        const double pp = block_sum(accp, red);
-        if (threadIdx.x == 0) {
-            rr_part[((long long)col * sp.nchunks + chunk) * 2 + 0] = rr;
-            rr_part[((long long)col * sp.nchunks + chunk) * 2 + 1] = pp;
+        for (int o = 16; o > 0; o >>= 1) {
+            acc += __shfl_down_sync(0xffffffffu, acc, o);
+            accp += __shfl_down_sync(0xffffffffu, accp, o);
         }
-        __syncthreads();
+        if ((threadIdx.x & 31) == 0) {
+            red[threadIdx.x >> 5] = acc;
+            red[16 + (threadIdx.x >> 5)] = accp;
+        }
+        __syncthreads();  // (the next item's first barrier comes before red is written again)
+        if (threadIdx.x < 2) {
+            double t = 0.0;
+            for (unsigned w = 0; w < blockDim.x / 32; ++w) t += red[16 * threadIdx.x + w];
+            rr_part[((long long)col * sp.nchunks + chunk) * 2 + threadIdx.x] = t;
+        }
     }
 }
 
