@@ -199,7 +199,10 @@ def cpu_port_sample(cfg, ncols_sample, seed=0, threads=0):
 def apply_kernel_name(variant, n1, tile_rows, threads):
     """The FP32 CG apply kernel a launch variant runs: variants 9 and 10 are
     the ring march on the lines it is built for (a CTA of 2 x roundup32(t2 n1)
-    + roundup32(2 t2) threads), every other variant the plane march."""
+    + roundup32(2 t2) threads), 12 is the x1 march, every other variant the
+    plane march (11 runs whole iterations on chip; its apply is timed streamed)."""
+    if variant == 12:
+        return "xmarch_kernel"
     r32 = lambda x: (x + 31) // 32 * 32
     if variant >= 9 and threads == 2 * r32(tile_rows * n1) + r32(2 * tile_rows):
         return f"ring_march_kernel<n1={n1},t2={tile_rows}>"

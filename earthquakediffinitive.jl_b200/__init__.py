@@ -125,8 +125,9 @@ class CGSolver:
     as `hbm_budget_bytes` allows), `reliable_delta` is the mixed engine's
     residual-drop factor for an FP64 true-residual update; `variant` picks
     the FP32 stencil launch variant for this solver's calls (0: the grid's,
-    chosen by `autotune` on first use or pinned by `set_stencil_variant`;
-    k > 0: variant k - 1 of `autotune`'s list). `split` and `fuse` change
+    pinned by `autotune` or `set_stencil_variant`, else on chip where the grid
+    has a plan, else the x1 march; k > 0: variant k - 1 of `autotune`'s list).
+    `split` and `fuse` change
     only the schedule, never the result bits: `split=False` runs a large
     batch as one chain of kernels instead of two overlapping halves, and
     `fuse=True` forms the CG direction inside the stencil apply (slower on

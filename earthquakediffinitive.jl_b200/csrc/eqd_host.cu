@@ -2285,14 +2285,30 @@ extern "C" int eqd_stiffness_toeplitz(eqd_grid *G, const eqd_solve_opts *opts, d
     return EQD_OK;
 }
 
+// Whether streamed mixed-precision solves of this grid apply the x1 march.
+static int streams_xmarch(eqd_grid *G, bool &xm) {
+    xm = false;
+    if (G->pin >= 0 && G->pin != kResidentVariant && G->pin != kXMarchVariant) return EQD_OK;
+    int rc = ensure_resident<float>(G, G->res32);
+    if (rc || (G->res32.ok && G->pin != kXMarchVariant)) return rc;
+    rc = ensure_xmarch(G);
+    xm = !rc && G->xm.ok;
+    return rc;
+}
+
 template <typename T>
 static int profile_apply_impl(eqd_grid *G, int ncols, int warmup, int reps, double *ms, double *bytes) {
     const GridConst &gc = G->gc;
     DevBuf x, y, part;
-    const long long n = gc.colstride * (long long)ncols;
+    bool xm = false;
+    if (sizeof(T) == 4) {
+        int rc = streams_xmarch(G, xm);
+        if (rc) return rc;
+    }
+    const long long n = (xm ? G->xm.g.colstride : gc.colstride) * (long long)ncols;
     CUDA_OR_RETURN(x.ensure(sizeof(T) * n));
     CUDA_OR_RETURN(y.ensure(sizeof(T) * n));
-    if (sizeof(T) == 4 && !G->tuned) {
+    if (sizeof(T) == 4 && !xm && !G->tuned) {
         eqd_solve_opts o;
         eqd_default_opts(&o);
         int rc = tune_by_iterations(G, o, std::min(ncols, 1024));
@@ -2300,15 +2316,23 @@ static int profile_apply_impl(eqd_grid *G, int ncols, int warmup, int reps, doub
     }
     int nt = nparts(G->m64);
     for (int v = 0; v < kNumVariants; ++v) nt = std::max(nt, nparts(G->v32[v]));
+    if (xm) nt = std::max(nt, G->xm.g.nt2 * G->xm.g.nt3);
     CUDA_OR_RETURN(part.ensure(sizeof(double) * 2 * ncols * nt));
+    CUtensorMap map{};
+    if (xm) {
+        int rc = make_plane_map(G->xm.g, x.as<float>(), ncols, map);
+        if (rc) return rc;
+    }
     fill_random_kernel<T><<<1184, 256, 0, G->stream>>>(x.as<T>(), n, 12345ull);
     CUDA_OR_RETURN(cudaGetLastError());
     ColumnSet cs{};
-    for (int i = 0; i < warmup; ++i)
-        CUDA_OR_RETURN((launch_march<T, T, MODE_A>(G, x.as<T>(), y.as<T>(), cs, part.as<double>(), ncols)));
+    auto apply = [&]() -> cudaError_t {
+        if (xm) return launch_xmarch(G, map, y.as<float>(), nullptr, part.as<double>(), 0, ncols, G->stream);
+        return launch_march<T, T, MODE_A>(G, x.as<T>(), y.as<T>(), cs, part.as<double>(), ncols);
+    };
+    for (int i = 0; i < warmup; ++i) CUDA_OR_RETURN(apply());
     CUDA_OR_RETURN(cudaEventRecord(G->ev0, G->stream));
-    for (int i = 0; i < reps; ++i)
-        CUDA_OR_RETURN((launch_march<T, T, MODE_A>(G, x.as<T>(), y.as<T>(), cs, part.as<double>(), ncols)));
+    for (int i = 0; i < reps; ++i) CUDA_OR_RETURN(apply());
     CUDA_OR_RETURN(cudaEventRecord(G->ev1, G->stream));
     CUDA_OR_RETURN(cudaEventSynchronize(G->ev1));
     float t = 0.f;
@@ -2341,7 +2365,8 @@ extern "C" int eqd_autotune(eqd_grid *G, int32_t ncols, int32_t *selected, doubl
         int rc = tune_by_iterations(G, o, ncols, true);
         if (rc) return rc;
     }
-    if (selected) *selected = G->pin >= 0 ? G->pin : G->sel32;
+    // (Nothing pinned: what the grid's solves have run with.)
+    if (selected) *selected = G->pin >= 0 ? G->pin : G->res32.ok ? kResidentVariant : G->xm.ok ? kXMarchVariant : G->sel32;
     if (nvariants) *nvariants = kAllVariants;
     for (int v = kNumVariants; v < kAllVariants; ++v) {
         if (ms_per_variant) ms_per_variant[v] = G->tune_ms[v];
