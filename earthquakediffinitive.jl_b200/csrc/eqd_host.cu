@@ -315,9 +315,12 @@ static MarchCfg segmented(const MarchCfg &m, long long groups, int num_sms) {
 }
 
 // Columns that a launch is split for: with flags (reliable updates, columns
-// that enter) four of them at most; where more are flagged the kernel joins
-// segments again, and where none is, more CTAs would only have to leave.
-static int flagged_cols(const ColumnSet &cs, int ncols) { return cs.flag ? std::min(ncols, 4) : ncols; }
+// that enter) as many as are flagged in most iterations, a column in 64 (five
+// times in about 320) and at least four; where more are flagged the kernel
+// joins segments again, and where none is, more CTAs would only have to leave.
+static int flagged_cols(const ColumnSet &cs, int ncols) {
+    return cs.flag ? std::min(ncols, std::max(4, ncols / 64)) : ncols;
+}
 
 template <typename T>
 static void fill_op(OpConst<T> &C, const GridConst &gc, const double h[3]) {

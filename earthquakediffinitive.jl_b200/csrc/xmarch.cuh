@@ -31,10 +31,10 @@
 // What bounds it: instruction issue (0.58 of the schedulers' slots, 256
 // instructions a line and step). Measured at h = 20 m, 48 columns: 201 us, the
 // plane march 360; 320-thread tiles of 16 x 10 lines (96 registers, spilling)
-// 309. 96 columns' solves there 338 ms (458 with the plane march), ten columns
-// at h = 25 m 229 ms (370).
+// 309. 96 columns' solves there 293 ms (458 with the plane march and its
+// vector kernels), ten columns at h = 25 m 193 ms (370).
 //
-// Dot products p.q and p.p are summed per (column, tile) in a fixed order.
+// Dot products p.q and q.q are summed per (column, tile) in a fixed order.
 #pragma once
 #include <cuda.h>
 
