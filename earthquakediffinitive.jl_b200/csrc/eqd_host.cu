@@ -817,7 +817,7 @@ static int ensure_xmarch(eqd_grid *G) {
     std::vector<int> b2, b3, off;
     std::vector<float> tab, rows((size_t)gc.n1 * 16, 0.f);
     // Tiles start every fourth line along x2 (a tiled copy starts on 16 bytes).
-    if (!x_tiles(gc.n2, 1, kXT2, 4, b2) || !x_tiles(gc.n3, 1, kXT3, 1, b3) ||
+    if (!x_offsets_fit(gc.n1, gc.n2, gc.n3) || !x_tiles(gc.n2, 1, kXT2, 4, b2) || !x_tiles(gc.n3, 1, kXT3, 1, b3) ||
         !fill_res_tables<float>(gc.n2, gc.n3, G->h[1], G->h[2], gc.mu, tab, off))
         return EQD_OK;
     E.smem = xmarch_smem(gc.n1);
@@ -850,7 +850,7 @@ static int ensure_xmarch(eqd_grid *G) {
     g.n2 = gc.n2;
     g.n3 = gc.n3;
     g.n2p = x_row_length(gc.n2);
-    g.colstride = 6LL * gc.n1 * gc.n3 * g.n2p;
+    g.colstride = x_column(gc.n1, gc.n2, gc.n3);
     g.nt2 = (int)b2.size() - 1;
     g.nt3 = (int)b3.size() - 1;
     g.b2 = E.b2.as<int>();
@@ -1262,7 +1262,7 @@ static int resolve_chunk(eqd_grid *G, const eqd_solve_opts &o, int ncols, int pr
     // x64 + r, p, q (+ d) (+ the second direction buffer of the fused update).
     // (The x1 march keeps its residuals in a second layout while they are formed, and pads x2 lines.)
     const int nvec = 3 + (prec == EQD_PREC_MIXED ? 2 : 0) + ((o.flags & EQD_FLAG_FUSE) ? 1 : 0);
-    const size_t per_col = (size_t)std::max(gc.colstride, 6LL * gc.n1 * gc.n3 * x_row_length(gc.n2)) * (8 + (size_t)nvec * (prec == EQD_PREC_MIXED ? 4 : 8)) +
+    const size_t per_col = (size_t)std::max(gc.colstride, x_column(gc.n1, gc.n2, gc.n3)) * (8 + (size_t)nvec * (prec == EQD_PREC_MIXED ? 4 : 8)) +
                            (size_t)16 * gc.nf + 1024;
     size_t budget = o.hbm_budget_bytes;
     if (budget == 0) {
@@ -3062,7 +3062,7 @@ extern "C" int eqd_server_add_grid(eqd_server *S, eqd_grid *G, int32_t slots) {
     const GridConst &gc = G->gc;
     const int mixed = S->opts.precision == EQD_PREC_MIXED;
     const int nvec = 3 + (mixed ? 2 : 0) + ((S->opts.flags & EQD_FLAG_FUSE) ? 1 : 0);  // as resolve_chunk
-    const size_t per_slot = (size_t)std::max(gc.colstride, 6LL * gc.n1 * gc.n3 * x_row_length(gc.n2)) * (8 + (size_t)nvec * (mixed ? 4 : 8)) + (size_t)16 * gc.nf + 1024;
+    const size_t per_slot = (size_t)std::max(gc.colstride, x_column(gc.n1, gc.n2, gc.n3)) * (8 + (size_t)nvec * (mixed ? 4 : 8)) + (size_t)16 * gc.nf + 1024;
     std::unique_ptr<SrvGrid> g(new SrvGrid());
     {
         std::lock_guard<std::mutex> lk(S->mu);

@@ -39,6 +39,7 @@
 #include <cuda.h>
 
 #include "resident_cg.cuh"
+#include "xmarch_plan.h"
 
 namespace eqd {
 
@@ -53,10 +54,8 @@ constexpr int kXF2 = kXR2a * kXT3 + 16, kXF3 = kXT2 * (kXT3 + 4) + 16;  // one s
 constexpr int kXF = 2 * (kXF2 + kXF3);                  // one step's F: both sides of F_2, then of F_3
 static_assert(kXSS % 32 == 16 && kXF2 % 32 == 16 && kXF3 % 32 == 16, "the two sides of a warp's lines fall on distinct banks");
 static_assert(kXPlane * 4 % 128 == 0, "a plane starts on a 128-byte boundary");
-constexpr int kXLead = 3;                               // x2 line i2 is stored at kXLead + i2
 constexpr int kXSmemRows = 128 + kXRing * kXPlane * 4;  // byte offset of the x1 rows
 constexpr int xmarch_smem(int n1) { return kXSmemRows + n1 * 16 * 4 + kXRing * kXF * 4; }
-inline int x_row_length(int n2) { return (n2 + kXLead + 3) / 4 * 4; }
 
 struct XGeom {
     int n1, n2, n3, n2p;
@@ -515,31 +514,6 @@ __global__ void xref_kernel(XLayout g, double *__restrict__ ref, float *__restri
     float *at = v + col * g.cnew + ((sc * g.n1 + x) * g.n3 + i3) * g.n2p + i2 + kXLead;
     if (TO) *at = (float)ref[gid];
     else ref[gid] = (double)*at;
-}
-
-// Host: tile bounds along an axis of n nodes, at most `width` lines a tile,
-// from `first` to n - 1 in multiples of `step`, as few tiles as possible. A
-// tile sees two lines of F and four of p beyond its own: no inner bound may
-// have a closure row that reaches further (rows 0 .. 3 read up to row 5, row 3
-// three lines back).
-inline bool x_tiles(int n, int first, int width, int step, std::vector<int> &b) {
-    const int end = n - 1;
-    std::vector<int> best(end + 1, 1 << 20), from(end + 1, -1);
-    best[first] = 0;
-    for (int e = first + 1; e <= end; ++e) {
-        if (e < end && ((e - first) % step || e < 4 || e > n - 4 || e == 5 || e == n - 5)) continue;
-        for (int a = std::max(first, e - width); a < e; ++a)
-            if (best[a] + 1 < best[e]) {
-                best[e] = best[a] + 1;
-                from[e] = a;
-            }
-    }
-    if (best[end] >= 1 << 20) return false;
-    b.clear();
-    for (int e = end; e != first; e = from[e]) b.push_back(e);
-    b.push_back(first);
-    std::reverse(b.begin(), b.end());
-    return true;
 }
 
 }  // namespace eqd
