@@ -329,7 +329,7 @@ resident_cg_kernel(const __grid_constant__ ResCoef<T> C, const __grid_constant__
     T *F3 = reinterpret_cast<T *>(smem_raw + G::oF3);
     T *tab = reinterpret_cast<T *>(smem_raw + G::oTab);  // x2 row classes, then x3
     int *off = reinterpret_cast<int *>(smem_raw + G::oOff);
-    double *red = reinterpret_cast<double *>(smem_raw + G::oRed);  // [rank][8], [warp][8], then alpha, beta, stop
+    double *red = reinterpret_cast<double *>(smem_raw + G::oRed);  // [rank][8], [warp][8], then alpha, beta, stop, sure
     double *wred = red + kResMaxTeam * 8;
     volatile double *step = wred + kResMaxWarps * 8;
     ResLine *lines = reinterpret_cast<ResLine *>(smem_raw + G::oLine);
@@ -593,7 +593,9 @@ resident_cg_kernel(const __grid_constant__ ResCoef<T> C, const __grid_constant__
         // ---- alpha, beta and the decision, by warp 0 of each CTA --------------
         // The next residual's norm from the same sums, |r - a q|^2 =
         // |r|^2 - 2 a r.q + a^2 q.q: no second exchange. |r|^2 is summed anew
-        // each time, so its rounding does not build up.
+        // each time, so its rounding does not build up; and where FP64 would
+        // stop on the difference, or it is small, the new residual is summed
+        // too (below).
         if (warp == 0) {
             if constexpr (GRID) {
                 c1 = 0.0;
@@ -613,6 +615,7 @@ resident_cg_kernel(const __grid_constant__ ResCoef<T> C, const __grid_constant__
             if (breakdown || !isfinite(alpha)) alpha = 0.0;
             const double ad = (double)(T)alpha;
             const double rr = fmax(gamma - 2.0 * ad * rq + ad * ad * qq, 0.0);
+            bool sure = true;
             ++iters;
             if (breakdown) {
                 if (mixed) flag = 1;  // let the true residual decide
@@ -621,8 +624,8 @@ resident_cg_kernel(const __grid_constant__ ResCoef<T> C, const __grid_constant__
                 status = COL_NONFINITE;
             } else if (mixed) {
                 if (rr <= tol * tol || rr <= sp.delta * sp.delta * rr_ref || iters >= itmax) flag = 1;
-            } else if (sqrt(rr) <= tol) {
-                status = COL_CONVERGED;
+            } else if (sqrt(rr) <= tol || rr <= 1e-10 * (gamma + ad * ad * qq)) {
+                sure = false;
             } else if (iters >= itmax) {
                 status = COL_MAXITER;
             }
@@ -634,11 +637,13 @@ resident_cg_kernel(const __grid_constant__ ResCoef<T> C, const __grid_constant__
                 step[0] = alpha;
                 step[1] = beta;
                 step[2] = stop || k + 1 >= kmax ? 1.0 : 0.0;
+                step[3] = sure ? 1.0 : 0.0;
             }
         }
         __syncthreads();
-        const T at = (T)step[0], b = (T)step[1];
-        const bool last = step[2] != 0.0;
+        const T at = (T)step[0];
+        T b = (T)step[1];
+        bool last = step[2] != 0.0;
         if (has) {
 #pragma unroll
             for (int x = 0; x < XH; ++x)
@@ -647,6 +652,61 @@ resident_cg_kernel(const __grid_constant__ ResCoef<T> C, const __grid_constant__
                     xs[x][c] += at * pv[x][c];
                     r[x][c] -= at * q[x][c];
                 }
+        }
+        if constexpr (sizeof(T) == 8) {
+            if (step[3] == 0.0) {
+                // The new residual's own norm, exchanged like the sums above in
+                // a place that they leave free. FP64 has no true residual to
+                // correct a decision, and the norm from the sums is a
+                // difference: below about 1e-14 |r|^2 of the old residual it is
+                // rounding (a right-hand side within 1e-9 of an eigenvector was
+                // called converged after one iteration). Once a column, as a
+                // rule.
+                constexpr int kOwn = 5;
+                double s = 0.0;
+                if (has) {
+#pragma unroll
+                    for (int x = 0; x < XH; ++x)
+#pragma unroll
+                        for (int c = 0; c < 3; ++c) s += r[x][c] * r[x][c];
+                }
+                auto warp_sum = [](double v) {
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                    return v;
+                };
+                s = warp_sum(s);
+                if (lane == 0) wred[warp * 8 + kOwn] = s;
+                __syncthreads();
+                if (warp == 0) {
+                    s = warp_sum(lane < kResMaxWarps ? wred[lane * 8 + kOwn] : 0.0);  // absent warps hold zero
+                    if constexpr (GRID) {
+                        if (lane == 0) __stcg(team_red + rank * 8 + kOwn, s);
+                    } else if (lane < M) {
+                        *(M > 1 ? map_cluster(red + rank * 8 + kOwn, lane) : red + kOwn) = s;
+                    }
+                }
+                if (!meet()) return;
+                if (warp == 0) {
+                    s = 0.0;
+                    if constexpr (GRID) {
+                        for (int w = lane; w < M; w += 32) s += __ldcg(team_red + w * 8 + kOwn);
+                    } else if (lane < kResMaxTeam) {
+                        s = red[lane * 8 + kOwn];  // ranks beyond M hold zero
+                    }
+                    const double rr = warp_sum(s);
+                    if (sqrt(rr) <= tol) status = COL_CONVERGED;
+                    else if (iters >= itmax) status = COL_MAXITER;
+                    else beta = rr / gamma;
+                    if (lane == 0) {
+                        step[1] = beta;
+                        if (status != COL_ACTIVE) step[2] = 1.0;
+                    }
+                }
+                __syncthreads();
+                b = step[1];
+                last = step[2] != 0.0;
+            }
         }
         if (last) break;
         if (has) {
