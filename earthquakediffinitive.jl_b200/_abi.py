@@ -65,7 +65,8 @@ EXPORTS = [
     "eqd_grid_create", "eqd_grid_destroy", "eqd_grid_info", "eqd_grid_fault_axes",
     "eqd_apply", "eqd_cg_solve", "eqd_shear_traction", "eqd_stiffness_exact",
     "eqd_stiffness_columns", "eqd_stiffness_columns_device", "eqd_stiffness_toeplitz", "eqd_diag",
-    "eqd_profile_apply", "eqd_autotune", "eqd_set_variant", "eqd_test_inject_wait_timeout", "eqd_assemble",
+    "eqd_profile_apply", "eqd_autotune", "eqd_set_variant", "eqd_test_inject_wait_timeout",
+    "eqd_test_inject_failure", "eqd_assemble",
     "eqd_tune_chunk",
     "eqd_kmat_create", "eqd_kmat_gemv", "eqd_kmat_gemv_device", "eqd_kmat_destroy", "eqd_kmat_gemv_static",
     "eqd_server_create", "eqd_server_add_grid", "eqd_server_submit", "eqd_server_wait",

@@ -442,6 +442,7 @@ struct eqd_grid {
     std::mutex mtx;
     std::vector<double> x2f, x3f;
     int tile_rows = 0;
+    bool test_fail_launch = false; // eqd_test_inject_failure: the next CG launch that is recorded fails on the host
     int test_drop_plane = -1;      // eqd_test_inject_wait_timeout: the next ring launch never copies this plane
     unsigned test_poll_limit = 0;
 };
@@ -1331,25 +1332,37 @@ static T *dir_in(const IterPtrs<T> &P, int k) { return (k & 1) ? P.p2 : P.p; }
 template <typename T>
 static T *dir_out(const IterPtrs<T> &P, int k) { return (k & 1) ? P.p : P.p2; }
 
+// Returns a launch's error from a function of CUDA errors.
+#define EQD_TRY(call)                                \
+    do {                                             \
+        const cudaError_t try_e = (call);            \
+        if (try_e != cudaSuccess) return try_e;      \
+    } while (0)
+
+// A pending eqd_test_inject_failure: the launch is not made.
+static bool injected_launch_error(eqd_grid *G) {
+    const bool f = G->test_fail_launch;
+    G->test_fail_launch = false;
+    return f;
+}
+
 // The stencil apply of CG iteration k (q = A p, partial p.q); fused: with
 // p = r + beta p formed on the way in.
 template <typename T>
-static void record_apply(eqd_grid *G, Workspace &W, int generic, int fused, int k, const SolveParams &sp,
+static cudaError_t record_apply(eqd_grid *G, Workspace &W, int generic, int fused, int k, const SolveParams &sp,
                          const ColState &st0, const Span &sn) {
     IterPtrs<T> P = span_ptrs<T>(G, W, sp, st0, sn);
-    if (sp.xlayout) {
-        launch_xmarch(G, W.pmap, (float *)P.q, P.cs.status, P.apply_part, sn.c0, sn.n, sn.s);
-    } else if (generic) {
-        launch_march<T, T, MODE_AP>(G, P.p, P.q, P.cs, P.apply_part, sn.n, -1, sn.s);
-    } else if (fused) {
+    if (injected_launch_error(G)) return cudaErrorLaunchOutOfResources;
+    if (sp.xlayout) return launch_xmarch(G, W.pmap, (float *)P.q, P.cs.status, P.apply_part, sn.c0, sn.n, sn.s);
+    if (generic) return launch_march<T, T, MODE_AP>(G, P.p, P.q, P.cs, P.apply_part, sn.n, -1, sn.s);
+    if (fused) {
         ColumnSet cs = P.cs;
         cs.pold = dir_in(P, k);
         cs.pnew = dir_out(P, k);
         cs.beta = P.st.beta;
-        launch_march<T, T, MODE_AF>(G, P.r, P.q, cs, P.apply_part, sn.n, -1, sn.s);
-    } else {
-        launch_march<T, T, MODE_A>(G, P.p, P.q, P.cs, P.apply_part, sn.n, -1, sn.s);
+        return launch_march<T, T, MODE_AF>(G, P.r, P.q, cs, P.apply_part, sn.n, -1, sn.s);
     }
+    return launch_march<T, T, MODE_A>(G, P.p, P.q, P.cs, P.apply_part, sn.n, -1, sn.s);
 }
 
 // CTA size of the vector kernels inside the iterations: small enough to fit
@@ -1366,7 +1379,7 @@ static constexpr int kVecCtasPerSm = 4;
 
 // Mixed precision: the flagged columns' FP64 true residual.
 template <typename T>
-static void record_reliable(eqd_grid *G, const IterPtrs<T> &P, const SolveParams &sp, const Span &sn) {
+static cudaError_t record_reliable(eqd_grid *G, const IterPtrs<T> &P, const SolveParams &sp, const Span &sn) {
     // One CTA per item: in most iterations no column is flagged and every
     // CTA returns at once.
     const unsigned items = (unsigned)((long long)sn.n * G->nchunks);
@@ -1375,19 +1388,21 @@ static void record_reliable(eqd_grid *G, const IterPtrs<T> &P, const SolveParams
     ColumnSet cf = P.cs;
     cf.flag = P.st.flag;
     cf.dinv = sp.precond ? G->dinv64.as<double>() : nullptr;
-    launch_march<double, float, MODE_RHS>(G, P.x64, sp.xlayout ? (float *)P.p2 : (float *)P.r, cf, P.res_part, sn.n, -1,
-                                          sn.s);
+    EQD_TRY(cudaGetLastError());
+    EQD_TRY((launch_march<double, float, MODE_RHS>(G, P.x64, sp.xlayout ? (float *)P.p2 : (float *)P.r, cf, P.res_part,
+                                                   sn.n, -1, sn.s)));
     if (sp.xlayout)
         launch_xresidual(G, (float *)P.r, (float *)P.p, (const float *)P.p2, P.st.status, P.st.flag, sn.n, sn.s);
     SolveParams sp2 = sp;
     sp2.ntiles = nparts(G->m64);
     cg_true_residual_kernel<<<(unsigned)((sn.n + 3) / 4), 128, 0, sn.s>>>(P.st, sp2, P.res_part, sn.n, 1);
+    return cudaGetLastError();
 }
 
 // The rest of iteration k: x, r updates; scalars; reliable update (mixed);
 // the next direction (unless the next apply forms it).
 template <typename T>
-static void record_rest(eqd_grid *G, Workspace &W, int mixed, int fused, int k, const SolveParams &sp,
+static cudaError_t record_rest(eqd_grid *G, Workspace &W, int mixed, int fused, int k, const SolveParams &sp,
                         const ColState &st0, const Span &sn) {
     IterPtrs<T> P = span_ptrs<T>(G, W, sp, st0, sn);
     const T *pk = fused ? dir_out(P, k) : P.p;  // this iteration's direction
@@ -1408,8 +1423,8 @@ static void record_rest(eqd_grid *G, Workspace &W, int mixed, int fused, int k, 
         cg_step_bulk_kernel<<<nb, kVecThreads, kStepBulkSmem, sn.s>>>(P.d, (float *)P.r, (float *)P.p, (const float *)P.q,
                                                                       P.apply_part, P.st, sp, P.rr_part, sn.n, err);
         cg_check_kernel<<<sb, 128, 0, sn.s>>>(P.st, sp, P.apply_part, P.rr_part, sn.n);
-        record_reliable<T>(G, P, sp, sn);
-        return;
+        EQD_TRY(cudaGetLastError());
+        return record_reliable<T>(G, P, sp, sn);
     }
     if (mixed) {
         cg_update_bulk_kernel<float, float><<<nb, kVecThreads, kUpdateBulkSmem, sn.s>>>(
@@ -1421,7 +1436,8 @@ static void record_rest(eqd_grid *G, Workspace &W, int mixed, int fused, int k, 
                                                               P.rr_part, dinv64, sn.n);
     }
     cg_scalar_kernel<<<sb, 128, 0, sn.s>>>(P.st, sp, P.apply_part, P.rr_part, sn.n, mixed);
-    if (mixed) record_reliable<T>(G, P, sp, sn);
+    EQD_TRY(cudaGetLastError());
+    if (mixed) EQD_TRY(record_reliable<T>(G, P, sp, sn));
     if (!fused) {
         const T *dinvT = (const T *)(sizeof(T) == 4 ? (const void *)dinv32 : (const void *)dinv64);
         if (mixed)
@@ -1429,6 +1445,7 @@ static void record_rest(eqd_grid *G, Workspace &W, int mixed, int fused, int k, 
         else
             cg_pupdate_kernel<T><<<nb, kVecThreads, 0, sn.s>>>(P.p, P.r, P.st, sp, nullptr, dinvT, sn.n);
     }
+    return cudaGetLastError();
 }
 
 // Capture kIter CG iterations over `cap` slots. Large batches are split in
@@ -1436,15 +1453,15 @@ static void record_rest(eqd_grid *G, Workspace &W, int mixed, int fused, int k, 
 // arithmetic-bound apply of one half runs while the memory-bound vector
 // updates of the other half stream through HBM.
 template <typename T>
-static void record_iterations(eqd_grid *G, Workspace &W, int cap, int mixed, int generic, int fused,
+static cudaError_t record_iterations(eqd_grid *G, Workspace &W, int cap, int mixed, int generic, int fused,
                               const SolveParams &sp, const ColState &st, int kIter, bool split) {
     if (!split) {
         const Span all{0, cap, G->stream, false};
         for (int k = 0; k < kIter; ++k) {
-            record_apply<T>(G, W, generic, fused, k, sp, st, all);
-            record_rest<T>(G, W, mixed, fused, k, sp, st, all);
+            EQD_TRY(record_apply<T>(G, W, generic, fused, k, sp, st, all));
+            EQD_TRY(record_rest<T>(G, W, mixed, fused, k, sp, st, all));
         }
-        return;
+        return cudaSuccess;
     }
     // Applies on normal-priority streams, the rest of each iteration on
     // high-priority streams (node priorities are kept at instantiation), so
@@ -1452,45 +1469,49 @@ static void record_iterations(eqd_grid *G, Workspace &W, int cap, int mixed, int
     const int h0 = cap / 2;
     const Span A{0, h0, G->stream, true}, B{h0, cap - h0, G->stream2, true};
     const Span Ah{0, h0, G->stream_hi, true}, Bh{h0, cap - h0, G->stream2_hi, true};
-    cudaEventRecord(G->evFork, A.s);
-    for (cudaStream_t t : {B.s, Ah.s, Bh.s}) cudaStreamWaitEvent(t, G->evFork, 0);
+    EQD_TRY(cudaEventRecord(G->evFork, A.s));
+    for (cudaStream_t t : {B.s, Ah.s, Bh.s}) EQD_TRY(cudaStreamWaitEvent(t, G->evFork, 0));
     for (int k = 0; k < kIter; ++k) {
         if (k > 0) {
-            cudaStreamWaitEvent(A.s, G->evB, 0);      // B's previous apply is done
-            cudaStreamWaitEvent(A.s, G->evArest, 0);  // A's previous direction is ready
+            EQD_TRY(cudaStreamWaitEvent(A.s, G->evB, 0));      // B's previous apply is done
+            EQD_TRY(cudaStreamWaitEvent(A.s, G->evArest, 0));  // A's previous direction is ready
         }
-        record_apply<T>(G, W, generic, fused, k, sp, st, A);
-        cudaEventRecord(G->evA, A.s);
-        cudaStreamWaitEvent(B.s, G->evA, 0);          // B's apply follows A's
-        if (k > 0) cudaStreamWaitEvent(B.s, G->evBrest, 0);
-        record_apply<T>(G, W, generic, fused, k, sp, st, B);
-        cudaEventRecord(G->evB, B.s);
-        cudaStreamWaitEvent(Ah.s, G->evA, 0);
-        record_rest<T>(G, W, mixed, fused, k, sp, st, Ah);
-        cudaEventRecord(G->evArest, Ah.s);
-        cudaStreamWaitEvent(Bh.s, G->evB, 0);
-        record_rest<T>(G, W, mixed, fused, k, sp, st, Bh);
-        cudaEventRecord(G->evBrest, Bh.s);
+        EQD_TRY(record_apply<T>(G, W, generic, fused, k, sp, st, A));
+        EQD_TRY(cudaEventRecord(G->evA, A.s));
+        EQD_TRY(cudaStreamWaitEvent(B.s, G->evA, 0));          // B's apply follows A's
+        if (k > 0) EQD_TRY(cudaStreamWaitEvent(B.s, G->evBrest, 0));
+        EQD_TRY(record_apply<T>(G, W, generic, fused, k, sp, st, B));
+        EQD_TRY(cudaEventRecord(G->evB, B.s));
+        EQD_TRY(cudaStreamWaitEvent(Ah.s, G->evA, 0));
+        EQD_TRY(record_rest<T>(G, W, mixed, fused, k, sp, st, Ah));
+        EQD_TRY(cudaEventRecord(G->evArest, Ah.s));
+        EQD_TRY(cudaStreamWaitEvent(Bh.s, G->evB, 0));
+        EQD_TRY(record_rest<T>(G, W, mixed, fused, k, sp, st, Bh));
+        EQD_TRY(cudaEventRecord(G->evBrest, Bh.s));
     }
-    cudaEventRecord(G->evJoin, B.s);
-    cudaStreamWaitEvent(A.s, G->evJoin, 0);
-    cudaStreamWaitEvent(A.s, G->evArest, 0);
-    cudaStreamWaitEvent(A.s, G->evBrest, 0);
+    EQD_TRY(cudaEventRecord(G->evJoin, B.s));
+    EQD_TRY(cudaStreamWaitEvent(A.s, G->evJoin, 0));
+    EQD_TRY(cudaStreamWaitEvent(A.s, G->evArest, 0));
+    EQD_TRY(cudaStreamWaitEvent(A.s, G->evBrest, 0));
+    return cudaSuccess;
 }
 
 // Resident iterations of `cap` slots: every active column runs until it needs
 // its true residual (mixed) or is done, at most kmax iterations, `rounds`
 // times.
 template <typename T>
-static void record_resident(eqd_grid *G, Workspace &W, int cap, int mixed, const SolveParams &sp, const ColState &st,
+static cudaError_t record_resident(eqd_grid *G, Workspace &W, int cap, int mixed, const SolveParams &sp, const ColState &st,
                             int kmax, int rounds) {
     const Span all{0, cap, G->stream, false};
     IterPtrs<T> P = span_ptrs<T>(G, W, sp, st, all);
     T *x = sizeof(T) == 4 ? (T *)P.d : (T *)P.x64;
     for (int k = 0; k < rounds; ++k) {
-        launch_resident<T>(G, sizeof(T) == 4 ? G->res32 : G->res64, x, P.r, P.p, P.st, sp, mixed, kmax, cap, G->stream);
-        if (mixed) record_reliable<T>(G, P, sp, all);
+        if (injected_launch_error(G)) return cudaErrorLaunchOutOfResources;
+        EQD_TRY(launch_resident<T>(G, sizeof(T) == 4 ? G->res32 : G->res64, x, P.r, P.p, P.st, sp, mixed, kmax, cap,
+                                   G->stream));
+        if (mixed) EQD_TRY(record_reliable<T>(G, P, sp, all));
     }
+    return cudaSuccess;
 }
 
 // Jacobi weights dinv = 1 / diag(A) (zeros floored to 1), computed once per
@@ -1557,6 +1578,7 @@ struct SlotRun {
     SolveParams sp{};
     ColState st{};
     std::vector<int> hn, hc, hslot, hdst;
+    std::vector<int> seen;  // a slot's iterations at the last collect()
     std::vector<int8_t> hnew;
     PinnedArr<int> hit;     // per-slot iteration counts (read back every graph launch)
     PinnedArr<int8_t> hst;  // per-slot status
@@ -1662,6 +1684,7 @@ struct SlotRun {
         CUDA_OR_RETURN(hit.assign(cap, 0));
         CUDA_OR_RETURN(hst.assign(cap, (int8_t)COL_IDLE));
         hnew.assign(cap, 0);
+        seen.assign(cap, 0);
         tag.assign(cap, -1);
         hslot.resize(cap);
         hdst.resize(cap);
@@ -1690,11 +1713,19 @@ struct SlotRun {
         if (!w.graph || w.graph_key != kv) {
             if (w.graph) cudaGraphExecDestroy(w.graph);
             w.graph = nullptr;
-            cudaGraph_t g;
+            w.graph_key.clear();
+            cudaGraph_t g = nullptr;
+            cudaGetLastError();  // (an earlier call's, already reported)
             CUDA_OR_RETURN(cudaStreamBeginCapture(G->stream, cudaStreamCaptureModeThreadLocal));
-            if (resident) record_resident<T>(G, w, cap, mixed, sp, st, kmax, rounds);
-            else record_iterations<T>(G, w, cap, mixed, generic, fused, sp, st, kIter, split);
+            const cudaError_t re = resident
+                                       ? record_resident<T>(G, w, cap, mixed, sp, st, kmax, rounds)
+                                       : record_iterations<T>(G, w, cap, mixed, generic, fused, sp, st, kIter, split);
             cudaError_t ce = cudaStreamEndCapture(G->stream, &g);
+            if (re != cudaSuccess) {  // a graph without one of its kernels must not run
+                if (g) cudaGraphDestroy(g);
+                cudaGetLastError();
+                return fail(EQD_ERR_CUDA, std::string("recording the CG iterations: ") + cudaGetErrorString(re));
+            }
             if (ce != cudaSuccess) return fail(EQD_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(ce));
             ce = cudaGraphInstantiate(&w.graph, g, cudaGraphInstantiateFlagUseNodePriority);
             cudaGraphDestroy(g);
@@ -1733,7 +1764,7 @@ struct SlotRun {
             hn[s] = c.slip_node;
             hc[s] = c.slip_comp;
             hst[s] = COL_ACTIVE;
-            hit[s] = 0;
+            hit[s] = seen[s] = 0;
             hnew[s] = 1;
             ++held;
             if (dense) {
@@ -1841,6 +1872,9 @@ struct SlotRun {
         bool forced = false;
         for (int s = 0; s < cap; ++s) {
             if (tag[s] < 0) continue;
+            if (hst[s] == COL_ACTIVE && hit[s] <= seen[s])
+                return fail(EQD_ERR_CUDA, "a launch of CG iterations left an active column where it was");
+            seen[s] = hit[s];
             if (hst[s] == COL_ACTIVE && hit[s] > itmax + 2 * std::max(kIter, resident ? kmax * rounds : 0)) {  // defensive: the kernels stop at itmax
                 hst[s] = COL_MAXITER;
                 forced = true;
@@ -2452,6 +2486,14 @@ extern "C" int eqd_set_variant(eqd_grid *G, int32_t variant) {
         G->sel32 = variant;
         G->tuned = true;
     }
+    return EQD_OK;
+}
+
+extern "C" int eqd_test_inject_failure(eqd_grid *G, int32_t where) {
+    if (!G || where != EQD_FAIL_CG_LAUNCH) return fail(EQD_ERR_ARG, "invalid argument");
+    std::lock_guard<std::mutex> lk(G->mtx);
+    if (G->served) return fail(EQD_ERR_ARG, "the grid is attached to a server");
+    G->test_fail_launch = true;
     return EQD_OK;
 }
 

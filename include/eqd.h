@@ -221,6 +221,13 @@ int eqd_set_variant(eqd_grid *grid, int32_t variant);
  * EQD_ERR_TIMEOUT; later calls run normally. One launch only. */
 int eqd_test_inject_wait_timeout(eqd_grid *grid, int32_t plane, uint32_t poll_limit);
 
+/* The same for errors of the host's own calls (no counterpart in the
+ * reference): EQD_FAIL_CG_LAUNCH, the next launch of CG iterations that this
+ * grid records is not made and reports an error; the call returns
+ * EQD_ERR_CUDA and later calls run normally. Once only. */
+#define EQD_FAIL_CG_LAUNCH 1
+int eqd_test_inject_failure(eqd_grid *grid, int32_t where);
+
 /* The assembled matrices of `split_node_system` (src/ElasticitySplitNode.jl:
  * 106-214) for callers that want them: which = 0 gives A = -H P (D+SAT) P,
  * which = 1 gives HP_DSAT = H P (D+SAT), CSR in reference DOF order (ntot
