@@ -443,6 +443,7 @@ struct eqd_grid {
     std::vector<double> x2f, x3f;
     int tile_rows = 0;
     bool test_fail_launch = false; // eqd_test_inject_failure: the next CG launch that is recorded fails on the host
+    bool test_fail_plan = false;   // and the next allocation for the tables of a plan
     int test_drop_plane = -1;      // eqd_test_inject_wait_timeout: the next ring launch never copies this plane
     unsigned test_poll_limit = 0;
 };
@@ -673,13 +674,23 @@ static void res_launch_config(const ResDims &d, int warps, int teams, bool grid,
     cfg.numAttrs = 1;
 }
 
+// A table of a plan, on the device. (A plan that an error cut short is made anew
+// by the next call: a grid keeps to one kernel, and so a column to its bits.)
+static cudaError_t put_table(eqd_grid *G, DevBuf &b, const void *src, size_t bytes) {
+    if (G->test_fail_plan) {
+        G->test_fail_plan = false;
+        return cudaErrorMemoryAllocation;
+    }
+    const cudaError_t e = b.ensure(std::max<size_t>(bytes, 16));
+    return e == cudaSuccess && bytes ? cudaMemcpyAsync(b.p, src, bytes, cudaMemcpyHostToDevice, G->stream) : e;
+}
+
 // The team and the instance with the least work per column-iteration over the
 // team (whole K at h = 50 m: 8 CTAs of 8 x 16 lines 205 ms, 16 of 8 x 8 227 ms;
 // h = 100 m: 2 of 8 x 16 9.2 ms, 4 of 8 x 8 9.9 ms, 9 of them 15.1 ms).
 template <typename T>
 static int ensure_resident(eqd_grid *G, ResEngine &E) {
     if (E.tried) return EQD_OK;
-    E.tried = true;
     const GridConst &gc = G->gc;
     ResPlan best;
     double best_cost = 1e300;
@@ -736,16 +747,14 @@ static int ensure_resident(eqd_grid *G, ResEngine &E) {
         }
         return false;
     });
-    if (best_cost == 1e300) return EQD_OK;
-    E.d = best.d;
     std::vector<T> tab;
     std::vector<int> off;
-    if (!fill_res_tables<T>(gc.n2, gc.n3, G->h[1], G->h[2], gc.mu, tab, off)) return EQD_OK;
-    auto put = [&](DevBuf &b, const void *src, size_t bytes) -> cudaError_t {
-        cudaError_t e = b.ensure(std::max<size_t>(bytes, 16));
-        if (e == cudaSuccess && bytes) e = cudaMemcpyAsync(b.p, src, bytes, cudaMemcpyHostToDevice, G->stream);
-        return e;
-    };
+    if (best_cost == 1e300 || !fill_res_tables<T>(gc.n2, gc.n3, G->h[1], G->h[2], gc.mu, tab, off)) {
+        E.tried = true;
+        return EQD_OK;
+    }
+    E.d = best.d;
+    auto put = [&](DevBuf &b, const void *src, size_t bytes) { return put_table(G, b, src, bytes); };
     CUDA_OR_RETURN(put(E.ranks, best.ranks.data(), best.ranks.size() * sizeof(ResRank)));
     CUDA_OR_RETURN(put(E.chunks, best.chunks.data(), best.chunks.size() * sizeof(int)));
     CUDA_OR_RETURN(put(E.lines, best.lines.data(), best.lines.size() * sizeof(ResLine)));
@@ -772,7 +781,7 @@ static int ensure_resident(eqd_grid *G, ResEngine &E) {
         CUDA_OR_RETURN(cudaMemsetAsync(E.team_p.p, 0, sizeof(T) * 3 * cs * ctas, G->stream));
         CUDA_OR_RETURN(cudaStreamSynchronize(G->stream));
     }
-    E.ok = true;
+    E.tried = E.ok = true;
     return EQD_OK;
 }
 
@@ -813,14 +822,15 @@ static cudaError_t launch_resident(eqd_grid *G, const ResEngine &E, T *x, T *r, 
 static int ensure_xmarch(eqd_grid *G) {
     XEngine &E = G->xm;
     if (E.tried) return EQD_OK;
-    E.tried = true;
     const GridConst &gc = G->gc;
     std::vector<int> b2, b3, off;
     std::vector<float> tab, rows((size_t)gc.n1 * 16, 0.f);
     // Tiles start every fourth line along x2 (a tiled copy starts on 16 bytes).
     if (!x_offsets_fit(gc.n1, gc.n2, gc.n3) || !x_tiles(gc.n2, 1, kXT2, 4, b2) || !x_tiles(gc.n3, 1, kXT3, 1, b3) ||
-        !fill_res_tables<float>(gc.n2, gc.n3, G->h[1], G->h[2], gc.mu, tab, off))
+        !fill_res_tables<float>(gc.n2, gc.n3, G->h[1], G->h[2], gc.mu, tab, off)) {
+        E.tried = true;
         return EQD_OK;
+    }
     E.smem = xmarch_smem(gc.n1);
     CUDA_OR_RETURN(cudaFuncSetAttribute((const void *)xmarch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         xmarch_smem(EQD_MAX_N1)));
@@ -836,10 +846,7 @@ static int ensure_xmarch(eqd_grid *G) {
         const int e = std::min(i, gc.n1 - 1 - i);
         r[14] = (float)(-gc.hvol * (e < 4 ? kHw[e].v() : 1.0));
     }
-    auto put = [&](DevBuf &b, const void *src, size_t bytes) -> cudaError_t {
-        cudaError_t e = b.ensure(bytes);
-        return e == cudaSuccess ? cudaMemcpyAsync(b.p, src, bytes, cudaMemcpyHostToDevice, G->stream) : e;
-    };
+    auto put = [&](DevBuf &b, const void *src, size_t bytes) { return put_table(G, b, src, bytes); };
     CUDA_OR_RETURN(put(E.b2, b2.data(), b2.size() * sizeof(int)));
     CUDA_OR_RETURN(put(E.b3, b3.data(), b3.size() * sizeof(int)));
     CUDA_OR_RETURN(put(E.rows, rows.data(), rows.size() * sizeof(float)));
@@ -876,7 +883,7 @@ static int ensure_xmarch(eqd_grid *G) {
     // Chunks of 8,192 elements: a column alone at h = 20 m 15.7 ms (17.4 with
     // 16,384, 15.0 with 4,096), 64 columns at h = 25 m 94 ms (93, 98).
     E.nchunks = (int)std::max<long long>(1, (g.colstride + 8191) / 8192);
-    E.ok = true;
+    E.tried = E.ok = true;
     return EQD_OK;
 }
 
@@ -2490,10 +2497,10 @@ extern "C" int eqd_set_variant(eqd_grid *G, int32_t variant) {
 }
 
 extern "C" int eqd_test_inject_failure(eqd_grid *G, int32_t where) {
-    if (!G || where != EQD_FAIL_CG_LAUNCH) return fail(EQD_ERR_ARG, "invalid argument");
+    if (!G || (where != EQD_FAIL_CG_LAUNCH && where != EQD_FAIL_PLAN)) return fail(EQD_ERR_ARG, "invalid argument");
     std::lock_guard<std::mutex> lk(G->mtx);
     if (G->served) return fail(EQD_ERR_ARG, "the grid is attached to a server");
-    G->test_fail_launch = true;
+    (where == EQD_FAIL_CG_LAUNCH ? G->test_fail_launch : G->test_fail_plan) = true;
     return EQD_OK;
 }
 

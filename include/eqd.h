@@ -223,9 +223,11 @@ int eqd_test_inject_wait_timeout(eqd_grid *grid, int32_t plane, uint32_t poll_li
 
 /* The same for errors of the host's own calls (no counterpart in the
  * reference): EQD_FAIL_CG_LAUNCH, the next launch of CG iterations that this
- * grid records is not made and reports an error; the call returns
- * EQD_ERR_CUDA and later calls run normally. Once only. */
+ * grid records is not made and reports an error; EQD_FAIL_PLAN, the next
+ * allocation for the tables of the on-chip CG or of the x1 march fails. The
+ * call returns the error and later calls run normally. Once only. */
 #define EQD_FAIL_CG_LAUNCH 1
+#define EQD_FAIL_PLAN 2
 int eqd_test_inject_failure(eqd_grid *grid, int32_t where);
 
 /* The assembled matrices of `split_node_system` (src/ElasticitySplitNode.jl:
