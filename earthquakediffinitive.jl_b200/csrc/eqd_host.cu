@@ -1572,6 +1572,11 @@ struct ColDone {
 
 static int tune_by_iterations(eqd_grid *G, const eqd_solve_opts &o, int ncols, bool with_resident = false);
 
+// Whether the options and the pinned variant leave a solve to the on-chip CG.
+static bool allows_resident(const eqd_grid *G, const eqd_solve_opts &o) {
+    return o.precond != EQD_PRECOND_JACOBI && (G->pin < 0 || G->pin == kResidentVariant);
+}
+
 template <typename T>
 struct SlotRun {
     eqd_grid *G = nullptr;
@@ -1594,10 +1599,10 @@ struct SlotRun {
     int64_t launches = 0;
     static constexpr int kIter = 10;
 
-    // `tuning`: the caller times kIter iterations a launch. `projected`: every
-    // explicit right-hand side is in the range of P.
+    // `tuning`: the caller times kIter iterations a launch. `on_chip`: the
+    // explicit right-hand sides run resident (explicit_on_chip).
     int setup(eqd_grid *g, const eqd_solve_opts &o, int capacity, bool gen, bool dns, bool tuning = false,
-              bool projected = false) {
+              bool on_chip = false) {
         G = g;
         W = &G->ws;
         cap = capacity;
@@ -1606,15 +1611,15 @@ struct SlotRun {
         dense = dns;
         const GridConst &gc = G->gc;
         const long long ntot = 6LL * gc.n1 * gc.n2 * gc.n3;
-        resident = 0;
-        if ((!gen || projected) && o.precond != EQD_PRECOND_JACOBI && (G->pin < 0 || G->pin == kResidentVariant)) {
+        resident = gen && on_chip;
+        if (!gen && allows_resident(G, o)) {
             ResEngine &E = sizeof(T) == 4 ? G->res32 : G->res64;
             int rc = ensure_resident<T>(G, E);
             if (rc) return rc;
-            resident = E.ok && (!E.few || (gen && cap <= 4 * E.teams));
-            kmax = tuning ? kIter : 256;
-            rounds = mixed && !tuning ? 2 : 1;
+            resident = E.ok && !E.few;
         }
+        kmax = tuning ? kIter : 256;
+        rounds = mixed && !tuning ? 2 : 1;
         xm = 0;
         if (mixed && !gen && !resident && o.precond != EQD_PRECOND_JACOBI &&
             (G->pin < 0 || G->pin == kResidentVariant || G->pin == kXMarchVariant)) {
@@ -2027,31 +2032,40 @@ static bool rhs_in_range(const GridConst &gc, const double *b) {
     return true;
 }
 
+// The explicit right-hand sides that run on chip: those in the range of P, each
+// for itself, on a grid with a plan. Where the plan is a team that only a few
+// columns are better off with, all of them while they are at most four a team.
+// That number is the call's, whatever width the memory allows, so a right-hand
+// side's bits depend on the call only where it is crossed.
+template <typename T>
+static int explicit_on_chip(eqd_grid *G, const eqd_solve_opts &o, const BatchSpec &B, std::vector<char> &on) {
+    on.assign(B.ncols, 0);
+    if (!allows_resident(G, o)) return EQD_OK;
+    ResEngine &E = sizeof(T) == 4 ? G->res32 : G->res64;
+    int rc = ensure_resident<T>(G, E);
+    if (rc || !E.ok) return rc;
+    const size_t ntot = (size_t)6 * G->gc.n1 * G->gc.n2 * G->gc.n3;
+    int n = 0;
+    for (int i = 0; i < B.ncols; ++i) n += on[i] = rhs_in_range(G->gc, B.rhs + i * ntot);
+    if (E.few && n > 4 * E.teams) on.assign(B.ncols, 0);
+    return EQD_OK;
+}
+
 // Batched solve through the slot engine: columns enter as slots free up; K
 // columns go to the caller's device or host buffer as each column finishes.
+// `work`: the call's columns that run alike; adds to *stats and to unconv.
 template <typename T>
-static int run_batch(eqd_grid *G, const eqd_solve_opts &o, const BatchSpec &B, eqd_stats *stats) {
+static int run_columns(eqd_grid *G, const eqd_solve_opts &o, const BatchSpec &B, const std::vector<ColWork> &work,
+                       bool on_chip, eqd_stats *stats, int64_t &unconv_all) {
     const GridConst &gc = G->gc;
-    const int generic = B.rhs != nullptr;
+    const int generic = B.rhs != nullptr, ncols = (int)work.size();
     const long long ntot = 6LL * gc.n1 * gc.n2 * gc.n3;
     int chunk = 0;
-    int rc = resolve_chunk(G, o, B.ncols, o.precision, chunk);
+    int rc = resolve_chunk(G, o, ncols, o.precision, chunk);
     if (rc) return rc;
     SlotRun<T> R;
-    bool projected = generic;
-    for (int i = 0; i < B.ncols && projected; ++i) projected = rhs_in_range(gc, B.rhs + (size_t)i * ntot);
-    rc = R.setup(G, o, chunk, generic, B.slip_dense != nullptr, false, projected);
+    rc = R.setup(G, o, chunk, generic, B.slip_dense != nullptr, false, on_chip);
     if (rc) return rc;
-
-    std::vector<ColWork> work(B.ncols);
-    for (int i = 0; i < B.ncols; ++i) {
-        ColWork &c = work[i];
-        c.tag = i;
-        c.slip_node = B.slip_node ? B.slip_node[i] : -1;
-        c.slip_comp = B.slip_comp ? B.slip_comp[i] : 0;
-        c.slip_dense = B.slip_dense ? B.slip_dense + (size_t)i * 2 * gc.nf : nullptr;
-        c.rhs = B.rhs ? B.rhs + (size_t)i * ntot : nullptr;
-    }
     int64_t tot_it = 0, max_it = 0, unconv = 0;
     PinnedArr<double> &kstage = R.W->kstage;
     if (!generic && B.kcols && !B.kdev && kstage.n < 2 * gc.nf * chunk)
@@ -2081,12 +2095,12 @@ static int run_batch(eqd_grid *G, const eqd_solve_opts &o, const BatchSpec &B, e
     CUDA_OR_RETURN(cudaEventRecord(G->ev0, G->stream));
     int next = 0, finished = 0;
     std::vector<ColDone> done;
-    while (finished < B.ncols) {
+    while (finished < ncols) {
         // Explicit-RHS solves refill only an empty engine (their staging
         // buffer holds one wave of right-hand sides).
-        if (next < B.ncols && R.free_slots() > 0 && (!generic || R.held == 0)) {
+        if (next < ncols && R.free_slots() > 0 && (!generic || R.held == 0)) {
             int taken = 0;
-            rc = R.admit(work.data() + next, B.ncols - next, taken);
+            rc = R.admit(work.data() + next, ncols - next, taken);
             if (rc) return rc;
             next += taken;
         }
@@ -2134,7 +2148,7 @@ static int run_batch(eqd_grid *G, const eqd_solve_opts &o, const BatchSpec &B, e
     float ms = 0.f;
     cudaEventElapsedTime(&ms, G->ev0, G->ev1);
     if (stats) {
-        stats->solves += B.ncols;
+        stats->solves += ncols;
         stats->iterations += tot_it;
         stats->max_iterations = std::max<int64_t>(stats->max_iterations, max_it);
         stats->unconverged += unconv;
@@ -2142,6 +2156,35 @@ static int run_batch(eqd_grid *G, const eqd_solve_opts &o, const BatchSpec &B, e
         stats->device_seconds += ms * 1e-3;
         stats->precision = o.precision;
         stats->precond = o.precond;
+    }
+    unconv_all += unconv;
+    return EQD_OK;
+}
+
+template <typename T>
+static int run_batch(eqd_grid *G, const eqd_solve_opts &o, const BatchSpec &B, eqd_stats *stats) {
+    const GridConst &gc = G->gc;
+    const long long ntot = 6LL * gc.n1 * gc.n2 * gc.n3;
+    std::vector<char> on(B.ncols, 0);
+    if (B.rhs) {
+        int rc = explicit_on_chip<T>(G, o, B, on);
+        if (rc) return rc;
+    }
+    std::vector<ColWork> work[2];  // explicit right-hand sides: streamed, on chip
+    for (int i = 0; i < B.ncols; ++i) {
+        ColWork c;
+        c.tag = i;
+        c.slip_node = B.slip_node ? B.slip_node[i] : -1;
+        c.slip_comp = B.slip_comp ? B.slip_comp[i] : 0;
+        c.slip_dense = B.slip_dense ? B.slip_dense + (size_t)i * 2 * gc.nf : nullptr;
+        c.rhs = B.rhs ? B.rhs + (size_t)i * ntot : nullptr;
+        work[on[i] ? 1 : 0].push_back(c);
+    }
+    int64_t unconv = 0;
+    for (int k = 0; k < 2; ++k) {
+        if (work[k].empty() && (k > 0 || !work[1].empty())) continue;
+        int rc = run_columns<T>(G, o, B, work[k], k > 0, stats, unconv);
+        if (rc) return rc;
     }
     if ((o.flags & EQD_FLAG_STRICT) && unconv > 0)
         return fail(EQD_ERR_NOT_CONVERGED, std::to_string(unconv) + " column(s) did not converge");

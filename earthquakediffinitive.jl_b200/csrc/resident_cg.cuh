@@ -49,6 +49,8 @@
 //
 // The order of every sum is fixed by the plan, which depends on the grid and
 // the precision only: a column gives the same bits alone and in any batch.
+// (Explicit right-hand sides on grids of a team that is for a few of them: while
+// a call has no more than four a team; beyond that it streams them.)
 #pragma once
 #include <type_traits>
 
