@@ -927,7 +927,7 @@ static void launch_xfold(eqd_grid *G, double *x64, float *d, const int8_t *statu
     xlayout_kernel<true><<<xlayout_blocks(l, ncols), 256, 0, s>>>(l, x64, d, nullptr, nullptr, status, flag, ncols);
 }
 
-static void launch_xresidual(eqd_grid *G, float *r, float *p, const float *src, const int8_t *status,
+static void launch_xresidual(eqd_grid *G, float *r, float *p, float *src, const int8_t *status,
                              const int8_t *flag, int ncols, cudaStream_t s) {
     const XLayout &l = G->xm.lay;
     xlayout_kernel<false><<<xlayout_blocks(l, ncols), 256, 0, s>>>(l, nullptr, r, src, p, status, flag, ncols);
@@ -1265,13 +1265,54 @@ struct BatchSpec {
     int8_t *status;
 };
 
-static int resolve_chunk(eqd_grid *G, const eqd_solve_opts &o, int ncols, int prec, int &chunk) {
+// Whether the options and the pinned variant leave a solve to the on-chip CG.
+static bool allows_resident(const eqd_grid *G, const eqd_solve_opts &o) {
+    return o.precond != EQD_PRECOND_JACOBI && (G->pin < 0 || G->pin == kResidentVariant);
+}
+
+// What runs a solve's iterations: resident_cg_kernel, or xmarch_kernel on
+// x2-fastest vectors, or (neither) the streamed x1-fastest path.
+struct Path {
+    bool resident = false, xm = false;
+};
+
+// `on_chip`: explicit right-hand sides (`gen`) that run resident.
+template <typename T>
+static int choose_path(eqd_grid *G, const eqd_solve_opts &o, bool gen, bool on_chip, Path &p) {
+    p = Path{};
+    p.resident = gen && on_chip;
+    if (!gen && allows_resident(G, o)) {
+        ResEngine &E = sizeof(T) == 4 ? G->res32 : G->res64;
+        int rc = ensure_resident<T>(G, E);
+        if (rc) return rc;
+        p.resident = E.ok && !E.few;
+    }
+    if (sizeof(T) == 4 && !gen && !p.resident && o.precond != EQD_PRECOND_JACOBI &&
+        (G->pin < 0 || G->pin == kResidentVariant || G->pin == kXMarchVariant)) {
+        int rc = ensure_xmarch(G);
+        if (rc) return rc;
+        p.xm = G->xm.ok;
+    }
+    return EQD_OK;
+}
+
+// Device bytes of a slot: x in FP64; r, p, q (mixed: and d) in the working
+// precision, and the second direction buffer where the direction update is fused
+// into the apply; the x1 march's vectors with padded x2 lines.
+template <typename T>
+static size_t slot_bytes(const eqd_grid *G, const eqd_solve_opts &o, bool gen, const Path &p) {
     const GridConst &gc = G->gc;
-    // x64 + r, p, q (+ d) (+ the second direction buffer of the fused update).
-    // (The x1 march keeps its residuals in a second layout while they are formed, and pads x2 lines.)
-    const int nvec = 3 + (prec == EQD_PREC_MIXED ? 2 : 0) + ((o.flags & EQD_FLAG_FUSE) ? 1 : 0);
-    const size_t per_col = (size_t)std::max(gc.colstride, x_column(gc.n1, gc.n2, gc.n3)) * (8 + (size_t)nvec * (prec == EQD_PREC_MIXED ? 4 : 8)) +
-                           (size_t)16 * gc.nf + 1024;
+    const bool fused = !p.resident && !p.xm && !gen && o.precond != EQD_PRECOND_JACOBI && (o.flags & EQD_FLAG_FUSE);
+    const size_t nvec = 3 + (sizeof(T) == 4 ? 1 : 0) + (fused ? 1 : 0);
+    const size_t vec = p.xm ? (size_t)x_column(gc.n1, gc.n2, gc.n3) : (size_t)gc.colstride;
+    return (size_t)gc.colstride * 8 + vec * nvec * sizeof(T) + (size_t)16 * gc.nf + 1024;
+}
+
+// The slots of a solve of `ncols` columns, and the path that they run on.
+template <typename T>
+static int resolve_chunk(eqd_grid *G, const eqd_solve_opts &o, int ncols, bool gen, bool on_chip, Path &path, int &chunk) {
+    int rc = choose_path<T>(G, o, gen, on_chip, path);
+    if (rc) return rc;
     size_t budget = o.hbm_budget_bytes;
     if (budget == 0) {
         size_t fr = 0, tot = 0;
@@ -1279,10 +1320,12 @@ static int resolve_chunk(eqd_grid *G, const eqd_solve_opts &o, int ncols, int pr
         const size_t keep = (size_t)2 << 30;
         budget = fr > keep ? fr - keep : fr / 2;
     }
-    long long cap = (long long)(budget / per_col);
+    // (A budget that only the padding overdraws streams x1-fastest.)
+    if (path.xm && budget < slot_bytes<T>(G, o, gen, path)) path.xm = false;
+    long long cap = (long long)(budget / slot_bytes<T>(G, o, gen, path));
     if (cap < 1) return fail(EQD_ERR_OOM, "HBM budget too small for one column");
     const long long want =
-        o.chunk > 0 ? o.chunk : ((G->chunk_tuned > 0 && prec == EQD_PREC_MIXED) ? G->chunk_tuned : cap);
+        o.chunk > 0 ? o.chunk : ((G->chunk_tuned > 0 && sizeof(T) == 4) ? G->chunk_tuned : cap);
     chunk = (int)std::min<long long>(want, ncols);
     if ((long long)chunk > cap) chunk = (int)cap;
     return EQD_OK;
@@ -1396,10 +1439,11 @@ static cudaError_t record_reliable(eqd_grid *G, const IterPtrs<T> &P, const Solv
     cf.flag = P.st.flag;
     cf.dinv = sp.precond ? G->dinv64.as<double>() : nullptr;
     EQD_TRY(cudaGetLastError());
-    EQD_TRY((launch_march<double, float, MODE_RHS>(G, P.x64, sp.xlayout ? (float *)P.p2 : (float *)P.r, cf, P.res_part,
+    // (x2-fastest vectors: q is read by now, and holds the residuals until r has them.)
+    EQD_TRY((launch_march<double, float, MODE_RHS>(G, P.x64, sp.xlayout ? (float *)P.q : (float *)P.r, cf, P.res_part,
                                                    sn.n, -1, sn.s)));
     if (sp.xlayout)
-        launch_xresidual(G, (float *)P.r, (float *)P.p, (const float *)P.p2, P.st.status, P.st.flag, sn.n, sn.s);
+        launch_xresidual(G, (float *)P.r, (float *)P.p, (float *)P.q, P.st.status, P.st.flag, sn.n, sn.s);
     SolveParams sp2 = sp;
     sp2.ntiles = nparts(G->m64);
     cg_true_residual_kernel<<<(unsigned)((sn.n + 3) / 4), 128, 0, sn.s>>>(P.st, sp2, P.res_part, sn.n, 1);
@@ -1572,11 +1616,6 @@ struct ColDone {
 
 static int tune_by_iterations(eqd_grid *G, const eqd_solve_opts &o, int ncols, bool with_resident = false);
 
-// Whether the options and the pinned variant leave a solve to the on-chip CG.
-static bool allows_resident(const eqd_grid *G, const eqd_solve_opts &o) {
-    return o.precond != EQD_PRECOND_JACOBI && (G->pin < 0 || G->pin == kResidentVariant);
-}
-
 template <typename T>
 struct SlotRun {
     eqd_grid *G = nullptr;
@@ -1599,10 +1638,9 @@ struct SlotRun {
     int64_t launches = 0;
     static constexpr int kIter = 10;
 
-    // `tuning`: the caller times kIter iterations a launch. `on_chip`: the
-    // explicit right-hand sides run resident (explicit_on_chip).
-    int setup(eqd_grid *g, const eqd_solve_opts &o, int capacity, bool gen, bool dns, bool tuning = false,
-              bool on_chip = false) {
+    // `tuning`: the caller times kIter iterations a launch.
+    int setup(eqd_grid *g, const eqd_solve_opts &o, int capacity, bool gen, bool dns, const Path &path,
+              bool tuning = false) {
         G = g;
         W = &G->ws;
         cap = capacity;
@@ -1611,22 +1649,10 @@ struct SlotRun {
         dense = dns;
         const GridConst &gc = G->gc;
         const long long ntot = 6LL * gc.n1 * gc.n2 * gc.n3;
-        resident = gen && on_chip;
-        if (!gen && allows_resident(G, o)) {
-            ResEngine &E = sizeof(T) == 4 ? G->res32 : G->res64;
-            int rc = ensure_resident<T>(G, E);
-            if (rc) return rc;
-            resident = E.ok && !E.few;
-        }
+        resident = path.resident;
+        xm = path.xm;
         kmax = tuning ? kIter : 256;
         rounds = mixed && !tuning ? 2 : 1;
-        xm = 0;
-        if (mixed && !gen && !resident && o.precond != EQD_PRECOND_JACOBI &&
-            (G->pin < 0 || G->pin == kResidentVariant || G->pin == kXMarchVariant)) {
-            int rc = ensure_xmarch(G);
-            if (rc) return rc;
-            xm = G->xm.ok;
-        }
         if (mixed && !G->tuned && !resident && !xm) {
             int rc = tune_by_iterations(G, o, std::min(cap, 1024));
             if (rc) return rc;
@@ -1643,7 +1669,7 @@ struct SlotRun {
             const MarchCfg &mc = sizeof(T) == 4 ? G->v32[G->sel32] : G->m64;
             fused = !resident && !xm && !generic && o.precond != EQD_PRECOND_JACOBI && (o.flags & EQD_FLAG_FUSE) && mc.smem_af > 0;
         }
-        if (fused || xm) CUDA_OR_RETURN(w.v4.ensure(sizeof(T) * vec64));
+        if (fused) CUDA_OR_RETURN(w.v4.ensure(sizeof(T) * vec64));
         else w.v4.release();
         int ntmax = std::max(nt64, nparts(G->m32));
         for (int v = 0; v < kNumVariants; ++v) ntmax = std::max(ntmax, nparts(G->v32[v]));
@@ -1811,11 +1837,11 @@ struct SlotRun {
             ColumnSet cs = colset();
             cs.flag = mask;
             cs.dinv = sp.precond ? G->dinv64.as<double>() : nullptr;
-            CUDA_OR_RETURN((launch_march<double, T, MODE_RHS>(G, w.x64.as<double>(), xm ? w.v4.as<T>() : w.v0.as<T>(), cs,
+            CUDA_OR_RETURN((launch_march<double, T, MODE_RHS>(G, w.x64.as<double>(), xm ? w.v2.as<T>() : w.v0.as<T>(), cs,
                                                                w.res_part.as<double>(), cap)));
             SolveParams sp2 = sp;
             sp2.ntiles = nparts(G->m64);
-            if (xm) launch_xresidual(G, w.v0.as<float>(), w.v1.as<float>(), w.v4.as<float>(), w.status.as<int8_t>(), mask, cap, G->stream);
+            if (xm) launch_xresidual(G, w.v0.as<float>(), w.v1.as<float>(), w.v2.as<float>(), w.status.as<int8_t>(), mask, cap, G->stream);
             cg_true_residual_kernel<<<sb, 128, 0, G->stream>>>(st, sp2, w.res_part.as<double>(), cap, mixed, mask);
             launches += 2 + (xm ? 1 : 0);
         } else {
@@ -1987,7 +2013,9 @@ static int tune_by_iterations(eqd_grid *G, const eqd_solve_opts &o, int ncols, b
         G->pin = v;
         if (v < kNumVariants) G->sel32 = v;
         SlotRun<float> R;
-        int rc = R.setup(G, ot, ncols, false, false, true);
+        Path path;
+        int rc = choose_path<float>(G, ot, false, false, path);
+        if (!rc) rc = R.setup(G, ot, ncols, false, false, path, true);
         if (rc) return rc;
         int taken = 0;
         rc = R.admit(work.data(), ncols, taken);
@@ -2061,10 +2089,11 @@ static int run_columns(eqd_grid *G, const eqd_solve_opts &o, const BatchSpec &B,
     const int generic = B.rhs != nullptr, ncols = (int)work.size();
     const long long ntot = 6LL * gc.n1 * gc.n2 * gc.n3;
     int chunk = 0;
-    int rc = resolve_chunk(G, o, ncols, o.precision, chunk);
+    Path path;
+    int rc = resolve_chunk<T>(G, o, ncols, generic, on_chip, path, chunk);
     if (rc) return rc;
     SlotRun<T> R;
-    rc = R.setup(G, o, chunk, generic, B.slip_dense != nullptr, false, on_chip);
+    rc = R.setup(G, o, chunk, generic, B.slip_dense != nullptr, path);
     if (rc) return rc;
     int64_t tot_it = 0, max_it = 0, unconv = 0;
     PinnedArr<double> &kstage = R.W->kstage;
@@ -2483,7 +2512,8 @@ extern "C" int eqd_tune_chunk(eqd_grid *G, const int32_t *widths, int32_t nwidth
     eqd_solve_opts o;
     eqd_default_opts(&o);
     int cap = 0;
-    int rc = resolve_chunk(G, o, 2 * gc.nf, EQD_PREC_MIXED, cap);
+    Path path;
+    int rc = resolve_chunk<float>(G, o, 2 * gc.nf, false, false, path, cap);
     if (rc) return rc;
     double bestms = 1e300;
     int bestw = 0;
@@ -2500,7 +2530,7 @@ extern "C" int eqd_tune_chunk(eqd_grid *G, const int32_t *widths, int32_t nwidth
             work[i].tag = i;
         }
         SlotRun<float> R;
-        rc = R.setup(G, o, w, false, false, true);
+        rc = R.setup(G, o, w, false, false, path, true);
         if (rc) return rc;
         int taken = 0;
         rc = R.admit(work.data(), w, taken);
@@ -3153,12 +3183,19 @@ extern "C" int eqd_server_add_grid(eqd_server *S, eqd_grid *G, int32_t slots) {
     CUDA_OR_RETURN(cudaSetDevice(G->desc.device));
     const GridConst &gc = G->gc;
     const int mixed = S->opts.precision == EQD_PREC_MIXED;
-    const int nvec = 3 + (mixed ? 2 : 0) + ((S->opts.flags & EQD_FLAG_FUSE) ? 1 : 0);  // as resolve_chunk
-    const size_t per_slot = (size_t)std::max(gc.colstride, x_column(gc.n1, gc.n2, gc.n3)) * (8 + (size_t)nvec * (mixed ? 4 : 8)) + (size_t)16 * gc.nf + 1024;
+    Path path;
+    int rc = mixed ? choose_path<float>(G, S->opts, false, false, path)
+                   : choose_path<double>(G, S->opts, false, false, path);
+    if (rc) return rc;
+    auto bytes = [&]() {
+        return mixed ? slot_bytes<float>(G, S->opts, false, path) : slot_bytes<double>(G, S->opts, false, path);
+    };
     std::unique_ptr<SrvGrid> g(new SrvGrid());
     {
         std::lock_guard<std::mutex> lk(S->mu);
         const uint64_t left = S->budget > S->used ? S->budget - S->used : 0;
+        if (path.xm && left / bytes() < (uint64_t)std::max(slots, 1)) path.xm = false;  // as resolve_chunk
+        const size_t per_slot = bytes();
         const long long fit = (long long)(left / per_slot);
         const int want = slots > 0 ? slots : (int)std::min<long long>(fit, 512);
         if (want < 1 || (long long)want > fit)
@@ -3169,7 +3206,7 @@ extern "C" int eqd_server_add_grid(eqd_server *S, eqd_grid *G, int32_t slots) {
         S->used += g->bytes;
     }
     g->G = G;
-    int rc = set_grid_priority(G);
+    rc = set_grid_priority(G);
     if (rc) {
         std::lock_guard<std::mutex> lk(S->mu);
         S->used -= g->bytes;
@@ -3177,10 +3214,10 @@ extern "C" int eqd_server_add_grid(eqd_server *S, eqd_grid *G, int32_t slots) {
     }
     if (mixed) {
         g->r32.reset(new SlotRun<float>());
-        rc = g->r32->setup(G, S->opts, g->slots, false, false);
+        rc = g->r32->setup(G, S->opts, g->slots, false, false, path);
     } else {
         g->r64.reset(new SlotRun<double>());
-        rc = g->r64->setup(G, S->opts, g->slots, false, false);
+        rc = g->r64->setup(G, S->opts, g->slots, false, false, path);
     }
     if (!rc) {
         cudaError_t e = g->kstage.assign(2 * gc.nf * g->slots, 0.0);

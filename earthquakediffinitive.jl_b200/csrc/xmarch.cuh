@@ -451,7 +451,10 @@ struct XLayout {
 
 // FOLD: x += d, d = 0 (x FP64, x1-fastest; d x2-fastest). Else: r = src (src
 // x1-fastest, r in d, x2-fastest) and p += the change of r, so that p = r +
-// beta p holds for the new r (a column that enters has r = p = 0: p = r).
+// beta p holds for the new r (a column that enters has r = p = 0: p = r). src
+// is q's memory, column after column at the x1-fastest stride (which is no
+// longer, x_column): zeroed once read, so that q's padding, which the step
+// kernel reads, is zero again. The rest of q the next apply writes.
 // The blocks share out the items of the flagged columns, of which there are
 // usually none or a few: one column then has the whole chip (a few blocks to
 // each column took 100 to 170 us whenever one was flagged, of 400 an iteration
@@ -459,7 +462,7 @@ struct XLayout {
 constexpr int kXLayoutBlocks = 592;  // four an SM
 template <bool FOLD>
 __global__ void __launch_bounds__(256) xlayout_kernel(XLayout g, double *__restrict__ x, float *__restrict__ d,
-                                                      const float *__restrict__ src, float *__restrict__ p,
+                                                      float *__restrict__ src, float *__restrict__ p,
                                                       const int8_t *__restrict__ status,
                                                       const int8_t *__restrict__ flag, int ncols) {
     __shared__ float t[32][EQD_MAX_N1 + 1];
@@ -486,7 +489,10 @@ __global__ void __launch_bounds__(256) xlayout_kernel(XLayout g, double *__restr
                     __syncthreads();
                     for (int i = threadIdx.x; i < m * g.n1; i += 256) x[po + i] += (double)t[i / g.n1][i % g.n1];
                 } else {
-                    for (int i = threadIdx.x; i < m * g.n1; i += 256) t[i / g.n1][i % g.n1] = src[po + i];
+                    for (int i = threadIdx.x; i < m * g.n1; i += 256) {
+                        t[i / g.n1][i % g.n1] = src[po + i];
+                        src[po + i] = 0.f;
+                    }
                     __syncthreads();
                     for (int xx = warp; xx < g.n1; xx += 8)
                         if (lane < m) {
