@@ -426,6 +426,7 @@ struct eqd_grid {
     bool tuned = false;
     int pin = -1;          // variant the caller (or eqd_autotune) chose, kResidentVariant included; -1: none,
                            // and solves run resident where the grid has a plan
+    int pin64 = -1;        // the same for FP64 solves, the caller's only: the tuner times mixed precision
     ResEngine res32, res64;
     XEngine xm;
     int chunk_tuned = 0;   // eqd_tune_chunk's choice of columns per batch (0: as many as the budget allows)
@@ -1266,8 +1267,10 @@ struct BatchSpec {
 };
 
 // Whether the options and the pinned variant leave a solve to the on-chip CG.
+template <typename T>
 static bool allows_resident(const eqd_grid *G, const eqd_solve_opts &o) {
-    return o.precond != EQD_PRECOND_JACOBI && (G->pin < 0 || G->pin == kResidentVariant);
+    const int pin = sizeof(T) == 4 ? G->pin : G->pin64;
+    return o.precond != EQD_PRECOND_JACOBI && (pin < 0 || pin == kResidentVariant);
 }
 
 // What runs a solve's iterations: resident_cg_kernel, or xmarch_kernel on
@@ -1281,7 +1284,7 @@ template <typename T>
 static int choose_path(eqd_grid *G, const eqd_solve_opts &o, bool gen, bool on_chip, Path &p) {
     p = Path{};
     p.resident = gen && on_chip;
-    if (!gen && allows_resident(G, o)) {
+    if (!gen && allows_resident<T>(G, o)) {
         ResEngine &E = sizeof(T) == 4 ? G->res32 : G->res64;
         int rc = ensure_resident<T>(G, E);
         if (rc) return rc;
@@ -2068,7 +2071,7 @@ static bool rhs_in_range(const GridConst &gc, const double *b) {
 template <typename T>
 static int explicit_on_chip(eqd_grid *G, const eqd_solve_opts &o, const BatchSpec &B, std::vector<char> &on) {
     on.assign(B.ncols, 0);
-    if (!allows_resident(G, o)) return EQD_OK;
+    if (!allows_resident<T>(G, o)) return EQD_OK;
     ResEngine &E = sizeof(T) == 4 ? G->res32 : G->res64;
     int rc = ensure_resident<T>(G, E);
     if (rc || !E.ok) return rc;
@@ -2237,10 +2240,10 @@ static int run_batch_any(eqd_grid *G, const eqd_solve_opts *opts, const BatchSpe
     CUDA_OR_RETURN(cudaSetDevice(G->desc.device));
     // A per-call variant replaces the grid's selection for this call only.
     const int sel_before = G->sel32;
-    const int pin_before = G->pin;
+    const int pin_before = G->pin, pin64_before = G->pin64;
     const bool tuned_before = G->tuned;
     if (o.variant > 0) {
-        G->pin = o.variant - 1;
+        G->pin = G->pin64 = o.variant - 1;
         if (G->pin < kNumVariants) {
             G->sel32 = G->pin;
             G->tuned = true;
@@ -2249,6 +2252,7 @@ static int run_batch_any(eqd_grid *G, const eqd_solve_opts *opts, const BatchSpe
     int rc = o.precision == EQD_PREC_MIXED ? run_batch<float>(G, o, B, stats) : run_batch<double>(G, o, B, stats);
     if (o.variant > 0) {
         G->pin = pin_before;
+        G->pin64 = pin64_before;
         if (o.variant - 1 < kNumVariants) {
             G->sel32 = sel_before;
             G->tuned = tuned_before;
@@ -2561,7 +2565,7 @@ extern "C" int eqd_set_variant(eqd_grid *G, int32_t variant) {
     if (!G || variant < 0 || variant >= kAllVariants) return fail(EQD_ERR_ARG, "invalid variant");
     std::lock_guard<std::mutex> lk(G->mtx);
     if (G->served) return fail(EQD_ERR_ARG, "the grid is attached to a server");
-    G->pin = variant;
+    G->pin = G->pin64 = variant;
     if (variant < kNumVariants) {
         G->sel32 = variant;
         G->tuned = true;

@@ -199,7 +199,7 @@ int eqd_profile_apply(eqd_grid *grid, int32_t ncols, int32_t precision, int32_t 
  * variant 12); variant 12 streams x2-fastest vectors with the x1-march
  * stencil. Times 20 mixed-precision CG iterations of ncols
  * unit-slip columns (<= 2nf) with every variant, keeps the fastest for this
- * grid (used by every later call) and reports milliseconds per iteration
+ * grid (used by every later mixed-precision call) and reports milliseconds per iteration
  * (0 for variants without a plan). Arrays hold *nvariants (<= 16) entries.
  * ncols = 0 re-tunes nothing: it reports the current selection and the times
  * of the last tuning (zeros if the grid was never tuned). */
