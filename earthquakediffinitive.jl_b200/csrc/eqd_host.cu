@@ -2845,7 +2845,9 @@ static int kmat_apply(eqd_kmat *M, const double *s, double *y, int nvec, cudaStr
 #undef EQD_KS
         gemv_reduce_kernel<<<(unsigned)((ne + 255) / 256), 256, 0, st>>>(M->part.as<double>(), n, ns, nvec, y);
     } else {
-        if (gemv_overlap(s, y, ne)) CUDA_OR_RETURN(M->part.ensure(sizeof(double) * (size_t)ne));
+        // (Also where this call does not need it: the first call with an n * nvec allocates, and a
+        // captured one after it, y over s or not, must not.)
+        CUDA_OR_RETURN(M->part.ensure(sizeof(double) * (size_t)ne));
         CUDA_OR_RETURN(launch_gemv_any(st, K, s, n, nvec, y, M->part.as<double>()));
     }
     CUDA_OR_RETURN(cudaGetLastError());
