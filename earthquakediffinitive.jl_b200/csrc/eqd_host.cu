@@ -547,8 +547,8 @@ static cudaError_t launch_march(eqd_grid *G, const T *in, TO *out, ColumnSet cs,
         return cudaGetLastError();
     }
     constexpr int MAXT = sizeof(T) == 4 ? kMaxT32 : kMaxT64;
-    MarchCfg m = segmented(sizeof(T) == 4 ? G->m32 : G->m64, flagged_cols(cs, ncols), G->num_sms);
-    if (sizeof(T) == 8 && cs.flag) m.g.target = 2 * G->num_sms;
+    MarchCfg m = segmented(sizeof(T) == 4 ? G->m32 : G->m64, MODE == MODE_RHS ? flagged_cols(cs, ncols) : ncols, G->num_sms);
+    if (MODE == MODE_RHS && sizeof(T) == 8 && cs.flag) m.g.target = 2 * G->num_sms;
     if (MODE == MODE_AF) m.smem = m.smem_af;
     const OpConst<T> &C = *reinterpret_cast<const OpConst<T> *>(sizeof(T) == 4 ? (const void *)&G->c32
                                                                                : (const void *)&G->c64);

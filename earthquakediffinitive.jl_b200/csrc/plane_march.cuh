@@ -298,16 +298,21 @@ plane_march_kernel(const __grid_constant__ OpConst<T> C, const __grid_constant__
 
     const int n1 = N1 > 0 ? N1 : g.n1;
     const int n2 = g.n2, n3 = g.n3;
+    // (Residual instances only, the ones that are launched with flags: as a
+    // run-time value in all of them it cost the FP64 applies 15 to 110 bytes of
+    // spills and 3 to 12 % of a solve.)
     int segblk = g.segblk;
-    if (SEG && g.target > 0) {
-        int busy = 0;  // columns with work
-        for (int c0 = 0; c0 < cs.ncols; c0 += blockDim.x) {
-            const int c = c0 + threadIdx.x;
-            busy += __syncthreads_count(c < cs.ncols && (!cs.status || cs.status[c] == COL_ACTIVE) && cs.flag[c]);
+    if constexpr (SEG && MODE == MODE_RHS) {
+        if (g.target > 0) {
+            int busy = 0;  // columns with work
+            for (int c0 = 0; c0 < cs.ncols; c0 += blockDim.x) {
+                const int c = c0 + threadIdx.x;
+                busy += __syncthreads_count(c < cs.ncols && (!cs.status || cs.status[c] == COL_ACTIVE) && cs.flag[c]);
+            }
+            const int ctas = busy * g.ntiles, want = ctas >= g.target ? 1 : min((g.target + ctas - 1) / ctas, g.nblk);
+            segblk = max(segblk, (g.nblk + want - 1) / want);
+            if (seg * segblk >= g.nblk) return;
         }
-        const int ctas = busy * g.ntiles, want = ctas >= g.target ? 1 : min((g.target + ctas - 1) / ctas, g.nblk);
-        segblk = max(segblk, (g.nblk + want - 1) / want);
-        if (seg * segblk >= g.nblk) return;
     }
     // x3 segment (FP64-input instances). March step s ingests plane s, does
     // the in-plane work and finishes components 1, 2 of plane p = s - 3, and
