@@ -300,7 +300,7 @@ def split_node_solve(solver, rhs):
     """`split_node_solve(s, rhs)`: solve A u = rhs (reference DOF layout)
     by FP64 CG with Krylov's stopping rule. `rhs` may hold several columns;
     a column's solution does not depend on the others, but for its last bits on
-    grids of lines of 19 to 29 points that only a team of CTAs holds, where a
+    grids of lines of 17 to 29 points that only a team of CTAs holds, where a
     call of more than four columns a team streams (include/eqd.h)."""
     fe = solver.fe
     if fe is None:

@@ -390,7 +390,7 @@ struct ResEngine {
     ResDims d{};
     int t2 = 0, t3 = 0;  // tile capacity of the kernel instance
     int teams = 0;       // > 0: teams that meet through global memory (else one cluster a column)
-    bool few = false;    // for a few explicit right-hand sides only
+    bool few = false;    // the teams are for a few explicit right-hand sides only
     DevBuf ranks, chunks, lines, gofs, push, pull, tab, off, team_p, team_red, team_count;
     ResTables tb{};
 };
@@ -612,12 +612,11 @@ static cudaError_t configure_kernels(int smem_max) {
 // Kernel instances: n1, the largest tile of own lines, and the parts that a
 // line is cut into. The x1 lines of the BP8 grids at 100, 80, 50 and 40 m (9 to
 // 21 points) and of the cubes up to 25. The last number: 0, one cluster to a
-// column; 2, a team that meets through global memory (17 points: 4 teams of 36
-// CTAs at 33 x 33, one column 3.1 ms against 19.6 streamed, 96 columns 67
-// against 89); 1, such a team for a few explicit right-hand sides only, up to
-// four a team (25^3: one 5.3 ms against 22, 12 32 against 45). Where a CTA has
-// fewer lines, the streamed iteration is the better one for many (25^3, 300
-// columns: 243 ms against 579), and the choice for columns does not depend on
+// column; 1, a team that meets through global memory, for a few explicit
+// right-hand sides, up to four a team (25^3: one 5.3 ms against 22, 12 32
+// against 45); 2, for columns too where team_fills. Where it does not, the
+// streamed iteration is the better one for many (25^3, 300 columns: 243 ms
+// against 579), and the choice for columns does not depend on
 // their number, so that a column's bits do not either. FP32 teams, tried at
 // 17 and 21 points, halve a single column's time (h = 40 m 6.8 ms against
 // 15.3) but lose from 16 on (h = 20 m, 64 columns: 548 ms against 220).
@@ -686,6 +685,19 @@ static cudaError_t put_table(eqd_grid *G, DevBuf &b, const void *src, size_t byt
     return e == cudaSuccess && bytes ? cudaMemcpyAsync(b.p, src, bytes, cudaMemcpyHostToDevice, G->stream) : e;
 }
 
+// Whether teams of M CTAs keep up with the streamed iteration for hundreds of
+// columns: 25 own lines for every SM of the device, and four teams at least
+// (larger ones wait longer for one another). FP64, 17 points, 300 columns,
+// streamed against teams: 33 x 33 nodes (26 lines, 4 teams) 220 ms against 208;
+// 25 x 33 (24, 5) 197, 190; 33 x 25 (24, 5) 161, 167; 41 x 33 (24.5, 3) 290, 339;
+// 29 x 29 (20, 4) 166, 211; 65 x 33 (26, 2) 452, 558; 49 x 17 (19, 4) 148, 183.
+// At 33 x 33 six columns take 3.2 ms against 21, 40 28 against 49, and 1,000 687
+// against 611: the price of one path for every number of columns.
+static bool team_fills(const GridConst &gc, int M, int num_sms) {
+    const int teams = num_sms / M;
+    return teams >= 4 && (long long)(gc.n2 - 2) * (gc.n3 - 2) * teams >= 25LL * num_sms;
+}
+
 // The team and the instance with the least work per column-iteration over the
 // team (whole K at h = 50 m: 8 CTAs of 8 x 16 lines 205 ms, 16 of 8 x 8 227 ms;
 // h = 100 m: 2 of 8 x 16 9.2 ms, 4 of 8 x 8 9.9 ms, 9 of them 15.1 ms).
@@ -728,7 +740,7 @@ static int ensure_resident(eqd_grid *G, ResEngine &E) {
             E.t2 = I.t2;
             E.t3 = I.t3;
             E.teams = I.grid ? fit : 0;
-            E.few = I.few;
+            E.few = I.few || (I.grid && !team_fills(gc, P.d.M, G->num_sms));
         };
         if (I.grid) {  // the fewest tiles that fit
             int m[2] = {1, 1};

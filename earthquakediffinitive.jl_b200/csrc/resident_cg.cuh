@@ -40,8 +40,8 @@
 // all 578 there 12.6 ms (34), all 2,178 at h = 50 m 217 ms (300).
 //
 // FP64 lines of more than 13 points take smaller tiles and more parts a line:
-// one column at 17^3 1.8 ms (streamed 14), 96 at 19^3 33 ms (48), 200 at 15^3
-// 21 ms (42). A grid that no cluster holds (GRID) is shared by a team of CTAs
+// one column at 17^3 1.8 ms (streamed 14), 96 at 19^3 33 ms (48), 200 at 17^3
+// 19 ms (41). A grid that no cluster holds (GRID) is shared by a team of CTAs
 // of one cooperative launch, which exchange p and the dot products through
 // global memory (L2) and meet at a counter there; each team takes columns in
 // turn. One right-hand side at 25^3 on 49 CTAs: 20 us an iteration, 5.3 ms

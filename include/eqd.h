@@ -153,7 +153,7 @@ int eqd_apply(eqd_grid *grid, const double *x, double *y, int32_t ncols, int32_t
  * sides; iters/status per column (may be NULL). FP64 only. A right-hand side
  * that is exactly in the range of P runs on chip where the grid has a plan for
  * that, any other one streamed; neither depends on the others in the call, with
- * one exception: on grids of lines of 19 to 29 points that only a team of CTAs
+ * one exception: on grids of lines of 17 to 29 points that only a team of CTAs
  * holds, those in range run on chip while they are at most four for each team that the
  * device has room for (opts->variant pins one path). */
 int eqd_cg_solve(eqd_grid *grid, const double *rhs, double *u, int32_t ncols, const eqd_solve_opts *opts,

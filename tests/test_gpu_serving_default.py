@@ -62,3 +62,18 @@ def test_teams_take_columns_in_turn(eqd):
     for j, c in enumerate(cols):
         K1, it1, _ = eqd.stiffness_columns(fe, [c])
         assert np.array_equal(K1[:, 0], K[:, j]) and it1[0] == it[j]
+
+
+@pytest.mark.parametrize("n,team", [((17, 33, 33), True), ((17, 49, 17), False), ((17, 65, 33), False)],
+                         ids=["fills", "too_few_lines", "too_few_teams"])
+def test_columns_take_teams_that_fill_the_device(eqd, n, team):
+    """`team_fills`: 25 own lines an SM in four teams at least. Other grids stream their columns,
+    and their explicit right-hand sides keep the team."""
+    L = [(k - 1) / 16 for k in n[1:]]
+    fe = eqd.FaultElasticity(eqd.GridPair(*n, 1.0, (-L[0], L[0]), (-L[1], L[1])), 2.0, 1.0, 0.5, precision="fp64")
+    short, streamed = (eqd.CGSolver(fe, precision="fp64", itmax=20, variant=v) for v in (0, 1))
+    cols = [fe.nf // 2, fe.nf + 3]
+    K, Ks = (eqd.stiffness_columns(fe, cols, solver=s)[0] for s in (short, streamed))
+    assert np.array_equal(K, Ks) == (not team)
+    b = eqd.apply_operator(fe, np.random.default_rng(1).standard_normal(fe.Ntot), mode="HP_DSAT")
+    assert not np.array_equal(eqd.split_node_solve(short, b), eqd.split_node_solve(streamed, b))
