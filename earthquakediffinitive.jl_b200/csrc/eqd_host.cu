@@ -2089,8 +2089,13 @@ static int explicit_on_chip(eqd_grid *G, const eqd_solve_opts &o, const BatchSpe
     if (rc || !E.ok) return rc;
     const size_t ntot = (size_t)6 * G->gc.n1 * G->gc.n2 * G->gc.n3;
     int n = 0;
-    for (int i = 0; i < B.ncols; ++i) n += on[i] = rhs_in_range(G->gc, B.rhs + i * ntot);
-    if (E.few && n > 4 * E.teams) on.assign(B.ncols, 0);
+    for (int i = 0; i < B.ncols; ++i) {
+        n += on[i] = rhs_in_range(G->gc, B.rhs + i * ntot);
+        if (E.few && n > 4 * E.teams) {  // (the rest need not be looked at)
+            on.assign(B.ncols, 0);
+            break;
+        }
+    }
     return EQD_OK;
 }
 
