@@ -2763,8 +2763,11 @@ extern "C" int eqd_kmat_create(int32_t device, int32_t n, const double *K, eqd_k
 }
 
 // Row pairs of a cluster (gemv_kernel): the least of 32, 64 and 128 whose
-// clusters run in one wave, 111 of them on 148 SMs (n = 7,104, 14,208).
-static int gemv_lx(long long n) { return n <= 7104 ? 32 : n <= 14208 ? 64 : 128; }
+// clusters run in one wave. 104 clusters of eight CTAs, six an SM, do on 148 SMs;
+// 106 do not, although the CTAs alone would fit (n = 13,568: 279 us with one
+// vector and 306 with two on 64 row pairs, 227 and 257 on 128; 6,784: 84 with two
+// on 32, 70 on 64).
+static int gemv_lx(long long n) { return n <= 104 * 64 ? 32 : n <= 104 * 128 ? 64 : 128; }
 
 // y = K s, nothing of y in s.
 static cudaError_t launch_gemv(cudaStream_t st, const double *K, const double *s, int n, int nvec, double *y) {
@@ -2809,15 +2812,21 @@ static cudaError_t launch_gemv_any(cudaStream_t st, const double *K, const doubl
 
 // Whether y = K s for nvec vectors runs as the GEMV (K read once per 4) or as
 // the blocked K S on the FP64 tensor cores (once per 16 to 64). Measured, GEMV
-// against blocked: 1 and 2 vectors always (n = 4,356: 27 us, and 40 from 3 on
-// blocked); 3 and 4 while one group of them is one wave (n = 4,356 31 us
-// against 40, n = 6,000 69 against 64); more while K is read a few times from
-// L2, groups x n^2 up to 1e7: n = 578 64 vectors 14.5 us against 22.8, n =
-// 1,156 16 12.5 against 12.6 and 32 18.7 against 15.7, n = 2,178 8 14.5 against
-// 16.7 and 12 20.7 against 17.6, n = 3,000 8 27 against 23.5.
+// against blocked, us. 1 and 2 vectors: always (n = 4,356: 27, and 40 from 3 on
+// blocked). More, while all groups of four are one wave, 71 clusters on 148 SMs:
+// n = 4,544 3 and 4 vectors 32.5 against 41, and 53.5 against 41.5 at 4,600; n =
+// 2,234 8 14.7 and 17.3, 1,400 12 10.6 and 12.9, 16 (88 clusters) 15.0 and 13.4.
+// Beyond one wave where a wave is short: n = 1,000 48 19 and 23, 900 64 23 and 21;
+// 1,156 24 15.8 and 15.8, 28 16.8 and 15.8; 1,300 16 14.7 and 13.8. Odd n has
+// 8-byte loads: n = 3,001 4 22.7 and 24, 3,501 33 and 29; 801 32 15.5 and 17, 1,001
+// 32 18.5 and 17.9, 1,157 16 (76 clusters) 17 and 13.8.
 static bool gemv_better(long long n, int nvec) {
-    const long long groups = (nvec + 3) / 4;
-    return nvec <= 2 || (groups == 1 && n <= 4736) || groups * n * n <= 10000000;
+    const long long groups = (nvec + 3) / 4, reads = groups * n * n;
+    const bool even = n % 2 == 0;
+    if (nvec <= 2) return true;
+    if (groups * ((n + 63) / 64) <= 71) return even || n <= 3200;
+    if (n <= 1000) return reads <= (even ? 10000000 : 5500000);
+    return even && n <= 1280 && reads <= 8200000;
 }
 
 // Column slices of the blocked K S: the count (1..16, slices of at least 128
