@@ -489,11 +489,9 @@ __global__ void __launch_bounds__(256) xlayout_kernel(XLayout g, double *__restr
                     __syncthreads();
                     for (int i = threadIdx.x; i < m * g.n1; i += 256) x[po + i] += (double)t[i / g.n1][i % g.n1];
                 } else {
-                    for (int i = threadIdx.x; i < m * g.n1; i += 256) {
-                        t[i / g.n1][i % g.n1] = src[po + i];
-                        src[po + i] = 0.f;
-                    }
+                    for (int i = threadIdx.x; i < m * g.n1; i += 256) t[i / g.n1][i % g.n1] = src[po + i];
                     __syncthreads();
+                    for (int i = threadIdx.x; i < m * g.n1; i += 256) src[po + i] = 0.f;  // (apart: the loads stay in flight)
                     for (int xx = warp; xx < g.n1; xx += 8)
                         if (lane < m) {
                             const float v = t[lane][side ? xx : g.n1 - 1 - xx];
