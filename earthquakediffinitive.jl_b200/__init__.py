@@ -131,7 +131,8 @@ class CGSolver:
     only the schedule, never the result bits: `split=False` runs a large
     batch as one chain of kernels instead of two overlapping halves, and
     `fuse=True` forms the CG direction inside the stencil apply (slower on
-    B200; for comparison)."""
+    B200; for comparison; of effect where the plane march runs the iterations:
+    a pinned variant 0 to 8, and FP64 on grids without an on-chip plan)."""
 
     def __init__(self, fe=None, rtol=1e-10, atol=0.0, itmax=0, precond="none", precision="mixed",
                  chunk=0, reliable_delta=0.01, hbm_budget_bytes=0, variant=0, split=True, fuse=False):
@@ -255,13 +256,15 @@ class FaultElasticity:
 
 
 def set_stencil_variant(fe, variant):
-    """Pin the FP32 stencil launch variant of this grid (skips autotuning)."""
+    """Pin the launch variant of this grid (skips autotuning); a streamed one
+    also keeps FP64 solves streamed."""
     check(lib().eqd_set_variant(fe.handle, C.c_int32(variant)))
 
 
 def autotune(fe, ncols=256):
-    """Time every FP32 stencil launch variant; returns (selected, [(tile_rows, threads, ms)]),
-    the list indexed by variant (`set_stencil_variant`, CGSolver(variant=k + 1))."""
+    """Time every launch variant and keep the fastest for mixed-precision solves; returns
+    (selected, [(tile_rows, threads, ms)]), the list indexed by variant
+    (`set_stencil_variant`, CGSolver(variant=k + 1))."""
     sel, nv = C.c_int32(), C.c_int32()
     ms, tr, tt = (C.c_double * 16)(), (C.c_int32 * 16)(), (C.c_int32 * 16)()
     check(lib().eqd_autotune(fe.handle, C.c_int32(ncols), C.byref(sel), ms, tr, tt, C.byref(nv)))

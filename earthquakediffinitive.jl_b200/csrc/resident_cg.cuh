@@ -35,9 +35,10 @@
 // What bounds it: latency at 16 warps an SM (the two cluster barriers, the
 // stores to the neighbours, the FP64 reduction), then shared-memory wavefronts
 // (about 45 a point). Measured against the streamed iteration: one column at
-// h = 50 m 15 us an iteration (was 98), one slip's traction 2.3 ms (14.5), the
-// ten Toeplitz columns 3.5 ms (15.7), three columns at h = 100 m 1.7 ms (8.5),
-// all 578 there 12.6 ms (34), all 2,178 at h = 50 m 217 ms (300).
+// h = 50 m 15 us an iteration (was 98), one slip's traction 2.2 ms (14.5), the
+// ten Toeplitz columns 3.2 ms (15.7), three columns at h = 100 m 1.6 ms (8.5),
+// all 578 there 9 ms (34), all 2,178 at h = 50 m 212 ms (300), where the host
+// does not hold a call up.
 //
 // FP64 lines of more than 13 points take smaller tiles and more parts a line:
 // one column at 17^3 1.8 ms (streamed 14), 96 at 19^3 33 ms (48), 200 at 17^3

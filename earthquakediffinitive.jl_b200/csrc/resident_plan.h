@@ -27,9 +27,8 @@ constexpr int kResMaxTeam = 16;        // CTAs of a cluster
 constexpr int kResMaxGridTeam = 100;   // CTAs of a team that meets through global memory
 constexpr int kResMaxWarps = 16;       // of a CTA: one per chunk of own lines and part of the lines
 constexpr int kResLinesPerChunk = 16;  // a warp holds 16 lines x 2 sides, the sides of a line in adjacent lanes
-constexpr int kResRow = 12;            // elements of a table row (ResAxisRow)
+constexpr int kResRow = 12;            // elements of a table row (fill_res_tables)
 constexpr size_t kResSmemMax = 232448; // 227 KB, the most a CTA of sm_100 may use
-constexpr size_t kResSmemTwo = 115712; // and two of them on an SM: (228 - 2) / 2 KB
 
 // The planes a kernel instance is compiled for: tiles of at most T2 x T3 own
 // lines, n1 = N1, elements of EB bytes. Every stride is a constant, so every

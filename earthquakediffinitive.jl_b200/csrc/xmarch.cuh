@@ -5,7 +5,8 @@
 // vectors stored x1-fastest: a thread has one point, reads its x1 neighbours
 // from shared memory with per-lane rows, and pays about 520 instructions a
 // point (900 GB/s at h = 20 m). Here vectors are stored
-//   v[col][side][comp][x][i3][n2p],  x = 0 at the fault on both sides,
+//   v[col][side][comp][x][i3][n2p],  x = 0 at the fault on both sides
+// (a column that 32-bit byte offsets reach: x_offsets_fit),
 // x2 line i2 at 3 + i2 of a row padded to a multiple of 4 (so that tiles, which
 // start at i2 = 1 mod 4, have their halo on a 16-byte boundary), and a CTA owns
 // a tile of 16 x 8 (x2, x3) lines of both sides and steps outwards from the

@@ -65,7 +65,9 @@ typedef enum { EQD_PRECOND_NONE = 0, EQD_PRECOND_JACOBI = 1 } eqd_precond;
                                  copies of r and the previous p) instead of in its own kernel; results
                                  are identical. Off by default: the apply is instruction-issue bound,
                                  and the extra work there costs more than the separate memory-bound
-                                 kernel, which overlaps the other half's apply. */
+                                 kernel, which overlaps the other half's apply. Of effect where the plane
+                                 march runs the iterations: a pinned variant 0-8, and FP64 on grids
+                                 without an on-chip plan. */
 
 /*
  * Two equidistant blocks meeting at the fault plane x1 = 0:
@@ -253,8 +255,8 @@ int eqd_diag(eqd_grid *grid, double *d);
 
 /* Time-loop GEMV `mul!(Δτ, K, slip)` (src/BP8.jl:366) ----------------------
  * K stays resident on the device; y = K s for nvec vectors (n x nvec each,
- * column-major), any n >= 1. From 3 vectors on, K S runs blocked on the FP64
- * tensor cores (K read once per 64 vectors); fewer run as the GEMV. s and y
+ * column-major), any n >= 1. Larger products of 3 and more vectors run blocked on the
+ * FP64 tensor cores (K read once per 16 to 64 vectors), others as the GEMV. s and y
  * are host arrays; the call copies them and returns when y is written. */
 int eqd_kmat_create(int32_t device, int32_t n, const double *K, eqd_kmat **out);
 int eqd_kmat_gemv(eqd_kmat *kmat, const double *s, double *y, int32_t nvec);
