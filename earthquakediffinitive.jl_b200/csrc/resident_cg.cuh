@@ -598,7 +598,8 @@ resident_cg_kernel(const __grid_constant__ ResCoef<T> C, const __grid_constant__
         // |r|^2 - 2 a r.q + a^2 q.q: no second exchange. |r|^2 is summed anew
         // each time, so its rounding does not build up; and where FP64 would
         // stop on the difference, or it is small, the new residual is summed
-        // too (below).
+        // too (below; that bound in explicit operations, so that the compiler
+        // shares none of them with rr and rounds it alike).
         if (warp == 0) {
             if constexpr (GRID) {
                 c1 = 0.0;
@@ -627,7 +628,7 @@ resident_cg_kernel(const __grid_constant__ ResCoef<T> C, const __grid_constant__
                 status = COL_NONFINITE;
             } else if (mixed) {
                 if (rr <= tol * tol || rr <= sp.delta * sp.delta * rr_ref || iters >= itmax) flag = 1;
-            } else if (sqrt(rr) <= tol || rr <= 1e-10 * (gamma + ad * ad * qq)) {
+            } else if (sqrt(rr) <= tol || rr <= 1e-10 * __fma_rn(__dmul_rn(ad, ad), qq, gamma)) {
                 sure = false;
             } else if (iters >= itmax) {
                 status = COL_MAXITER;
